@@ -257,6 +257,10 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
         s_sc[3] = tol * tol;     /* compared with rho = r.r, so no square root per iteration */
         s_sc[4] = sqrt(bb[0]);
     }
+    /* every thread reads s_sc[4] at the top of the loop: without this barrier a warp can take
+     * an earlier kernel's value there for the norm, end its solve at once and leave the CTA's
+     * other warps waiting for it at a barrier that counts warps */
+    __syncthreads();
 
     V3 x = { 0.0, 0.0, 0.0 };   /* FP64 solution (P.x4 holds it during an inner solve) */
     V3 r64 = mine ? ldg3(P.b4, row) : V3{ 0.0, 0.0, 0.0 }; /* FP64 residual, = xi for x = 0 */
