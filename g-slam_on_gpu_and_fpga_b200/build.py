@@ -31,7 +31,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", "-fPIC",
           "-Xcompiler", "-ffp-contract=off", "-I", CSRC, "-I", INC]
 
-LIB_SOURCES = ["structure.cpp", "kernels.cu", "pcg.cu", "pcg_resident.cu", "pcg_mixed.cu", "pcg_static.cu",
+LIB_SOURCES = ["structure.cpp", "kernels.cu", "pcg.cu", "pcg_resident.cu", "pcg_mixed.cu", "pcg_cluster.cu",
+               "cluster_plan.cpp", "pcg_static.cu",
                "adjoint.cu", "batch.cu", "gj.cu", "api.cu", "batch_api.cu", "dropin.cu", "logio.cpp"]
 CLI_SOURCES = ["cli.cpp"]
 DATA_SOURCES = ["datasets.cpp"]

@@ -191,7 +191,9 @@ int gslam_adjoint(gslam_graph *g, const double *dL_dposes, double *dL_dlambda, d
     ACK(cudaGetLastError());
     gslam_solve_stats st;
     memset(&st, 0, sizeof st);
-    rc = gslam_layout_solve(&g->L, g->st, o, g->h_res, &st);
+    /* the exact Hessian can be indefinite away from the optimum; CG then amplifies rounding, so
+     * the sums keep one order whichever solver the graph's size selects */
+    rc = gslam_layout_solve(&g->L, g->st, o, g->h_res, &st, true);
     if (stats) *stats = st;
     if (rc != GSLAM_OK) return rc;
     k_rows_to_poses<<<nblk(n, 256), 256, 0, g->st>>>(n, g->L.iperm, g->L.x4, d_mu);

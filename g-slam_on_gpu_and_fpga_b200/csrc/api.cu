@@ -21,6 +21,7 @@
 #include <string>
 #include <vector>
 
+#include "cluster_plan.h"
 #include "gslam.h"
 #include "gslam_api_internal.h"
 #include "gslam_internal.h"
@@ -108,8 +109,54 @@ void DevMem::release() {
     ptrs.clear();
 }
 
+/* The cluster solver's plan of a single graph, where it is the faster one. One CTA up to 13
+ * slices: such a solve can go past convergence within its 500 iterations, where rounding
+ * decides the iterates, and one CTA adds in the grid-wide solver's order (2.1 us per
+ * iteration at 100 poses, where 2 and 4 CTAs take 2.7). Then four slices per CTA (a warp
+ * per SM sub-partition) up to 16 CTAs: 2.7 us at 800 poses with 8 CTAs (4: 2.9, 2: 3.4),
+ * 2.85 at 2,001 with 16 (8: 3.1, 4: 3.8), 4.8 at 10,000; the grid-wide solver takes 7 to 8.3
+ * at all of these. More than one row per thread (above 10,240 poses) needs values from L2:
+ * 7.8 at 12,000 and 9.5 at 16,000, so such graphs stay with the grid-wide solver. */
+#define CLUSTER_ONE_SLICES 13
+#define CLUSTER_CTA_SLICES 4
+
+static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, int device,
+                          const std::vector<int> &grid_slices) {
+    if (S.n_slices > GSLAM_CLUSTER_CTAS * (GSLAM_CLUSTER_THREADS / 32)) return GSLAM_OK;
+    const int max_ctas = pcg_cluster_max_ctas(device, GSLAM_RES_SMEM_MAX);
+    int ctas = 1;
+    if (S.n_slices > CLUSTER_ONE_SLICES)
+        while (ctas < max_ctas && CLUSTER_CTA_SLICES * ctas < S.n_slices) ctas *= 2;
+    gslam_cluster_part part;
+    std::vector<int> lcol(S.n_slots, 0);
+    if (max_ctas == 0 || !gslam_cluster_plan(S, 0, S.n_slices, ctas, 8, GSLAM_RES_SMEM_MAX, &part, &lcol) || part.rows > 1)
+        return GSLAM_OK;
+    /* the grid-wide solver's CTAs that own slices (the order of its sums) */
+    int vctas = 0;
+    for (size_t c = 0; c + 1 < grid_slices.size(); c++)
+        if (grid_slices[c + 1] > grid_slices[c]) vctas = (int)c + 1;
+    if (vctas > (ctas == 1 ? 32 : GSLAM_CLUSTER_VCTAS)) return GSLAM_OK;
+    DevMem &m = L->mem;
+    std::vector<ClusterJob> job(1);
+    job[0] = ClusterJob{ 0, 0, S.n_slices, 0, 0, 0, part.halo_max };
+    CK(dupload(m, st, &L->cluster_job, job));
+    CK(dupload(m, st, &L->cluster_bounds, part.bounds));
+    CK(dupload(m, st, &L->cluster_halo, part.n_halo));
+    CK(dupload(m, st, &L->cluster_lcol, lcol));
+    CK(dupload(m, st, &L->cluster_exp_ptr, part.exp_ptr));
+    CK(dupload(m, st, &L->cluster_exp, part.exp));
+    L->cluster_ctas = part.ctas;
+    L->cluster_threads = part.threads;
+    L->cluster_rows = part.rows;
+    L->cluster_smem = part.smem;
+    L->cluster_smem_ordered = part.smem_ordered;
+    L->cluster_vctas = vctas;
+    L->cluster_ok = true;
+    return GSLAM_OK;
+}
+
 int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, int device,
-                        const gslam_opts &o) {
+                        const gslam_opts &o, bool batch) {
     DevMem &m = L->mem;
     L->n_rows = S.n_rows;
     L->n_slices = S.n_slices;
@@ -169,7 +216,7 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
     L->cg_ok = false;
     const int rgrid = std::min(pcg_resident_max_grid(device, GSLAM_RES_SMEM_MAX),
                                pcg_mixed_max_grid(device, GSLAM_RES_SMEM_MAX));
-    if (rgrid > 0 && S.n_slices <= 32 * rgrid) {
+    if (!batch && rgrid > 0 && S.n_slices <= 32 * rgrid) {
         const int block = (S.n_slices <= 24 * rgrid) ? 768 : 1024;
         const int cap_sl = block / 32;          /* one slice per warp */
         /* contiguous slice ranges of at most cap_sl slices that minimise the largest
@@ -261,6 +308,8 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 L->resident = true;
                 L->smem_val_cap = cap_res_min; /* the smallest CTA's share (statistics only) */
                 L->smem_bytes = (size_t)end_res;
+                const int rc = cluster_upload(L, S, st, device, cs);
+                if (rc != GSLAM_OK) return rc;
             }
             /* mixed: FP32 values | local columns | D^-1 of own rows (2304 B per slice) | z of
              * own and halo rows (16 B each) | u, v of the first `block` halo rows (32 B each,
@@ -316,7 +365,8 @@ int gslam_layout_ensure_fp32(DevLayout *L, cudaStream_t st) {
 /* Runs the persistent solver on L->val / L->b4; result in L->x4 (new order). */
 /* everything of one solve up to the read-back of its result into h_res, without waiting
  * (also what a captured round records) */
-static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts &o, PcgResult *h_res) {
+static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts &o, PcgResult *h_res,
+                                bool grid_order = false) {
     const int fused_prec = o.precision;
     if (fused_prec == GSLAM_PREC_MIXED) {
         int rc = gslam_layout_ensure_fp32(L, st);
@@ -382,6 +432,10 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
         P.max_refine = 1;
     }
     const bool resident = !mixed && !cg && L->resident && !o.disable_resident;
+    /* a graph that fits one cluster. The test hook names a CTA of the solver that runs; one the cluster does not have goes to
+     * the grid-wide solver, and so does a single CTA, which has nobody to wait for it. */
+    const bool cluster = resident && L->cluster_ok &&
+                         (o.test_absent_cta < 0 || (o.test_absent_cta < L->cluster_ctas && L->cluster_ctas > 1));
     const int grid = (resident || mixed || cg) ? L->res_grid : L->grid;
     {
         /* 2 barriers per iteration + 1: the arrival counter must not wrap */
@@ -402,7 +456,36 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
     P.row_export = L->row_export;
     tr.step("memsets");
     CK(record_event(L->ev0, st));
-    if (mixed) CK(launch_pcg_mixed(st, P, grid, L->res_block, L->mixed_smem_bytes, false));
+    if (cluster) {
+        ClusterParams Q;
+        memset(&Q, 0, sizeof Q);
+        Q.jobs = L->cluster_job;
+        Q.ctas = L->cluster_ctas;
+        Q.cta_slice = L->cluster_bounds;
+        Q.n_halo = L->cluster_halo;
+        Q.lcol = L->cluster_lcol;
+        Q.exp_ptr = L->cluster_exp_ptr;
+        Q.exp = L->cluster_exp;
+        Q.slice_ptr = L->slice_ptr;
+        Q.row_len = L->row_len;
+        Q.n_rows = L->n_rows;
+        Q.val = L->val;
+        Q.dinv = L->dinv;
+        Q.b4 = L->b4;
+        Q.x4 = L->x4;
+        Q.vcta_slice = L->cta_slice;
+        Q.n_vcta = L->cluster_vctas;
+        Q.tol_rel = o.tol;
+        Q.max_iter = o.max_iter;
+        Q.spin_limit = P.spin_limit;
+        Q.absent_cta = o.test_absent_cta;
+        Q.smem_budget = GSLAM_RES_SMEM_MAX;
+        Q.res = L->res;
+        const bool gather = grid_order && L->cluster_ctas > 1; /* one CTA keeps that order anyway */
+        Q.gather = gather ? L->n_slices : 0;
+        CK(launch_pcg_cluster(st, Q, 1, L->cluster_threads, L->cluster_rows,
+                              gather ? L->cluster_smem_ordered : L->cluster_smem, false, false));
+    } else if (mixed) CK(launch_pcg_mixed(st, P, grid, L->res_block, L->mixed_smem_bytes, false));
     else if (cg) CK(launch_pcg_mixed(st, P, grid, L->res_block, L->cg_smem_bytes, true));
     else if (resident) CK(launch_pcg_resident(st, P, grid, L->res_block, L->smem_bytes));
     else CK(launch_pcg(st, P, fused_prec, grid, L->block));
@@ -453,8 +536,8 @@ static int layout_solve_finish(DevLayout *L, cudaStream_t st, const gslam_opts &
 }
 
 int gslam_layout_solve(DevLayout *L, cudaStream_t st, const gslam_opts &o, PcgResult *h_res,
-                       gslam_solve_stats *stats) {
-    int rc = layout_solve_enqueue(L, st, o, h_res);
+                       gslam_solve_stats *stats, bool grid_order) {
+    int rc = layout_solve_enqueue(L, st, o, h_res, grid_order);
     if (rc != GSLAM_OK) return rc;
     HostTrace tr;
     CK(cudaStreamSynchronize(st));
@@ -489,7 +572,7 @@ int finish_setup(gslam_graph *g, const std::vector<unsigned> &t1, const std::vec
     int rc = gslam_build_structure_ex(g->n_poses, (int64_t)t1.size(), t1.data(), t2.data(),
                                       g->o.sell_window, diag_rows, segments, &g->S);
     if (rc != GSLAM_OK) { g_last_error = "bad edge list"; return rc; }
-    rc = gslam_layout_upload(&g->L, g->S, g->st, g->device, g->o);
+    rc = gslam_layout_upload(&g->L, g->S, g->st, g->device, g->o, segments != nullptr);
     if (rc != GSLAM_OK) return rc;
     DevMem &m = g->mem;
     CK(dupload(m, g->st, &g->d_ctr_ptr, g->S.ctr_ptr));
@@ -626,6 +709,9 @@ int gslam_destroy(gslam_graph *g) {
         if (g->batch->h_res) cudaFreeHost(g->batch->h_res);
         if (g->batch->h_gdiff) cudaFreeHost(g->batch->h_gdiff);
         if (g->batch->h_gres) cudaFreeHost(g->batch->h_gres);
+        for (cudaStream_t t : g->batch->side) cudaStreamDestroy(t);
+        for (cudaEvent_t e : g->batch->side_done) cudaEventDestroy(e);
+        if (g->batch->fork) cudaEventDestroy(g->batch->fork);
         delete g->batch;
     }
     round_graph_release(g);

@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(BS, 2) k_pcg_batch(PcgParams P, BatchParams B)
     /* results: each graph's first CTA */
     if ((int)threadIdx.x < nlg) {
         const int t = threadIdx.x, g = g0 + t;
-        if (c == __ldg(B.graph_cta0 + g)) {
+        if (c == __ldg(B.graph_cta0 + g) && (B.skip == nullptr || !__ldg(B.skip + g))) {
             PcgResult r;
             r.iterations = s_iter[t];
             r.reason = s_done[t] ? s_done[t] - 1 : GSLAM_STOP_MAXIT;

@@ -1,0 +1,108 @@
+/*
+ * cluster_plan.cpp — splits one graph's slices over the CTAs of a thread-block cluster for
+ * the cluster solver (pcg_cluster.cu): slice ranges, CTA-local columns, and for every row
+ * the CTAs that read it. Host code, once per graph.
+ */
+#include <algorithm>
+
+#include "cluster_plan.h"
+
+namespace {
+
+/* contiguous ranges of at most `cap` slices over exactly `ctas` CTAs, none empty, each of
+ * at most `bound` slots unless a single slice is larger; false if they do not suffice */
+bool fill(const gslam_structure &S, int sl0, int sl1, int ctas, int cap, int64_t bound, std::vector<int> *out) {
+    int used = 1, nsl = 0;
+    int64_t cur = 0;
+    if (out) out->assign(1, sl0);
+    for (int sl = sl0; sl < sl1; sl++) {
+        const int64_t w = S.slice_ptr[sl + 1] - S.slice_ptr[sl];
+        /* the CTAs still to come need a slice each */
+        const bool must = nsl > 0 && sl1 - sl <= ctas - used;
+        if (must || (nsl > 0 && (cur + w > bound || nsl == cap))) {
+            if (++used > ctas) return false;
+            if (out) out->push_back(sl);
+            cur = 0;
+            nsl = 0;
+        }
+        cur += w;
+        nsl++;
+    }
+    if (out) out->push_back(sl1);
+    return used == ctas;
+}
+
+}  // namespace
+
+bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, int elem, int64_t budget,
+                        gslam_cluster_part *part, std::vector<int> *lcol) {
+    const int ns = sl1 - sl0;
+    const int warps = GSLAM_CLUSTER_THREADS / 32;
+    if (ns < ctas || ns > ctas * warps * GSLAM_CLUSTER_ROWS) return false;
+    part->ctas = ctas;
+    part->rows = ns <= ctas * warps ? 1 : 2;
+    const int cap = warps * part->rows;
+    int64_t lo = 0, hi = S.slice_ptr[sl1] - S.slice_ptr[sl0];
+    for (int sl = sl0; sl < sl1; sl++) lo = std::max(lo, S.slice_ptr[sl + 1] - S.slice_ptr[sl]);
+    while (lo < hi) {
+        const int64_t mid = lo + (hi - lo) / 2;
+        if (fill(S, sl0, sl1, ctas, cap, mid, nullptr)) hi = mid;
+        else lo = mid + 1;
+    }
+    if (!fill(S, sl0, sl1, ctas, cap, lo, &part->bounds)) return false;
+    int most = 0;
+    for (int r = 0; r < ctas; r++) most = std::max(most, part->bounds[r + 1] - part->bounds[r]);
+    part->threads = 32 * ((most + part->rows - 1) / part->rows);
+    /* local columns and halos; the rows each CTA reads from others */
+    part->n_halo.assign(ctas, 0);
+    std::vector<std::vector<int>> halo(ctas);
+    const int row_base = 32 * sl0, n_rows = 32 * ns;
+    part->exp_ptr.assign((size_t)n_rows + 1, 0);
+    part->halo_max = 0;
+    for (int r = 0; r < ctas; r++) {
+        const int row0 = 32 * part->bounds[r], row1 = 32 * part->bounds[r + 1], nloc = row1 - row0;
+        const int64_t a0 = S.slice_ptr[part->bounds[r]], a1 = S.slice_ptr[part->bounds[r + 1]];
+        std::vector<int> &rem = halo[r];
+        for (int64_t t = a0; t < a1; t++) {
+            const int c = S.col[t];
+            if (c >= 0 && (c < row0 || c >= row1)) rem.push_back(c);
+        }
+        std::sort(rem.begin(), rem.end());
+        rem.erase(std::unique(rem.begin(), rem.end()), rem.end());
+        for (int64_t t = a0; t < a1; t++) {
+            const int c = S.col[t];
+            if (c < 0) (*lcol)[t] = 0;
+            else if (c >= row0 && c < row1) (*lcol)[t] = c - row0;
+            else (*lcol)[t] = nloc + (int)(std::lower_bound(rem.begin(), rem.end(), c) - rem.begin());
+        }
+        for (int c : rem) {
+            if (c < row_base || c >= row_base + n_rows) return false; /* a block that leaves the graph's rows */
+            part->exp_ptr[c - row_base + 1]++;
+        }
+        part->n_halo[r] = (int)rem.size();
+        part->halo_max = std::max(part->halo_max, (int)rem.size());
+    }
+    for (int i = 0; i < n_rows; i++) part->exp_ptr[i + 1] += part->exp_ptr[i];
+    part->exp.resize(part->exp_ptr[n_rows]);
+    std::vector<int> at(part->exp_ptr.begin(), part->exp_ptr.end() - 1);
+    for (int r = 0; r < ctas; r++)
+        for (int h = 0; h < part->n_halo[r]; h++)
+            part->exp[at[halo[r][h] - row_base]++] = (unsigned)r << 20 | (unsigned)h;
+    /* shared memory */
+    part->smem = part->smem_ordered = 0;
+    part->on_chip = true;
+    for (int r = 0; r < ctas; r++) {
+        const int64_t n_slots = S.slice_ptr[part->bounds[r + 1]] - S.slice_ptr[part->bounds[r]];
+        const ClusterSmem m = cluster_smem_layout(elem, n_slots, part->bounds[r + 1] - part->bounds[r], part->n_halo[r],
+                                                  part->halo_max, 0, budget);
+        const ClusterSmem mo = cluster_smem_layout(elem, n_slots, part->bounds[r + 1] - part->bounds[r], part->n_halo[r],
+                                                   part->halo_max, ns, budget);
+        if (m.val_cap < 0 || mo.val_cap < 0) return false;
+        if (m.val_cap < 9 * n_slots) part->on_chip = false;
+        part->smem = std::max(part->smem, (size_t)m.end);
+        part->smem_ordered = std::max(part->smem_ordered, (size_t)mo.end);
+    }
+    /* one mbarrier phase counts at most 2^20 - 1 bytes; halo slots are 20-bit */
+    if (16 * (int64_t)ns + 16 * GSLAM_CLUSTER_CTAS + 24 * (int64_t)part->halo_max >= (1 << 20) - 1) return false;
+    return true;
+}

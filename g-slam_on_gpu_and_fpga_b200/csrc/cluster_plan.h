@@ -1,0 +1,31 @@
+/* cluster_plan.h — host-side plan of the cluster solver (internal). */
+#ifndef GSLAM_CLUSTER_PLAN_H
+#define GSLAM_CLUSTER_PLAN_H
+
+#include <cstddef>
+#include <vector>
+
+#include "gslam_internal.h"
+#include "kernels.cuh"
+
+/* one graph's split over a cluster */
+struct gslam_cluster_part {
+    int ctas = 0, threads = 0, rows = 1; /* rows: block rows per thread */
+    int halo_max = 0;
+    bool on_chip = false;                /* every value is in shared memory */
+    size_t smem = 0;                     /* dynamic shared memory of the largest CTA */
+    size_t smem_ordered = 0;             /* the same with the slices' sums gathered in one CTA */
+    std::vector<int> bounds;             /* [ctas + 1] slices */
+    std::vector<int> n_halo;             /* [ctas] */
+    std::vector<int> exp_ptr;            /* [rows of the graph + 1] */
+    std::vector<unsigned> exp;           /* rank << 20 | halo slot */
+};
+
+/* Splits the slices [sl0, sl1) over a cluster of `ctas` CTAs for values of `elem` bytes;
+ * lcol (all slots of the layout) gets the graph's CTA-local columns. False when the graph
+ * does not fit (more rows than the threads own, or the fixed parts of a CTA's shared
+ * memory exceed the budget); *part and the graph's part of lcol are then undefined. */
+bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, int elem, int64_t budget,
+                        gslam_cluster_part *part, std::vector<int> *lcol);
+
+#endif

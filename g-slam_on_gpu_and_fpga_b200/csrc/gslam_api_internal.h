@@ -52,9 +52,33 @@ struct DevLayout {
     bool cg_ok = false;             /* the FP64 one-reduction solver's layout fits */
     int64_t cg_val_cap = 0;        /* doubles staged by the CTA that stages fewest */
     size_t cg_smem_bytes = 0;
+    /* cluster solver (pcg_cluster.cu), when the graph fits one thread-block cluster */
+    bool cluster_ok = false;
+    int cluster_ctas = 0, cluster_threads = 0, cluster_rows = 1, cluster_vctas = 0;
+    size_t cluster_smem = 0, cluster_smem_ordered = 0;
+    ClusterJob *cluster_job = nullptr;
+    int *cluster_bounds = nullptr, *cluster_halo = nullptr, *cluster_lcol = nullptr, *cluster_exp_ptr = nullptr;
+    unsigned *cluster_exp = nullptr;
     double *w4 = nullptr;          /* its sixth published vector (made on first use) */
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;   /* brackets the solver launch */
     int max_grid_alloc() const { return partial_capacity; }
+};
+
+/* A batch's graphs that are solved by one cluster each (pcg_cluster.cu), in one precision:
+ * launches of equal cluster shape, largest clusters first. */
+struct BatchClusters {
+    struct Launch {
+        int job0, n_jobs, ctas, threads, rows;
+        size_t smem;
+    };
+    bool built = false;
+    std::vector<Launch> launches;
+    std::vector<int> in_cluster; /* [n_graphs] 1: has a cluster */
+    bool all = false;            /* every graph has one */
+    ClusterJob *d_jobs = nullptr;
+    int *d_bounds = nullptr, *d_halo = nullptr, *d_lcol = nullptr, *d_exp_ptr = nullptr;
+    unsigned *d_exp = nullptr;
+    int *d_rest_skip = nullptr;  /* [n_graphs] graphs that the grid-wide solver leaves alone */
 };
 
 /* A batch of independent SE(2) graphs as one block-diagonal graph (batch.cu). */
@@ -81,7 +105,12 @@ struct BatchState {
     int *d_gactive = nullptr;
     int *d_gcap = nullptr;       /* mixed: each graph's iteration cap for the current inner pass */
     double *d_gres = nullptr, *h_gres = nullptr;
-    int *d_skip = nullptr;       /* graphs the FP64 rerun of a stagnated mixed batch leaves alone */
+    BatchClusters clusters[2];   /* FP64, FP32 */
+    std::vector<cudaStream_t> side; /* the launches' streams, and their fork and join events */
+    std::vector<cudaEvent_t> side_done;
+    cudaEvent_t fork = nullptr;
+    int *d_skip = nullptr;       /* [2 n_graphs] graphs the FP64 rerun of a stagnated mixed batch leaves
+                                  * alone; the same and those with a cluster */
     /* chunk sums of the per-graph norm kernels */
     double *d_chunk_part = nullptr;
     int max_chunks = 1;
@@ -129,11 +158,14 @@ struct gslam_graph {
     int eager_rounds = 0;
 };
 
+/* batch: a batch's layout, which the single-graph resident solvers never run on */
 int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, int device,
-                        const gslam_opts &o);
+                        const gslam_opts &o, bool batch = false);
 int gslam_layout_ensure_fp32(DevLayout *L, cudaStream_t st);
+/* grid_order: the dot products are added in the grid-wide solver's order whichever solver
+ * runs (same bits), for systems that may be indefinite, where CG amplifies rounding */
 int gslam_layout_solve(DevLayout *L, cudaStream_t st, const gslam_opts &o, PcgResult *h_res,
-                       gslam_solve_stats *stats);
+                       gslam_solve_stats *stats, bool grid_order = false);
 void gslam_layout_release(DevLayout *L);
 /* Assembles Omega / xi from edge blocks; optionally also writes the reference's CSR
  * values (csr_vals) and xi in original order (xi_orig), both device pointers. */
@@ -193,6 +225,6 @@ int finish_setup(gslam_graph *g, const std::vector<unsigned> &t1, const std::vec
                  const std::vector<int> *diag_rows = nullptr, const std::vector<int> *segments = nullptr);
 /* the batched solve behind gslam_solve / gslam_round on a batch handle (batch_api.cu) */
 int batch_solve(gslam_graph *g, gslam_solve_stats *per_graph, gslam_solve_stats *total,
-                const int *d_skip = nullptr);
+                const std::vector<int> *skip = nullptr);
 
 #endif

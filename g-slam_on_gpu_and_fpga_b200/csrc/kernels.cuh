@@ -167,8 +167,9 @@ struct BatchParams {
     int *active;             /* graphs still iterating (set to n_graphs before launch) */
     const float *bf4;        /* FP32 inner solve: right-hand side (padded rows) */
     const int *skip;         /* [n_graphs] or null: graphs left exactly as they are (done from the
-                              * start, their vectors untouched: the mixed batch's FP64 rerun of
-                              * only the graphs that stagnated) */
+                              * start, their vectors and results untouched: graphs a cluster
+                              * solves, and the mixed batch's FP64 rerun of only the graphs that
+                              * stagnated) */
     const int *cap;          /* [n_graphs] or null: each graph's own iteration cap (at most the
                               * launch's max_iter; the mixed batch's inner passes, each graph
                               * with what is left of its budget) */
@@ -201,6 +202,83 @@ int pcg_max_grid(int precision, int block, int device);
 cudaError_t launch_pcg_resident(cudaStream_t st, const PcgParams &p, int grid, int block,
                                 size_t smem_bytes);
 int pcg_resident_max_grid(int device, size_t smem_bytes);
+
+/* Solver of a graph inside one thread-block cluster (pcg_cluster.cu). */
+#define GSLAM_CLUSTER_CTAS 16    /* largest cluster (non-portable size) */
+#define GSLAM_CLUSTER_THREADS 640 /* largest CTA: 20 warps, up to 96 registers a thread */
+#define GSLAM_CLUSTER_ROWS 2     /* block rows a thread may own */
+
+/* one graph for one cluster: the range of its slices and where its per-CTA data lie */
+struct ClusterJob {
+    int graph;            /* batches: the graph whose result and cap it is */
+    int slice0, n_slices;
+    int cta0;             /* first entry in n_halo */
+    int bound0;           /* first entry in cta_slice ([ctas + 1] slice bounds) */
+    int exp0;             /* first entry in exp_ptr ([32 n_slices + 1]) */
+    int halo_max;         /* largest halo of its CTAs */
+};
+
+struct ClusterParams {
+    const ClusterJob *jobs;
+    int job0;             /* the launch's first job */
+    int ctas;             /* CTAs per cluster */
+    const int *cta_slice; /* slice bounds of every job's CTAs */
+    const int *n_halo;    /* halo rows of every job's CTAs */
+    const int *lcol;      /* per slot, CTA-local column index (own rows, then halo) */
+    const int *exp_ptr;   /* per row of a job, bounds in exp */
+    const unsigned *exp;  /* the CTAs that read a row and the halo slot there: rank << 20 | slot */
+    const int64_t *slice_ptr;
+    const int *row_len;
+    int n_rows;
+    const double *val, *dinv, *b4;
+    double *x4;
+    const float *val32, *bf4;  /* FP32 inner solve */
+    float *xf4;
+    const int *vcta_slice;     /* single graphs: the grid-wide solver's slice partition */
+    int n_vcta;                /* its CTAs that own slices */
+    int gather;                /* single graphs: the job's slices when the sums are added in the
+                                * grid-wide solver's order by the cluster's first CTA, else 0 */
+    double tol_rel;
+    int max_iter;
+    long long spin_limit;
+    int absent_cta;
+    int64_t smem_budget;
+    PcgResult *res;            /* single graph: the result; batch: the timeout flag */
+    PcgResult *gres;           /* batch: per graph */
+    const int *skip, *cap;     /* batch: as in BatchParams */
+};
+
+/* Dynamic shared memory of one CTA: what other CTAs store into first, at offsets that depend
+ * on the job alone (the halo's z; with gather = the job's slices, every slice's partial
+ * sums), then local columns, p of own and halo rows, and as many
+ * values (whole multiples of 288) as the budget leaves (val_cap < 0: the fixed parts do not
+ * fit). */
+struct ClusterSmem {
+    int64_t gather2_off, gather_off, zh2_off, col_off, p_off, val_off, val_cap, end;
+};
+__host__ __device__ inline ClusterSmem cluster_smem_layout(int64_t elem, int64_t n_slots, int64_t n_slices,
+                                                           int64_t n_halo, int64_t halo_max, int64_t gather,
+                                                           int64_t budget) {
+    auto up = [](int64_t b) { return (b + 127) / 128 * 128; };
+    ClusterSmem m;
+    m.gather2_off = up(16 * halo_max);
+    m.gather_off = m.gather2_off + up(16 * gather);
+    m.zh2_off = m.gather_off + up(8 * gather);
+    m.col_off = m.zh2_off + (elem == 8 ? up(8 * halo_max) : 0);
+    m.p_off = m.col_off + up(4 * n_slots);
+    m.val_off = m.p_off + up(3 * elem * (32 * n_slices + n_halo));
+    m.val_cap = budget >= m.val_off ? (budget - m.val_off) / elem / 288 * 288 : -1;
+    const int64_t nv = m.val_cap > 9 * n_slots ? 9 * n_slots : (m.val_cap > 0 ? m.val_cap : 0);
+    m.end = m.val_off + up(elem * nv);
+    return m;
+}
+
+cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jobs, int threads, int rows_per_thread,
+                               size_t smem_bytes, bool fp32, bool batch);
+#define GSLAM_CLUSTER_VCTAS 160 /* CTAs of the grid-wide solver whose order a cluster can keep */
+/* Largest cluster the solver's kernels can be launched with (0: none), with this much
+ * dynamic shared memory per CTA; also sets their attributes. */
+int pcg_cluster_max_ctas(int device, size_t smem_bytes);
 
 /* Mixed-precision solver (pcg_mixed.cu); fp64: the same kernel as the FP64 one-reduction
  * solver. */

@@ -1,0 +1,680 @@
+/*
+ * pcg_cluster.cu — block-Jacobi PCG of a whole graph inside one thread-block cluster
+ * (reference algorithm: src/cpu_pcg_fp64/MatrixOps.c:281-391).
+ *
+ * The grid-wide solvers spend most of an iteration in their two grid reductions, each of
+ * several L2 round trips: with 148 CTAs of 768 threads one all-reduce of two doubles takes
+ * 2.4 us, whatever the graph's size. Inside one cluster the same reduction through
+ * distributed shared memory takes 0.66 us (16 CTAs x 256 threads) to 0.87 us (16 x 768),
+ * and a cluster's shared memory (16 x 227 KB) holds the matrix of a graph of about 10,000
+ * poses. So a graph that fits is solved by one cluster of 1 to 16 CTAs, and a batch by one
+ * cluster per graph, as many at a time as the GPU holds.
+ *
+ * Layout: CTA r of a graph's cluster owns a contiguous range of its slices (balanced by
+ * slot count), one thread per block row (R slices per warp). Values (as far as they fit),
+ * CTA-local column indices and p of own and halo rows are in shared memory; x, r, z, p, q
+ * and, for R = 1, the row's D^-1 are in registers. Nothing but the values that do not fit
+ * (and D^-1 for R = 2) is read from L2 during the solve.
+ *
+ * Exchange: warp 0 adds its CTA's partials and stores the sum into every CTA of the cluster
+ * (st.async: the data and the count on the receiver's mbarrier in one message, no fence and
+ * no polling of global memory); each owner stores z of a row that other CTAs read into
+ * their halo arrays the same way, while the sums travel. A CTA's mbarrier completes when
+ * all sums, and the halo's z, are there: one one-way trip per reduction. Warp 0 then adds
+ * the sums and one thread advances the scalars. (Every warp storing its own slice's sum
+ * into every CTA saves the step through warp 0, but the 320 messages per CTA and reduction
+ * of a 16 x 640 cluster take longer: 6.6 us per iteration at 10,000 poses against 4.8, and
+ * 5.2 against 4.0 at 7,120.)
+ *
+ * The two barriers' phases alternate (p.q, then r.r and r.z), and a CTA sends its sums of
+ * phase n + 1 only after it has received every sum of phase n, so one buffer and one
+ * mbarrier per kind are enough: no CTA can overwrite sums, or a halo's z, that another one
+ * still reads (that one's sums of the phase in between come after those reads).
+ *
+ * Summation orders. Each scalar row of q adds its blocks in ascending original column
+ * order with separate multiply and add, as everywhere. Dot products are summed per slice,
+ * then per CTA, then over the CTAs. A single graph's cluster of one CTA sums exactly as the
+ * grid-wide solver (pcg_resident.cu) does: per slice, per CTA of that solver's partition
+ * (vcta_slice; the same tree over its warps), then over its CTAs, so both give the same
+ * bits: the solves of such small graphs can go on past convergence, where rounding alone
+ * decides the iterates. With ORD a larger cluster keeps that order too: every slice's
+ * partials go to the first CTA, which adds them and sends the step back, two trips per
+ * reduction instead of one (for the adjoint, whose matrix may be indefinite).
+ *
+ * T = float is the inner solve of the mixed batch (FP32 values and vectors, FP64 D^-1 and
+ * dot products), with batch.cu's arithmetic.
+ *
+ * Waits are bounded: a wait that runs out marks the solve as timed out and the CTA leaves
+ * through the final cluster barrier (no CTA exits while another may store into its shared
+ * memory).
+ */
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "cluster_common.cuh"
+#include "gslam.h"
+#include "kernels.cuh"
+#include "pcg_common.cuh"
+#include "tma_bulk.cuh"
+
+template <typename T> struct C3 { T a, b, c; };
+
+__device__ __forceinline__ C3<double> cl_ld_row(const double *v4, int row) {
+    const V3 v = ldg3(v4, row);
+    return { v.a, v.b, v.c };
+}
+__device__ __forceinline__ C3<float> cl_ld_row(const float *v4, int row) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(v4 + 4 * (size_t)row));
+    return { v.x, v.y, v.z };
+}
+__device__ __forceinline__ void cl_st_row(double *v4, int row, C3<double> v) { st3(v4, row, V3{ v.a, v.b, v.c }); }
+__device__ __forceinline__ void cl_st_row(float *v4, int row, C3<float> v) {
+    *reinterpret_cast<float4 *>(v4 + 4 * (size_t)row) = make_float4(v.a, v.b, v.c, 0.f);
+}
+
+/* z of halo slot h: FP64 as 16 + 8 bytes in two arrays, FP32 as one float4 */
+__device__ __forceinline__ void cl_send_z(unsigned zh, unsigned zh2, unsigned rank, int h, C3<double> z, unsigned bar) {
+    const unsigned rb = cl_mapa(bar, rank);
+    cl_st_async2(cl_mapa(zh + 16 * h, rank), z.a, z.b, rb);
+    cl_st_async(cl_mapa(zh2 + 8 * h, rank), z.c, rb);
+}
+__device__ __forceinline__ void cl_send_z(unsigned zh, unsigned, unsigned rank, int h, C3<float> z, unsigned bar) {
+    cl_st_async4(cl_mapa(zh + 16 * h, rank), z.a, z.b, z.c, cl_mapa(bar, rank));
+}
+template <typename T>
+__device__ __forceinline__ C3<T> cl_halo_z(const unsigned char *zh, const unsigned char *zh2, int h);
+template <> __device__ __forceinline__ C3<double> cl_halo_z<double>(const unsigned char *zh, const unsigned char *zh2, int h) {
+    const double2 ab = *reinterpret_cast<const double2 *>(zh + 16 * h);
+    return { ab.x, ab.y, *reinterpret_cast<const double *>(zh2 + 8 * h) };
+}
+template <> __device__ __forceinline__ C3<float> cl_halo_z<float>(const unsigned char *zh, const unsigned char *, int h) {
+    const float4 v = *reinterpret_cast<const float4 *>(zh + 16 * h);
+    return { v.x, v.y, v.z };
+}
+
+/* z = D^-1 r in FP64 from the nine entries d(e), rounded to T (apply_dinv's order) */
+template <typename T, typename F>
+__device__ __forceinline__ C3<T> cl_dinv(F d, C3<T> rv) {
+    const double ra = rv.a, rb = rv.b, rc = rv.c;
+    double z0 = 0.0, z1 = 0.0, z2 = 0.0;
+    z0 = z0 + d(0) * ra; z0 = z0 + d(1) * rb; z0 = z0 + d(2) * rc;
+    z1 = z1 + d(3) * ra; z1 = z1 + d(4) * rb; z1 = z1 + d(5) * rc;
+    z2 = z2 + d(6) * ra; z2 = z2 + d(7) * rb; z2 = z2 + d(8) * rc;
+    return { (T)z0, (T)z1, (T)z2 };
+}
+
+template <typename T>
+__device__ __forceinline__ void cl_blk(const T *v, C3<T> p, T &q0, T &q1, T &q2) {
+    q0 = q0 + v[0] * p.a;   q0 = q0 + v[32] * p.b;  q0 = q0 + v[64] * p.c;
+    q1 = q1 + v[96] * p.a;  q1 = q1 + v[128] * p.b; q1 = q1 + v[160] * p.c;
+    q2 = q2 + v[192] * p.a; q2 = q2 + v[224] * p.b; q2 = q2 + v[256] * p.c;
+}
+
+/* butterfly sum: lane 0's value is the shuffle-down tree's bit for bit (each step adds the
+ * same two numbers, and addition is commutative), and every lane has it */
+__device__ __forceinline__ double cl_warp_sum(double a) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a = a + __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+}
+
+/* the sum of the partials v(a) .. v(a + n - 1), n <= 32, as the grid-wide solver's warp
+ * tree adds a CTA's warps (offsets 16, 8, 4, 2, 1; missing warps are 0) */
+template <typename F>
+__device__ __forceinline__ double cl_tree(F v, int a, int n) {
+    auto at = [&](int i) { return i < n ? v(a + i) : 0.0; };
+    if (n <= 1) return at(0);
+    if (n <= 4) return (at(0) + at(2)) + (at(1) + at(3));
+    double b[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) b[i] = n <= 8 ? at(i) : (at(i) + at(i + 16)) + (at(i + 8) + at(i + 24));
+    return ((b[0] + b[4]) + (b[2] + b[6])) + ((b[1] + b[5]) + (b[3] + b[7]));
+}
+
+template <typename T> struct ClVec;
+template <> struct ClVec<double> {
+    static __device__ const double *val(const ClusterParams &P) { return P.val; }
+    static __device__ const double *b(const ClusterParams &P) { return P.b4; }
+    static __device__ double *x(const ClusterParams &P) { return P.x4; }
+};
+template <> struct ClVec<float> {
+    static __device__ const float *val(const ClusterParams &P) { return P.val32; }
+    static __device__ const float *b(const ClusterParams &P) { return P.bf4; }
+    static __device__ float *x(const ClusterParams &P) { return P.xf4; }
+};
+
+/* the smallest number whose rounded square root is not below tol, so that
+ * rr < cl_square_limit(tol) decides as sqrt(rr) < tol does (sqrt is monotonic and correctly
+ * rounded) without a square root on the critical path */
+__device__ __forceinline__ double cl_square_limit(double tol) {
+    double y = tol * tol;
+    for (int i = 0; i < 8 && sqrt(y) < tol; i++) y = __longlong_as_double(__double_as_longlong(y) + 1);
+    for (int i = 0; i < 8 && y > 0.0 && sqrt(__longlong_as_double(__double_as_longlong(y) - 1)) >= tol; i++)
+        y = __longlong_as_double(__double_as_longlong(y) - 1);
+    return y;
+}
+
+/* U blocks of one row with values in shared memory: every load is issued before the first
+ * sum (the warp's slots up to its slice's width exist, padded ones included; a shorter
+ * row's lane leaves its sums alone) */
+template <int U, typename T>
+__device__ __forceinline__ void cl_blocks(const int *cb, const T *sv, const T *sp0, const T *sp1, const T *sp2, int left,
+                                          T &q0, T &q1, T &q2) {
+    int c[U];
+    C3<T> p[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) c[u] = cb[32 * u];
+#pragma unroll
+    for (int u = 0; u < U; u++) p[u] = C3<T>{ sp0[c[u]], sp1[c[u]], sp2[c[u]] };
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        T n0 = q0, n1 = q1, n2 = q2;
+        cl_blk(sv + 288 * u, p[u], n0, n1, n2);
+        if (u < left) {
+            q0 = n0;
+            q1 = n1;
+            q2 = n2;
+        }
+    }
+}
+
+__device__ __forceinline__ void cl_bar_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void cl_bar_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+/* ONE: the cluster is one CTA (its partials stay in its shared memory)
+ * ORD: the sums are added in the grid-wide solver's order by the first CTA (see above) */
+template <typename T, int R, bool ONE, bool BATCH, bool ORD>
+__global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const ClusterParams P) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int MAXS = GSLAM_CLUSTER_THREADS / 32 * R; /* slices of a CTA */
+    __shared__ __align__(8) uint64_t s_mb[5];            /* staging; p.q; r.z, r.r and halo z; ORD: the gathers */
+    __shared__ __align__(16) double s_part[MAXS];        /* the slices' p.q */
+    __shared__ __align__(16) double2 s_part2[MAXS];      /* the slices' (r.z, r.r) */
+    __shared__ __align__(16) double s_all[GSLAM_CLUSTER_CTAS];   /* the CTAs' p.q */
+    __shared__ __align__(16) double2 s_all2[GSLAM_CLUSTER_CTAS]; /* the CTAs' (r.z, r.r) */
+    __shared__ double s_rz, s_rr, s_bn, s_limit;
+    __shared__ double s_alpha, s_beta;
+    /* 0 go on, else 1 + GSLAM_STOP_*: one word per reduction, because a warp may read the
+     * first one while the second reduction is already being decided */
+    __shared__ int s_flag_pq, s_flag;
+    /* first slice and count of each CTA of the grid-wide solver */
+    constexpr bool GRID_SUMS = ORD || (ONE && !BATCH);
+    __shared__ int s_vt[GRID_SUMS ? GSLAM_CLUSTER_VCTAS : 1];
+    __shared__ __align__(16) double2 s_step[2]; /* ORD: (alpha, flag) and (beta, flag) from the first CTA */
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+    const int C = ONE ? 1 : P.ctas, rank = ONE ? 0 : (int)cl_rank(), job = P.job0 + (int)blockIdx.x / C;
+    const ClusterJob J = P.jobs[job];
+    if (BATCH && P.skip != nullptr && __ldg(P.skip + J.graph)) return; /* the whole cluster */
+    const int cta = J.cta0 + rank;
+    const int s0 = __ldg(P.cta_slice + J.bound0 + rank), s1 = __ldg(P.cta_slice + J.bound0 + rank + 1), ns = s1 - s0;
+    const int64_t slot0 = __ldg(P.slice_ptr + s0), slot1 = __ldg(P.slice_ptr + s1);
+    const int n_halo = __ldg(P.n_halo + cta);
+    const int n_loc = 32 * ns, row0 = 32 * s0;
+    const ClusterSmem ml = cluster_smem_layout(sizeof(T), slot1 - slot0, ns, n_halo, J.halo_max, ORD ? P.gather : 0,
+                                               P.smem_budget);
+    const int64_t nval = 9 * (slot1 - slot0), nsm = nval < ml.val_cap ? nval : ml.val_cap;
+    unsigned char *zh = smem, *zh2 = smem + ml.zh2_off;
+    int *scol = reinterpret_cast<int *>(smem + ml.col_off);
+    const int np = n_loc + n_halo;
+    T *sp0 = reinterpret_cast<T *>(smem + ml.p_off), *sp1 = sp0 + np, *sp2 = sp1 + np;
+    T *sval = reinterpret_cast<T *>(smem + ml.val_off);
+    const unsigned b_pq = cl_smem_u32(&s_mb[1]), b_rz = cl_smem_u32(&s_mb[2]);
+    const unsigned a_zh = cl_smem_u32(zh), a_zh2 = cl_smem_u32(zh2);
+    const unsigned bytes_pq = ORD ? 16u : 8u * C;
+    const unsigned bytes_rz = (ORD ? 16u : 16u * C) + (sizeof(T) == 8 ? 24u : 16u) * n_halo;
+    double *g_pq = reinterpret_cast<double *>(smem + ml.gather_off);
+    double2 *g_rz = reinterpret_cast<double2 *>(smem + ml.gather2_off);
+    const unsigned b_gpq = cl_smem_u32(&s_mb[3]), b_grz = cl_smem_u32(&s_mb[4]);
+    auto arm = [&](unsigned bar, unsigned bytes) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    };
+
+    /* ---- barriers, then this CTA's matrix share by TMA ---- */
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 5; i++) tma_mbar_init(&s_mb[i], 1);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (!ONE) {
+            arm(b_pq, bytes_pq);
+            arm(b_rz, bytes_rz);
+        }
+        if (ORD && rank == 0) {
+            arm(b_gpq, 8u * J.n_slices);
+            arm(b_grz, 16u * J.n_slices);
+        }
+        s_flag = s_flag_pq = 0;
+    }
+    if (GRID_SUMS)
+        for (int v = threadIdx.x; v < P.n_vcta; v += blockDim.x) {
+            const int a = __ldg(P.vcta_slice + v), b = __ldg(P.vcta_slice + v + 1);
+            s_vt[v] = a << 6 | (b - a);
+        }
+    /* every CTA's barriers are ready before anything is stored to it */
+    if (ONE) __syncthreads();
+    else cl_sync();
+    const bool absent = rank == P.absent_cta; /* test hook: leaves without sending, the others time out */
+    if (!absent && threadIdx.x == 0) {
+        const unsigned vbytes = (unsigned)(sizeof(T) * nsm), cbytes = (unsigned)(4 * (slot1 - slot0));
+        tma_mbar_expect_tx(&s_mb[0], vbytes + cbytes);
+        if (vbytes) tma_bulk_g2s(sval, ClVec<T>::val(P) + 9 * slot0, vbytes, &s_mb[0]);
+        if (cbytes) tma_bulk_g2s(scol, P.lcol + slot0, cbytes, &s_mb[0]);
+        /* waited for by every thread below, after its first rows are read */
+    }
+
+    /* ---- this thread's rows ---- */
+    int row[R], len[R], wsm[R], width[R], voff[R], e0[R], ecnt[R];
+    bool mine[R];
+    C3<T> x[R], r[R], z[R], p[R];
+    double d[R == 1 ? 9 : 1];
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int s = s0 + warp + i * W;
+        const bool own = s < s1;
+        row[i] = 32 * s + lane;
+        mine[i] = own && row[i] < P.n_rows;
+        len[i] = mine[i] ? __ldg(P.row_len + row[i]) : 0;
+        voff[i] = own ? (int)(__ldg(P.slice_ptr + s) - slot0) : 0;
+        width[i] = own ? (int)(__ldg(P.slice_ptr + s + 1) - slot0 - voff[i]) >> 5 : 0;
+        /* the slice's block positions with values in shared memory (the rest are in L2) */
+        wsm[i] = min(width[i], max(0, ((int)nsm - 9 * voff[i]) / 288));
+        const int er = J.exp0 + row[i] - 32 * J.slice0;
+        e0[i] = mine[i] && !ONE ? __ldg(P.exp_ptr + er) : 0;
+        ecnt[i] = mine[i] && !ONE ? __ldg(P.exp_ptr + er + 1) - e0[i] : 0;
+        x[i] = r[i] = z[i] = p[i] = C3<T>{ 0, 0, 0 };
+        if (R == 1 && mine[i]) {
+            const double *g = P.dinv + 288 * (size_t)s + lane;
+#pragma unroll
+            for (int e = 0; e < 9; e++) d[e] = __ldg(g + 32 * e);
+        }
+    }
+    auto dinv_row = [&](int i, C3<T> rv) {
+        if (R == 1) return cl_dinv<T>([&](int e) { return d[R == 1 ? e : 0]; }, rv);
+        const double *g = P.dinv + 288 * (size_t)(row[i] >> 5) + lane;
+        return cl_dinv<T>([&](int e) { return __ldg(g + 32 * e); }, rv);
+    };
+    /* z of an exported row to the CTAs that read it */
+    auto send_z = [&]() {
+        if constexpr (!ONE) {
+#pragma unroll
+            for (int i = 0; i < R; i++)
+                for (int k = 0; k < ecnt[i]; k++) {
+                    const unsigned code = __ldg(P.exp + e0[i] + k);
+                    cl_send_z(a_zh, a_zh2, code >> 20, (int)(code & 0xfffffu), z[i], b_rz);
+                }
+        }
+    };
+    /* the sum over this CTA's slices, by warp 0, on lane 0 (on every lane unless ONE).
+     * ONE single graphs: in the grid-wide solver's order (per CTA of its partition, then
+     * over its CTAs; steps of the tree that would only add zeros are left out) */
+    const int n_sum = ONE && !BATCH ? P.n_vcta : ns;
+    auto sum_slices = [&](auto v) {
+        double s = 0.0;
+        if (ONE && !BATCH) {
+            if (lane < n_sum) s = cl_tree(v, s_vt[lane] >> 6, s_vt[lane] & 63);
+        } else {
+            for (int c = lane; c < ns; c += 32) s = s + v(c);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            if (o < n_sum) s = s + __shfl_xor_sync(0xffffffffu, s, o);
+        return ONE ? s : __shfl_sync(0xffffffffu, s, 0);
+    };
+    /* the sum over the cluster's CTAs, on lane 0 */
+    auto sum_ctas = [&](double s) {
+#pragma unroll
+        for (int o = GSLAM_CLUSTER_CTAS / 2; o > 0; o >>= 1)
+            if (o < C) s = s + __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    };
+
+    /* ORD: the sum over every slice of the graph in the grid-wide solver's order, by warp 0 of
+     * the first CTA, on every lane */
+    auto sum_grid = [&](auto v) {
+        double s = 0.0;
+        for (int c = lane; c < P.n_vcta; c += 32) s = s + cl_tree(v, s_vt[c] >> 6, s_vt[c] & 63);
+        return cl_warp_sum(s);
+    };
+
+    bool ok = true;
+    int k = 0, reason = GSLAM_STOP_MAXIT;
+    /* ORD, warp 0: every slice's (r.z, r.r) to the first CTA, whose warp 0 makes (beta, flag)
+     * of the totals with `decide` and sends them to every CTA; true on lane 0 of all CTAs
+     * once they, and the halo's z, are in s_step[1] */
+    auto step_rz = [&](auto decide, auto between) {
+        for (int i = lane; i < ns; i += 32)
+            cl_st_async2(cl_mapa(cl_smem_u32(&g_rz[s0 - J.slice0 + i]), 0), s_part2[i].x, s_part2[i].y, cl_mapa(b_grz, 0));
+        between();
+        if (rank == 0) {
+            ok = cl_wait(b_grz, k & 1, P.spin_limit);
+            if (lane == 0 && ok) arm(b_grz, 16u * J.n_slices);
+            const double rz = sum_grid([&](int c) { return g_rz[c].x; }), rr = sum_grid([&](int c) { return g_rz[c].y; });
+            const double2 t = decide(rz, rr);
+            if (lane < C)
+                cl_st_async2(cl_mapa(cl_smem_u32(&s_step[1]), lane), t.x, ok ? t.y : 1.0 + GSLAM_STOP_TIMEOUT, cl_mapa(b_rz, lane));
+        }
+        ok = cl_wait(b_rz, k & 1, P.spin_limit);
+        if (lane == 0 && ok) arm(b_rz, bytes_rz);
+        if (lane == 0) {
+            s_beta = s_step[1].x;
+            s_flag = ok ? (int)s_step[1].y : 1 + GSLAM_STOP_TIMEOUT;
+        }
+    };
+    /* warp 0: totals of (r.z, r.r) once every warp's partials are in s_part2; the caller's
+     * other work between sending and waiting is `between` */
+    auto total_rz = [&](double2 &t, auto between) {
+        t.x = sum_slices([&](int c) { return s_part2[c].x; });
+        t.y = sum_slices([&](int c) { return s_part2[c].y; });
+        if (!ONE) {
+            if (lane < C) cl_st_async2(cl_mapa(cl_smem_u32(&s_all2[rank]), lane), t.x, t.y, cl_mapa(b_rz, lane));
+        }
+        between();
+        if (!ONE) {
+            ok = cl_wait(b_rz, k & 1, P.spin_limit);
+            if (lane == 0 && ok) arm(b_rz, bytes_rz);
+            const double2 v = lane < C ? s_all2[lane] : make_double2(0.0, 0.0);
+            t.x = sum_ctas(v.x);
+            t.y = sum_ctas(v.y);
+        }
+    };
+    if (!absent) {
+        /* ---- x = 0, r = b, z = D^-1 r; r.z and r.r ---- */
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            double rz = 0.0, rr = 0.0;
+            if (mine[i]) {
+                r[i] = cl_ld_row(ClVec<T>::b(P), row[i]);
+                z[i] = dinv_row(i, r[i]);
+                const double r0 = r[i].a, r1 = r[i].b, r2 = r[i].c;
+                rz = rz + r0 * (double)z[i].a; rz = rz + r1 * (double)z[i].b; rz = rz + r2 * (double)z[i].c;
+                rr = rr + r0 * r0; rr = rr + r1 * r1; rr = rr + r2 * r2;
+            }
+            rz = cl_warp_sum(rz);
+            rr = cl_warp_sum(rr);
+            if (lane == 0 && warp + i * W < ns) s_part2[warp + i * W] = make_double2(rz, rr);
+        }
+        __syncthreads();
+        if (ORD && warp == 0) {
+            step_rz([&](double rz, double rr) {
+                if (lane == 0) {
+                    s_rz = rz;
+                    s_rr = rr;
+                    s_bn = sqrt(rr);
+                    s_limit = cl_square_limit(P.tol_rel * sqrt(rr));
+                }
+                return make_double2(0.0, 0.0);
+            }, send_z);
+        } else if (warp == 0) {
+            double2 t;
+            total_rz(t, send_z);
+            if (lane == 0) {
+                s_rz = t.x;
+                s_rr = t.y;
+                s_bn = sqrt(t.y);
+                s_limit = cl_square_limit(P.tol_rel * sqrt(t.y));
+                s_beta = 0.0;
+                if (!ok) s_flag = 1 + GSLAM_STOP_TIMEOUT;
+                else if (BATCH && t.y == 0.0) s_flag = 1 + GSLAM_STOP_TOL; /* zero right-hand side: x = 0 */
+            }
+        } else {
+            send_z();
+        }
+        if (!tma_wait(&s_mb[0], 0, P.spin_limit)) {
+            s_flag = 1 + GSLAM_STOP_TIMEOUT;
+            tma_wait(&s_mb[0], 0, P.spin_limit); /* let the copy finish before the CTA leaves */
+        }
+        __syncthreads();
+        const int cap = BATCH && P.cap != nullptr ? min(P.max_iter, __ldg(P.cap + J.graph)) : P.max_iter;
+        int flag = s_flag;
+        while (flag == 0) {
+            if (k >= cap) break;
+            /* ---- phase A: p = z + beta p, of own rows and (from its own copy) of the halo;
+             *      q = A p; p.q ---- */
+            const T beta = (T)s_beta;
+#pragma unroll
+            for (int i = 0; i < R; i++)
+                if (mine[i]) {
+                    p[i] = k == 0 ? z[i] : C3<T>{ z[i].a + beta * p[i].a, z[i].b + beta * p[i].b, z[i].c + beta * p[i].c };
+                    sp0[row[i] - row0] = p[i].a;
+                    sp1[row[i] - row0] = p[i].b;
+                    sp2[row[i] - row0] = p[i].c;
+                }
+            if (!ONE)
+                for (int h = threadIdx.x; h < n_halo; h += blockDim.x) {
+                    C3<T> hz = cl_halo_z<T>(zh, zh2, h);
+                    T *h0 = sp0 + n_loc + h, *h1 = sp1 + n_loc + h, *h2 = sp2 + n_loc + h;
+                    if (k > 0) hz = C3<T>{ hz.a + beta * *h0, hz.b + beta * *h1, hz.c + beta * *h2 };
+                    *h0 = hz.a;
+                    *h1 = hz.b;
+                    *h2 = hz.c;
+                }
+            __syncthreads();
+            C3<T> q[R];
+#pragma unroll
+            for (int i = 0; i < R; i++) {
+                T q0 = 0, q1 = 0, q2 = 0;
+                const int *cb = scol + voff[i] + lane;
+                const T *sv = sval + 9 * voff[i] + lane;
+                int j = 0;
+                for (; j + 4 <= wsm[i]; j += 4)
+                    cl_blocks<4>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2);
+                switch (wsm[i] - j) {
+                case 1: cl_blocks<1>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2); break;
+                case 2: cl_blocks<2>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2); break;
+                case 3: cl_blocks<3>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2); break;
+                default: break;
+                }
+                /* the share's tail, from L2 */
+                for (j = wsm[i]; j < len[i]; j++) {
+                    const T *gv = ClVec<T>::val(P) + 9 * (slot0 + voff[i]) + lane + 288 * j;
+                    T vb[9];
+#pragma unroll
+                    for (int e = 0; e < 9; e++) vb[e] = __ldg(gv + 32 * e);
+                    const int c = cb[32 * j];
+                    const C3<T> pc = { sp0[c], sp1[c], sp2[c] };
+                    q0 = q0 + vb[0] * pc.a; q0 = q0 + vb[1] * pc.b; q0 = q0 + vb[2] * pc.c;
+                    q1 = q1 + vb[3] * pc.a; q1 = q1 + vb[4] * pc.b; q1 = q1 + vb[5] * pc.c;
+                    q2 = q2 + vb[6] * pc.a; q2 = q2 + vb[7] * pc.b; q2 = q2 + vb[8] * pc.c;
+                }
+                q[i] = C3<T>{ q0, q1, q2 };
+                double pq = 0.0;
+                if (mine[i]) {
+                    pq = pq + (double)p[i].a * (double)q0; pq = pq + (double)p[i].b * (double)q1;
+                    pq = pq + (double)p[i].c * (double)q2;
+                }
+                pq = cl_warp_sum(pq);
+                if (lane == 0 && warp + i * W < ns) s_part[warp + i * W] = pq;
+            }
+            if (warp == 0) {
+                cl_bar_sync(1, blockDim.x);
+                if (ORD) {
+                    for (int i = lane; i < ns; i += 32)
+                        cl_st_async(cl_mapa(cl_smem_u32(&g_pq[s0 - J.slice0 + i]), 0), s_part[i], cl_mapa(b_gpq, 0));
+                    if (rank == 0) {
+                        ok = cl_wait(b_gpq, k & 1, P.spin_limit);
+                        if (lane == 0 && ok) arm(b_gpq, 8u * J.n_slices);
+                        const double pq = sum_grid([&](int c) { return g_pq[c]; });
+                        const double flag = !ok ? 1.0 + GSLAM_STOP_TIMEOUT : pq == 0.0 ? 1.0 + GSLAM_STOP_PQ_ZERO : 0.0;
+                        if (lane < C)
+                            cl_st_async2(cl_mapa(cl_smem_u32(&s_step[0]), lane), s_rz / pq, flag, cl_mapa(b_pq, lane));
+                    }
+                    ok = cl_wait(b_pq, k & 1, P.spin_limit);
+                    if (lane == 0 && ok) arm(b_pq, bytes_pq);
+                    if (lane == 0) {
+                        s_alpha = s_step[0].x;
+                        s_flag_pq = ok ? (int)s_step[0].y : 1 + GSLAM_STOP_TIMEOUT;
+                    }
+                } else {
+                double pq = sum_slices([&](int c) { return s_part[c]; });
+                if (!ONE) {
+                    if (lane < C) cl_st_async(cl_mapa(cl_smem_u32(&s_all[rank]), lane), pq, cl_mapa(b_pq, lane));
+                    ok = cl_wait(b_pq, k & 1, P.spin_limit);
+                    if (lane == 0 && ok) arm(b_pq, bytes_pq);
+                    pq = sum_ctas(lane < C ? s_all[lane] : 0.0);
+                }
+                if (lane == 0) {
+                    if (!ok) s_flag_pq = 1 + GSLAM_STOP_TIMEOUT;
+                    else if (pq == 0.0) s_flag_pq = 1 + GSLAM_STOP_PQ_ZERO;
+                    s_alpha = s_rz / pq;
+                }
+                }
+            } else {
+                cl_bar_arrive(1, blockDim.x);
+            }
+            __syncthreads();
+            flag = s_flag_pq;
+            if (flag) break;
+            /* ---- phase B: x += alpha p, r -= alpha q, z = D^-1 r; r.r and r.z ---- */
+            const T alpha = (T)s_alpha;
+#pragma unroll
+            for (int i = 0; i < R; i++) {
+                double rr = 0.0, rz = 0.0;
+                if (mine[i]) {
+                    r[i] = C3<T>{ r[i].a - alpha * q[i].a, r[i].b - alpha * q[i].b, r[i].c - alpha * q[i].c };
+                    z[i] = dinv_row(i, r[i]);
+                    const double r0 = r[i].a, r1 = r[i].b, r2 = r[i].c;
+                    rr = rr + r0 * r0; rr = rr + r1 * r1; rr = rr + r2 * r2;
+                    rz = rz + r0 * (double)z[i].a; rz = rz + r1 * (double)z[i].b; rz = rz + r2 * (double)z[i].c;
+                }
+                rr = cl_warp_sum(rr);
+                rz = cl_warp_sum(rz);
+                if (lane == 0 && warp + i * W < ns) s_part2[warp + i * W] = make_double2(rz, rr);
+            }
+            k++;
+            /* while the sums travel: the halo's z, and x */
+            auto rest = [&]() {
+                send_z();
+#pragma unroll
+                for (int i = 0; i < R; i++)
+                    x[i] = C3<T>{ x[i].a + alpha * p[i].a, x[i].b + alpha * p[i].b, x[i].c + alpha * p[i].c };
+            };
+            if (warp == 0) {
+                cl_bar_sync(2, blockDim.x);
+                double2 t;
+                if (ORD)
+                    step_rz([&](double rz, double rr) {
+                        const double b = rz / s_rz;
+                        __syncwarp();
+                        if (lane == 0) {
+                            s_rz = rz;
+                            s_rr = rr;
+                        }
+                        return make_double2(b, rr < s_limit ? 1.0 + GSLAM_STOP_TOL : 0.0);
+                    }, rest);
+                else total_rz(t, rest);
+                if (!ORD && lane == 0) {
+                    if (!ok) s_flag = 1 + GSLAM_STOP_TIMEOUT;
+                    else if (t.y < s_limit) s_flag = 1 + GSLAM_STOP_TOL;
+                    s_beta = t.x / s_rz;
+                    s_rz = t.x;
+                    s_rr = t.y;
+                }
+            } else {
+                cl_bar_arrive(2, blockDim.x);
+                rest();
+            }
+            __syncthreads();
+            flag = s_flag;
+        }
+        if (flag) reason = flag - 1;
+        if (!ONE && reason == GSLAM_STOP_TIMEOUT) {
+            /* a message sent before another CTA gave up has long arrived; the margin covers
+             * a limit of a few cycles */
+            const long long t0 = clock64();
+            while (clock64() - t0 < 100000) {}
+        }
+        if (reason == GSLAM_STOP_TIMEOUT && threadIdx.x == 0) res_mark_timeout(P.res);
+#pragma unroll
+        for (int i = 0; i < R; i++)
+            if (mine[i]) cl_st_row(ClVec<T>::x(P), row[i], x[i]);
+        if (rank == 0 && threadIdx.x == 0 && (BATCH || reason != GSLAM_STOP_TIMEOUT)) {
+            PcgResult *res = BATCH ? P.gres + J.graph : P.res;
+            res->iterations = k;
+            res->refinements = 0;
+            res->rnorm = sqrt(s_rr);
+            res->bnorm = s_bn;
+            if (BATCH) res->reason = reason;
+            else atomicCAS(&res->reason, 0, reason); /* another CTA's timeout stays */
+        }
+    }
+    if (!ONE) {
+        __syncthreads();
+        cl_sync();
+    }
+}
+
+template <typename T, bool BATCH>
+static const void *fn_of(int rows, bool one) {
+    if (rows == 1)
+        return one ? (const void *)k_pcg_cluster<T, 1, true, BATCH, false> : (const void *)k_pcg_cluster<T, 1, false, BATCH, false>;
+    return one ? (const void *)k_pcg_cluster<T, 2, true, BATCH, false> : (const void *)k_pcg_cluster<T, 2, false, BATCH, false>;
+}
+
+/* kinds of launches: FP32 batches, FP64 batches, single graphs, single graphs with ordered
+ * sums (single graphs have one row per thread) */
+static const void *cluster_fn(int kind, int rows, bool one) {
+    switch (kind) {
+    case 0: return fn_of<float, true>(rows, one);
+    case 1: return fn_of<double, true>(rows, one);
+    case 2: return one ? (const void *)k_pcg_cluster<double, 1, true, false, false>
+                       : (const void *)k_pcg_cluster<double, 1, false, false, false>;
+    default: return (const void *)k_pcg_cluster<double, 1, false, false, true>;
+    }
+}
+
+static void cluster_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at, int grid, int ctas, int threads,
+                           size_t smem, cudaStream_t st) {
+    *cfg = {};
+    cfg->gridDim = dim3(grid);
+    cfg->blockDim = dim3(threads);
+    cfg->dynamicSmemBytes = smem;
+    cfg->stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg->attrs = at;
+    cfg->numAttrs = 1;
+}
+
+cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jobs, int threads, int rows_per_thread,
+                               size_t smem_bytes, bool fp32, bool batch) {
+    if (n_jobs <= 0) return cudaSuccess;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    cluster_config(&cfg, at, n_jobs * p.ctas, p.ctas, threads, smem_bytes, st);
+    ClusterParams copy = p;
+    void *args[] = { &copy };
+    const int kind = fp32 ? 0 : batch ? 1 : p.gather ? 3 : 2;
+    if (kind > 1 && rows_per_thread != 1) return cudaErrorInvalidValue;
+    return cudaLaunchKernelExC(&cfg, cluster_fn(kind, rows_per_thread, p.ctas == 1), args);
+}
+
+int pcg_cluster_max_ctas(int device, size_t smem_bytes) {
+    (void)device;
+    int best = 0;
+    for (int v = 0; v < 16; v++) {
+        const void *fn = cluster_fn(v >> 2, 1 + (v & 1), (v & 2) != 0);
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess ||
+            cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        if (v & 2) continue; /* one CTA needs no cluster */
+        int can = 0;
+        for (int c = GSLAM_CLUSTER_CTAS; c > 1; c /= 2) {
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute at[1];
+            cluster_config(&cfg, at, c, c, GSLAM_CLUSTER_THREADS, smem_bytes, nullptr);
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) { can = c; break; }
+            cudaGetLastError();
+        }
+        best = v == 0 ? can : std::min(best, can);
+    }
+    return std::max(best, 1);
+}
