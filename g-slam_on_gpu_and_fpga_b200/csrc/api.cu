@@ -109,20 +109,22 @@ void DevMem::release() {
     ptrs.clear();
 }
 
-/* The cluster solver's plan of a single graph, where it is the faster one. One CTA up to 13
- * slices: such a solve can go past convergence within its 500 iterations, where rounding
- * decides the iterates, and one CTA adds in the grid-wide solver's order (2.1 us per
- * iteration at 100 poses, where 2 and 4 CTAs take 2.7). Then four slices per CTA (a warp
- * per SM sub-partition) up to 16 CTAs: 2.7 us at 800 poses with 8 CTAs (4: 2.9, 2: 3.4),
- * 2.85 at 2,001 with 16 (8: 3.1, 4: 3.8), 4.8 at 10,000; the grid-wide solver takes 7 to 8.3
- * at all of these. More than one row per thread (above 10,240 poses) needs values from L2:
- * 7.8 at 12,000 and 9.5 at 16,000, so such graphs stay with the grid-wide solver. */
+/* The cluster solver's plan of a single graph, where it is the faster one. Us per iteration,
+ * cluster / grid-wide solver: 1.5 / 3.4 at 100 poses, 2.7 / 3.35 at 800, 2.85 / 3.4 at 2,001,
+ * 3.2 / 3.5 at 4,000, 3.45 / 3.47 at 5,000 (city walks); landmark logs, with longer rows,
+ * 3.4 / 4.0 at 2,001, 3.8 / 4.1 at 4,000, 4.2 / 3.9 at 5,000: up to 144 slices (4,608 rows).
+ * One CTA up to 13 slices: such a solve can go past convergence within its 500 iterations,
+ * where rounding decides the iterates, and one CTA adds in the grid-wide solver's order (2.1
+ * at 100 poses, where 2 and 4 CTAs take 2.7). Then four slices per CTA (a warp per SM
+ * sub-partition) up to 16 CTAs: 2.7 at 800 poses with 8 CTAs (4: 2.9, 2: 3.4), 2.85 at
+ * 2,001 with 16 (8: 3.1, 4: 3.8). */
 #define CLUSTER_ONE_SLICES 13
 #define CLUSTER_CTA_SLICES 4
+#define CLUSTER_MAX_SLICES 144
 
 static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, int device,
                           const std::vector<int> &grid_slices) {
-    if (S.n_slices > GSLAM_CLUSTER_CTAS * (GSLAM_CLUSTER_THREADS / 32)) return GSLAM_OK;
+    if (S.n_slices > CLUSTER_MAX_SLICES) return GSLAM_OK;
     const int max_ctas = pcg_cluster_max_ctas(device, GSLAM_RES_SMEM_MAX);
     int ctas = 1;
     if (S.n_slices > CLUSTER_ONE_SLICES)
@@ -135,7 +137,7 @@ static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t s
     int vctas = 0;
     for (size_t c = 0; c + 1 < grid_slices.size(); c++)
         if (grid_slices[c + 1] > grid_slices[c]) vctas = (int)c + 1;
-    if (vctas > (ctas == 1 ? 32 : GSLAM_CLUSTER_VCTAS)) return GSLAM_OK;
+    if (ctas == 1 && vctas > 32) return GSLAM_OK;
     DevMem &m = L->mem;
     std::vector<ClusterJob> job(1);
     job[0] = ClusterJob{ 0, 0, S.n_slices, 0, 0, 0, part.halo_max };
@@ -149,7 +151,6 @@ static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t s
     L->cluster_threads = part.threads;
     L->cluster_rows = part.rows;
     L->cluster_smem = part.smem;
-    L->cluster_smem_ordered = part.smem_ordered;
     L->cluster_vctas = vctas;
     L->cluster_ok = true;
     return GSLAM_OK;
@@ -214,7 +215,7 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
     L->resident = false;
     L->mixed_ok = false;
     L->cg_ok = false;
-    const int rgrid = std::min(pcg_resident_max_grid(device, GSLAM_RES_SMEM_MAX),
+    const int rgrid = std::min(pcg_resident_max_grid(device, GSLAM_GRID_SMEM_MAX),
                                pcg_mixed_max_grid(device, GSLAM_RES_SMEM_MAX));
     if (!batch && rgrid > 0 && S.n_slices <= 32 * rgrid) {
         const int block = (S.n_slices <= 24 * rgrid) ? 768 : 1024;
@@ -257,12 +258,14 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
         if (ok) {
             L->res_grid = rgrid;
             L->res_block = block;
+            for (int i = 0; i < rgrid; i++) L->res_slices = std::max(L->res_slices, cs[i + 1] - cs[i]);
             CK(dupload(m, st, &L->cta_slice, cs));
             L->partial_capacity = std::max(L->partial_capacity, rgrid);
             /* CTA-local column indices (own rows first, then the CTA's halo) and halo lists */
             std::vector<int> lcol(S.n_slots, 0), hptr(rgrid + 1, 0), hrows;
             /* mixed / FP64 one-reduction solvers: every CTA's own layout must fit */
             bool fit32 = true, fit64 = true, fit_res = true;
+            std::vector<int> keep(S.n_slices, 0), pos(S.n_slices, 0);
             int64_t cap32_min = INT64_MAX, cap64_min = INT64_MAX, cap_res_min = INT64_MAX;
             /* the largest CTA's layout end: the launch asks for no more shared memory than
              * that (shared memory and L1 share the SM's SRAM, and these kernels read D^-1 and
@@ -291,8 +294,16 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 const MixedSmem l64 = mixed_smem_layout(8, true, a1 - a0, cs[i + 1] - cs[i], (int64_t)rem.size(), block,
                                                         GSLAM_RES_SMEM_MAX);
                 const ResidentSmem lr = resident_smem_layout(a1 - a0, cs[i + 1] - cs[i], (int64_t)rem.size(),
-                                                             GSLAM_RES_SMEM_MAX);
+                                                             GSLAM_GRID_SMEM_MAX);
                 fit_res = fit_res && lr.val_cap >= 0;
+                /* positions that do not fit are left out evenly: the last one of every slice,
+                 * then of every slice that still has one, and so on */
+                int64_t out = std::max<int64_t>(0, (9 * (a1 - a0) - std::max<int64_t>(lr.val_cap, 0)) / 288);
+                for (int sl = cs[i]; sl < cs[i + 1]; sl++) keep[sl] = (int)((S.slice_ptr[sl + 1] - S.slice_ptr[sl]) / 32);
+                while (out > 0)
+                    for (int sl = cs[i]; sl < cs[i + 1] && out > 0; sl++)
+                        if (keep[sl] > 0) { keep[sl]--; out--; }
+                for (int sl = cs[i] + 1; sl < cs[i + 1]; sl++) pos[sl] = pos[sl - 1] + keep[sl - 1];
                 cap_res_min = std::min(cap_res_min, std::min<int64_t>(lr.val_cap, 9 * (a1 - a0)));
                 fit32 = fit32 && l32.val_cap >= 0;
                 fit64 = fit64 && l64.val_cap >= 0;
@@ -308,6 +319,8 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 L->resident = true;
                 L->smem_val_cap = cap_res_min; /* the smallest CTA's share (statistics only) */
                 L->smem_bytes = (size_t)end_res;
+                CK(dupload(m, st, &L->res_keep, keep));
+                CK(dupload(m, st, &L->res_pos, pos));
                 const int rc = cluster_upload(L, S, st, device, cs);
                 if (rc != GSLAM_OK) return rc;
             }
@@ -341,7 +354,11 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
         }
     }
     CK(dalloc(m, &L->partials, 8 * (size_t)L->partial_capacity));
-    CK(dalloc(m, &L->gs, 1));
+    /* barrier state and, behind it, the tagged reductions' slots: one memset clears both */
+    L->tag_bytes = 256 + 2 * TAG_VALUES * sizeof(TagWord) * (size_t)L->res_grid;
+    unsigned char *sync = nullptr;
+    CK(dalloc(m, &sync, L->tag_bytes));
+    L->gs = reinterpret_cast<GridSync *>(sync);
     CK(dalloc(m, &L->res, 1));
     CK(cudaEventCreate(&L->ev0));
     CK(cudaEventCreate(&L->ev1));
@@ -407,7 +424,8 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
         P.spin_limit = (long long)(ms * (double)L->clock_khz);
     }
     P.absent_cta = o.test_absent_cta;
-    CK(cudaMemsetAsync(L->gs, 0, sizeof(GridSync), st));
+    P.tags = reinterpret_cast<TagWord *>(reinterpret_cast<unsigned char *>(L->gs) + 256);
+    CK(cudaMemsetAsync(L->gs, 0, L->tag_bytes, st));
     CK(cudaMemsetAsync(L->res, 0, sizeof(PcgResult), st));
     const bool mixed = fused_prec == GSLAM_PREC_MIXED;
     const bool cg = fused_prec == GSLAM_PREC_FP64_CG;
@@ -434,7 +452,7 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
     const bool resident = !mixed && !cg && L->resident && !o.disable_resident;
     /* a graph that fits one cluster. The test hook names a CTA of the solver that runs; one the cluster does not have goes to
      * the grid-wide solver, and so does a single CTA, which has nobody to wait for it. */
-    const bool cluster = resident && L->cluster_ok &&
+    const bool cluster = resident && L->cluster_ok && (!grid_order || L->cluster_ctas == 1) &&
                          (o.test_absent_cta < 0 || (o.test_absent_cta < L->cluster_ctas && L->cluster_ctas > 1));
     const int grid = (resident || mixed || cg) ? L->res_grid : L->grid;
     {
@@ -449,12 +467,16 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
     P.smem_val_cap = L->smem_val_cap;
     /* every CTA lays its share out against the full budget, as the host's check did; the
      * launch asks for the largest resulting layout */
-    P.smem_budget = GSLAM_RES_SMEM_MAX;
+    P.smem_budget = resident ? GSLAM_GRID_SMEM_MAX : GSLAM_RES_SMEM_MAX;
     P.lcol = L->lcol;
     P.halo_ptr = L->halo_ptr;
     P.halo_rows = L->halo_rows;
     P.row_export = L->row_export;
+    P.res_keep = L->res_keep;
+    P.res_pos = L->res_pos;
     tr.step("memsets");
+    /* published rows carry their iteration's number: none may be left from an earlier solve */
+    if (resident && !cluster) CK(cudaMemsetAsync(L->z4, 0, 4 * 32 * (size_t)L->n_slices * sizeof(double), st));
     CK(record_event(L->ev0, st));
     if (cluster) {
         ClusterParams Q;
@@ -481,13 +503,10 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
         Q.absent_cta = o.test_absent_cta;
         Q.smem_budget = GSLAM_RES_SMEM_MAX;
         Q.res = L->res;
-        const bool gather = grid_order && L->cluster_ctas > 1; /* one CTA keeps that order anyway */
-        Q.gather = gather ? L->n_slices : 0;
-        CK(launch_pcg_cluster(st, Q, 1, L->cluster_threads, L->cluster_rows,
-                              gather ? L->cluster_smem_ordered : L->cluster_smem, false, false));
+        CK(launch_pcg_cluster(st, Q, 1, L->cluster_threads, L->cluster_rows, L->cluster_smem, false, false));
     } else if (mixed) CK(launch_pcg_mixed(st, P, grid, L->res_block, L->mixed_smem_bytes, false));
     else if (cg) CK(launch_pcg_mixed(st, P, grid, L->res_block, L->cg_smem_bytes, true));
-    else if (resident) CK(launch_pcg_resident(st, P, grid, L->res_block, L->smem_bytes));
+    else if (resident) CK(launch_pcg_resident(st, P, grid, L->res_slices, L->smem_bytes));
     else CK(launch_pcg(st, P, fused_prec, grid, L->block));
     tr.step("solver launch");
     CK(record_event(L->ev1, st));

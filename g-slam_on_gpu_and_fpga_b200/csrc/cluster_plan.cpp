@@ -89,20 +89,17 @@ bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, in
         for (int h = 0; h < part->n_halo[r]; h++)
             part->exp[at[halo[r][h] - row_base]++] = (unsigned)r << 20 | (unsigned)h;
     /* shared memory */
-    part->smem = part->smem_ordered = 0;
+    part->smem = 0;
     part->on_chip = true;
     for (int r = 0; r < ctas; r++) {
         const int64_t n_slots = S.slice_ptr[part->bounds[r + 1]] - S.slice_ptr[part->bounds[r]];
         const ClusterSmem m = cluster_smem_layout(elem, n_slots, part->bounds[r + 1] - part->bounds[r], part->n_halo[r],
-                                                  part->halo_max, 0, budget);
-        const ClusterSmem mo = cluster_smem_layout(elem, n_slots, part->bounds[r + 1] - part->bounds[r], part->n_halo[r],
-                                                   part->halo_max, ns, budget);
-        if (m.val_cap < 0 || mo.val_cap < 0) return false;
+                                                  part->halo_max, budget);
+        if (m.val_cap < 0) return false;
         if (m.val_cap < 9 * n_slots) part->on_chip = false;
         part->smem = std::max(part->smem, (size_t)m.end);
-        part->smem_ordered = std::max(part->smem_ordered, (size_t)mo.end);
     }
     /* one mbarrier phase counts at most 2^20 - 1 bytes; halo slots are 20-bit */
-    if (16 * (int64_t)ns + 16 * GSLAM_CLUSTER_CTAS + 24 * (int64_t)part->halo_max >= (1 << 20) - 1) return false;
+    if (16 * GSLAM_CLUSTER_CTAS + 24 * (int64_t)part->halo_max >= (1 << 20) - 1) return false;
     return true;
 }

@@ -14,7 +14,6 @@ struct gslam_cluster_part {
     int halo_max = 0;
     bool on_chip = false;                /* every value is in shared memory */
     size_t smem = 0;                     /* dynamic shared memory of the largest CTA */
-    size_t smem_ordered = 0;             /* the same with the slices' sums gathered in one CTA */
     std::vector<int> bounds;             /* [ctas + 1] slices */
     std::vector<int> n_halo;             /* [ctas] */
     std::vector<int> exp_ptr;            /* [rows of the graph + 1] */

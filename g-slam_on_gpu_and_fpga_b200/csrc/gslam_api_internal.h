@@ -33,7 +33,8 @@ struct DevLayout {
     double *p4a = nullptr, *p4b = nullptr, *q4 = nullptr;
     float *f[6] = { nullptr, nullptr, nullptr, nullptr, nullptr, nullptr };
     double *partials = nullptr;
-    GridSync *gs = nullptr;
+    GridSync *gs = nullptr;        /* followed by the tagged reductions' slots (tag_words) */
+    size_t tag_bytes = 0;
     PcgResult *res = nullptr;
     int grid = 0, block = 0, n_sm = 0;
     int clock_khz = 2000000;       /* SM clock, for barrier wait limits */
@@ -41,6 +42,8 @@ struct DevLayout {
     /* shared-memory-resident solver (pcg_resident.cu), when the layout fits */
     bool resident = false;
     int res_grid = 0, res_block = 0;
+    int res_slices = 0;            /* slices of the CTA that owns most */
+    int *res_keep = nullptr, *res_pos = nullptr; /* per slice: block positions in shared memory, and where */
     int *cta_slice = nullptr;      /* [res_grid + 1] */
     int64_t smem_val_cap = 0;      /* doubles staged by the CTA that stages fewest */
     int *lcol = nullptr, *halo_ptr = nullptr, *halo_rows = nullptr; /* CTA-local columns, halo lists */
@@ -55,7 +58,7 @@ struct DevLayout {
     /* cluster solver (pcg_cluster.cu), when the graph fits one thread-block cluster */
     bool cluster_ok = false;
     int cluster_ctas = 0, cluster_threads = 0, cluster_rows = 1, cluster_vctas = 0;
-    size_t cluster_smem = 0, cluster_smem_ordered = 0;
+    size_t cluster_smem = 0;
     ClusterJob *cluster_job = nullptr;
     int *cluster_bounds = nullptr, *cluster_halo = nullptr, *cluster_lcol = nullptr, *cluster_exp_ptr = nullptr;
     unsigned *cluster_exp = nullptr;
@@ -162,8 +165,9 @@ struct gslam_graph {
 int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, int device,
                         const gslam_opts &o, bool batch = false);
 int gslam_layout_ensure_fp32(DevLayout *L, cudaStream_t st);
-/* grid_order: the dot products are added in the grid-wide solver's order whichever solver
- * runs (same bits), for systems that may be indefinite, where CG amplifies rounding */
+/* grid_order: the dot products are added in the grid-wide solver's order (a cluster of one
+ * CTA keeps it, a larger one is not used), for systems that may be indefinite, where CG
+ * amplifies rounding */
 int gslam_layout_solve(DevLayout *L, cudaStream_t st, const gslam_opts &o, PcgResult *h_res,
                        gslam_solve_stats *stats, bool grid_order = false);
 void gslam_layout_release(DevLayout *L);

@@ -73,6 +73,7 @@ struct PcgParams {
     int inner_max_iter;
     int max_refine;
     double *partials;      /* [2][4 * gridDim.x]: two alternating buffers */
+    struct TagWord *tags;  /* resident solver: the reductions' slots, [2][TAG_VALUES][gridDim.x], zeroed before a launch */
     GridSync *gs;
     PcgResult *res;
     long long spin_limit;  /* clock cycles a barrier may wait */
@@ -83,11 +84,13 @@ struct PcgParams {
     const int *halo_ptr;   /* resident solver: [grid + 1] halo list bounds per CTA */
     const int *halo_rows;  /* resident solver: halo rows (new row indices) */
     const unsigned char *row_export; /* 1 for rows in another CTA's halo: only those are published */
+    const int *res_keep, *res_pos; /* resident solver, per slice: block positions kept in shared memory, and the
+                            * first one's place there (in positions of 288 values) */
     int64_t smem_budget;   /* resident, mixed and FP64 one-reduction solvers: dynamic shared memory per CTA */
 };
 
 /* Shared-memory layout of one CTA of the FP64 resident solver, from its own sizes: local
- * columns and p of own and halo rows (32 B each) after the values, and as many values (whole
+ * columns and p of own and halo rows (24 B each) after the values, and as many values (whole
  * multiples of 288) as the budget leaves (val_cap < 0: the fixed parts alone do not fit). */
 struct ResidentSmem {
     int64_t val_cap, col_off, p_off, end;
@@ -95,7 +98,7 @@ struct ResidentSmem {
 __host__ __device__ inline ResidentSmem resident_smem_layout(int64_t n_slots, int64_t n_slices, int64_t n_halo,
                                                              int64_t budget) {
     auto up = [](int64_t b) { return (b + 127) / 128 * 128; };
-    const int64_t col_b = up(4 * n_slots), p_b = 32 * (32 * n_slices + n_halo);
+    const int64_t col_b = up(4 * n_slots), p_b = up(24 * (32 * n_slices + n_halo));
     ResidentSmem m;
     const int64_t fixed = col_b + p_b;
     m.val_cap = budget >= fixed ? (budget - fixed) / 8 / 288 * 288 : -1;
@@ -199,7 +202,7 @@ cudaError_t launch_pcg(cudaStream_t st, const PcgParams &p, int precision, int g
 int pcg_max_grid(int precision, int block, int device);
 
 /* Shared-memory-resident solver (pcg_resident.cu). */
-cudaError_t launch_pcg_resident(cudaStream_t st, const PcgParams &p, int grid, int block,
+cudaError_t launch_pcg_resident(cudaStream_t st, const PcgParams &p, int grid, int max_slices,
                                 size_t smem_bytes);
 int pcg_resident_max_grid(int device, size_t smem_bytes);
 
@@ -235,9 +238,7 @@ struct ClusterParams {
     const float *val32, *bf4;  /* FP32 inner solve */
     float *xf4;
     const int *vcta_slice;     /* single graphs: the grid-wide solver's slice partition */
-    int n_vcta;                /* its CTAs that own slices */
-    int gather;                /* single graphs: the job's slices when the sums are added in the
-                                * grid-wide solver's order by the cluster's first CTA, else 0 */
+    int n_vcta;                /* its CTAs that own slices (used by clusters of one CTA) */
     double tol_rel;
     int max_iter;
     long long spin_limit;
@@ -248,22 +249,18 @@ struct ClusterParams {
     const int *skip, *cap;     /* batch: as in BatchParams */
 };
 
-/* Dynamic shared memory of one CTA: what other CTAs store into first, at offsets that depend
- * on the job alone (the halo's z; with gather = the job's slices, every slice's partial
- * sums), then local columns, p of own and halo rows, and as many
+/* Dynamic shared memory of one CTA: the halo's z first (other CTAs store into it, so its
+ * offsets depend on the job alone), then local columns, p of own and halo rows, and as many
  * values (whole multiples of 288) as the budget leaves (val_cap < 0: the fixed parts do not
  * fit). */
 struct ClusterSmem {
-    int64_t gather2_off, gather_off, zh2_off, col_off, p_off, val_off, val_cap, end;
+    int64_t zh2_off, col_off, p_off, val_off, val_cap, end;
 };
 __host__ __device__ inline ClusterSmem cluster_smem_layout(int64_t elem, int64_t n_slots, int64_t n_slices,
-                                                           int64_t n_halo, int64_t halo_max, int64_t gather,
-                                                           int64_t budget) {
+                                                           int64_t n_halo, int64_t halo_max, int64_t budget) {
     auto up = [](int64_t b) { return (b + 127) / 128 * 128; };
     ClusterSmem m;
-    m.gather2_off = up(16 * halo_max);
-    m.gather_off = m.gather2_off + up(16 * gather);
-    m.zh2_off = m.gather_off + up(8 * gather);
+    m.zh2_off = up(16 * halo_max);
     m.col_off = m.zh2_off + (elem == 8 ? up(8 * halo_max) : 0);
     m.p_off = m.col_off + up(4 * n_slots);
     m.val_off = m.p_off + up(3 * elem * (32 * n_slices + n_halo));
@@ -275,7 +272,6 @@ __host__ __device__ inline ClusterSmem cluster_smem_layout(int64_t elem, int64_t
 
 cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jobs, int threads, int rows_per_thread,
                                size_t smem_bytes, bool fp32, bool batch);
-#define GSLAM_CLUSTER_VCTAS 160 /* CTAs of the grid-wide solver whose order a cluster can keep */
 /* Largest cluster the solver's kernels can be launched with (0: none), with this much
  * dynamic shared memory per CTA; also sets their attributes. */
 int pcg_cluster_max_ctas(int device, size_t smem_bytes);

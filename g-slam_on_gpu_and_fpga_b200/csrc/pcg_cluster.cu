@@ -37,9 +37,7 @@
  * grid-wide solver (pcg_resident.cu) does: per slice, per CTA of that solver's partition
  * (vcta_slice; the same tree over its warps), then over its CTAs, so both give the same
  * bits: the solves of such small graphs can go on past convergence, where rounding alone
- * decides the iterates. With ORD a larger cluster keeps that order too: every slice's
- * partials go to the first CTA, which adds them and sends the step back, two trips per
- * reduction instead of one (for the adjoint, whose matrix may be indefinite).
+ * decides the iterates.
  *
  * T = float is the inner solve of the mixed batch (FP32 values and vectors, FP64 D^-1 and
  * dot products), with batch.cu's arithmetic.
@@ -145,17 +143,6 @@ template <> struct ClVec<float> {
     static __device__ float *x(const ClusterParams &P) { return P.xf4; }
 };
 
-/* the smallest number whose rounded square root is not below tol, so that
- * rr < cl_square_limit(tol) decides as sqrt(rr) < tol does (sqrt is monotonic and correctly
- * rounded) without a square root on the critical path */
-__device__ __forceinline__ double cl_square_limit(double tol) {
-    double y = tol * tol;
-    for (int i = 0; i < 8 && sqrt(y) < tol; i++) y = __longlong_as_double(__double_as_longlong(y) + 1);
-    for (int i = 0; i < 8 && y > 0.0 && sqrt(__longlong_as_double(__double_as_longlong(y) - 1)) >= tol; i++)
-        y = __longlong_as_double(__double_as_longlong(y) - 1);
-    return y;
-}
-
 /* U blocks of one row with values in shared memory: every load is issued before the first
  * sum (the warp's slots up to its slice's width exist, padded ones included; a shorter
  * row's lane leaves its sums alone) */
@@ -187,13 +174,12 @@ __device__ __forceinline__ void cl_bar_arrive(int id, int threads) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-/* ONE: the cluster is one CTA (its partials stay in its shared memory)
- * ORD: the sums are added in the grid-wide solver's order by the first CTA (see above) */
-template <typename T, int R, bool ONE, bool BATCH, bool ORD>
+/* ONE: the cluster is one CTA (its partials stay in its shared memory) */
+template <typename T, int R, bool ONE, bool BATCH>
 __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const ClusterParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int MAXS = GSLAM_CLUSTER_THREADS / 32 * R; /* slices of a CTA */
-    __shared__ __align__(8) uint64_t s_mb[5];            /* staging; p.q; r.z, r.r and halo z; ORD: the gathers */
+    __shared__ __align__(8) uint64_t s_mb[3];            /* staging; p.q; r.z, r.r and halo z */
     __shared__ __align__(16) double s_part[MAXS];        /* the slices' p.q */
     __shared__ __align__(16) double2 s_part2[MAXS];      /* the slices' (r.z, r.r) */
     __shared__ __align__(16) double s_all[GSLAM_CLUSTER_CTAS];   /* the CTAs' p.q */
@@ -203,10 +189,7 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
     /* 0 go on, else 1 + GSLAM_STOP_*: one word per reduction, because a warp may read the
      * first one while the second reduction is already being decided */
     __shared__ int s_flag_pq, s_flag;
-    /* first slice and count of each CTA of the grid-wide solver */
-    constexpr bool GRID_SUMS = ORD || (ONE && !BATCH);
-    __shared__ int s_vt[GRID_SUMS ? GSLAM_CLUSTER_VCTAS : 1];
-    __shared__ __align__(16) double2 s_step[2]; /* ORD: (alpha, flag) and (beta, flag) from the first CTA */
+    __shared__ int s_vt[MAXS]; /* ONE single graphs: first slice and count of each CTA of the grid-wide solver */
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
     const int C = ONE ? 1 : P.ctas, rank = ONE ? 0 : (int)cl_rank(), job = P.job0 + (int)blockIdx.x / C;
     const ClusterJob J = P.jobs[job];
@@ -216,8 +199,7 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
     const int64_t slot0 = __ldg(P.slice_ptr + s0), slot1 = __ldg(P.slice_ptr + s1);
     const int n_halo = __ldg(P.n_halo + cta);
     const int n_loc = 32 * ns, row0 = 32 * s0;
-    const ClusterSmem ml = cluster_smem_layout(sizeof(T), slot1 - slot0, ns, n_halo, J.halo_max, ORD ? P.gather : 0,
-                                               P.smem_budget);
+    const ClusterSmem ml = cluster_smem_layout(sizeof(T), slot1 - slot0, ns, n_halo, J.halo_max, P.smem_budget);
     const int64_t nval = 9 * (slot1 - slot0), nsm = nval < ml.val_cap ? nval : ml.val_cap;
     unsigned char *zh = smem, *zh2 = smem + ml.zh2_off;
     int *scol = reinterpret_cast<int *>(smem + ml.col_off);
@@ -226,30 +208,22 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
     T *sval = reinterpret_cast<T *>(smem + ml.val_off);
     const unsigned b_pq = cl_smem_u32(&s_mb[1]), b_rz = cl_smem_u32(&s_mb[2]);
     const unsigned a_zh = cl_smem_u32(zh), a_zh2 = cl_smem_u32(zh2);
-    const unsigned bytes_pq = ORD ? 16u : 8u * C;
-    const unsigned bytes_rz = (ORD ? 16u : 16u * C) + (sizeof(T) == 8 ? 24u : 16u) * n_halo;
-    double *g_pq = reinterpret_cast<double *>(smem + ml.gather_off);
-    double2 *g_rz = reinterpret_cast<double2 *>(smem + ml.gather2_off);
-    const unsigned b_gpq = cl_smem_u32(&s_mb[3]), b_grz = cl_smem_u32(&s_mb[4]);
+    const unsigned bytes_pq = 8u * C, bytes_rz = 16u * C + (sizeof(T) == 8 ? 24u : 16u) * n_halo;
     auto arm = [&](unsigned bar, unsigned bytes) {
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     };
 
     /* ---- barriers, then this CTA's matrix share by TMA ---- */
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 5; i++) tma_mbar_init(&s_mb[i], 1);
+        for (int i = 0; i < 3; i++) tma_mbar_init(&s_mb[i], 1);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (!ONE) {
             arm(b_pq, bytes_pq);
             arm(b_rz, bytes_rz);
         }
-        if (ORD && rank == 0) {
-            arm(b_gpq, 8u * J.n_slices);
-            arm(b_grz, 16u * J.n_slices);
-        }
         s_flag = s_flag_pq = 0;
     }
-    if (GRID_SUMS)
+    if (ONE && !BATCH)
         for (int v = threadIdx.x; v < P.n_vcta; v += blockDim.x) {
             const int a = __ldg(P.vcta_slice + v), b = __ldg(P.vcta_slice + v + 1);
             s_vt[v] = a << 6 | (b - a);
@@ -332,38 +306,8 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
         return s;
     };
 
-    /* ORD: the sum over every slice of the graph in the grid-wide solver's order, by warp 0 of
-     * the first CTA, on every lane */
-    auto sum_grid = [&](auto v) {
-        double s = 0.0;
-        for (int c = lane; c < P.n_vcta; c += 32) s = s + cl_tree(v, s_vt[c] >> 6, s_vt[c] & 63);
-        return cl_warp_sum(s);
-    };
-
     bool ok = true;
     int k = 0, reason = GSLAM_STOP_MAXIT;
-    /* ORD, warp 0: every slice's (r.z, r.r) to the first CTA, whose warp 0 makes (beta, flag)
-     * of the totals with `decide` and sends them to every CTA; true on lane 0 of all CTAs
-     * once they, and the halo's z, are in s_step[1] */
-    auto step_rz = [&](auto decide, auto between) {
-        for (int i = lane; i < ns; i += 32)
-            cl_st_async2(cl_mapa(cl_smem_u32(&g_rz[s0 - J.slice0 + i]), 0), s_part2[i].x, s_part2[i].y, cl_mapa(b_grz, 0));
-        between();
-        if (rank == 0) {
-            ok = cl_wait(b_grz, k & 1, P.spin_limit);
-            if (lane == 0 && ok) arm(b_grz, 16u * J.n_slices);
-            const double rz = sum_grid([&](int c) { return g_rz[c].x; }), rr = sum_grid([&](int c) { return g_rz[c].y; });
-            const double2 t = decide(rz, rr);
-            if (lane < C)
-                cl_st_async2(cl_mapa(cl_smem_u32(&s_step[1]), lane), t.x, ok ? t.y : 1.0 + GSLAM_STOP_TIMEOUT, cl_mapa(b_rz, lane));
-        }
-        ok = cl_wait(b_rz, k & 1, P.spin_limit);
-        if (lane == 0 && ok) arm(b_rz, bytes_rz);
-        if (lane == 0) {
-            s_beta = s_step[1].x;
-            s_flag = ok ? (int)s_step[1].y : 1 + GSLAM_STOP_TIMEOUT;
-        }
-    };
     /* warp 0: totals of (r.z, r.r) once every warp's partials are in s_part2; the caller's
      * other work between sending and waiting is `between` */
     auto total_rz = [&](double2 &t, auto between) {
@@ -398,24 +342,14 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
             if (lane == 0 && warp + i * W < ns) s_part2[warp + i * W] = make_double2(rz, rr);
         }
         __syncthreads();
-        if (ORD && warp == 0) {
-            step_rz([&](double rz, double rr) {
-                if (lane == 0) {
-                    s_rz = rz;
-                    s_rr = rr;
-                    s_bn = sqrt(rr);
-                    s_limit = cl_square_limit(P.tol_rel * sqrt(rr));
-                }
-                return make_double2(0.0, 0.0);
-            }, send_z);
-        } else if (warp == 0) {
+        if (warp == 0) {
             double2 t;
             total_rz(t, send_z);
             if (lane == 0) {
                 s_rz = t.x;
                 s_rr = t.y;
                 s_bn = sqrt(t.y);
-                s_limit = cl_square_limit(P.tol_rel * sqrt(t.y));
+                s_limit = square_limit(P.tol_rel * sqrt(t.y));
                 s_beta = 0.0;
                 if (!ok) s_flag = 1 + GSLAM_STOP_TIMEOUT;
                 else if (BATCH && t.y == 0.0) s_flag = 1 + GSLAM_STOP_TOL; /* zero right-hand side: x = 0 */
@@ -491,24 +425,6 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
             }
             if (warp == 0) {
                 cl_bar_sync(1, blockDim.x);
-                if (ORD) {
-                    for (int i = lane; i < ns; i += 32)
-                        cl_st_async(cl_mapa(cl_smem_u32(&g_pq[s0 - J.slice0 + i]), 0), s_part[i], cl_mapa(b_gpq, 0));
-                    if (rank == 0) {
-                        ok = cl_wait(b_gpq, k & 1, P.spin_limit);
-                        if (lane == 0 && ok) arm(b_gpq, 8u * J.n_slices);
-                        const double pq = sum_grid([&](int c) { return g_pq[c]; });
-                        const double flag = !ok ? 1.0 + GSLAM_STOP_TIMEOUT : pq == 0.0 ? 1.0 + GSLAM_STOP_PQ_ZERO : 0.0;
-                        if (lane < C)
-                            cl_st_async2(cl_mapa(cl_smem_u32(&s_step[0]), lane), s_rz / pq, flag, cl_mapa(b_pq, lane));
-                    }
-                    ok = cl_wait(b_pq, k & 1, P.spin_limit);
-                    if (lane == 0 && ok) arm(b_pq, bytes_pq);
-                    if (lane == 0) {
-                        s_alpha = s_step[0].x;
-                        s_flag_pq = ok ? (int)s_step[0].y : 1 + GSLAM_STOP_TIMEOUT;
-                    }
-                } else {
                 double pq = sum_slices([&](int c) { return s_part[c]; });
                 if (!ONE) {
                     if (lane < C) cl_st_async(cl_mapa(cl_smem_u32(&s_all[rank]), lane), pq, cl_mapa(b_pq, lane));
@@ -520,7 +436,6 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
                     if (!ok) s_flag_pq = 1 + GSLAM_STOP_TIMEOUT;
                     else if (pq == 0.0) s_flag_pq = 1 + GSLAM_STOP_PQ_ZERO;
                     s_alpha = s_rz / pq;
-                }
                 }
             } else {
                 cl_bar_arrive(1, blockDim.x);
@@ -555,18 +470,8 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
             if (warp == 0) {
                 cl_bar_sync(2, blockDim.x);
                 double2 t;
-                if (ORD)
-                    step_rz([&](double rz, double rr) {
-                        const double b = rz / s_rz;
-                        __syncwarp();
-                        if (lane == 0) {
-                            s_rz = rz;
-                            s_rr = rr;
-                        }
-                        return make_double2(b, rr < s_limit ? 1.0 + GSLAM_STOP_TOL : 0.0);
-                    }, rest);
-                else total_rz(t, rest);
-                if (!ORD && lane == 0) {
+                total_rz(t, rest);
+                if (lane == 0) {
                     if (!ok) s_flag = 1 + GSLAM_STOP_TIMEOUT;
                     else if (t.y < s_limit) s_flag = 1 + GSLAM_STOP_TOL;
                     s_beta = t.x / s_rz;
@@ -610,19 +515,16 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
 template <typename T, bool BATCH>
 static const void *fn_of(int rows, bool one) {
     if (rows == 1)
-        return one ? (const void *)k_pcg_cluster<T, 1, true, BATCH, false> : (const void *)k_pcg_cluster<T, 1, false, BATCH, false>;
-    return one ? (const void *)k_pcg_cluster<T, 2, true, BATCH, false> : (const void *)k_pcg_cluster<T, 2, false, BATCH, false>;
+        return one ? (const void *)k_pcg_cluster<T, 1, true, BATCH> : (const void *)k_pcg_cluster<T, 1, false, BATCH>;
+    return one ? (const void *)k_pcg_cluster<T, 2, true, BATCH> : (const void *)k_pcg_cluster<T, 2, false, BATCH>;
 }
 
-/* kinds of launches: FP32 batches, FP64 batches, single graphs, single graphs with ordered
- * sums (single graphs have one row per thread) */
+/* kinds of launches: FP32 batches, FP64 batches, single graphs (one row per thread) */
 static const void *cluster_fn(int kind, int rows, bool one) {
     switch (kind) {
     case 0: return fn_of<float, true>(rows, one);
     case 1: return fn_of<double, true>(rows, one);
-    case 2: return one ? (const void *)k_pcg_cluster<double, 1, true, false, false>
-                       : (const void *)k_pcg_cluster<double, 1, false, false, false>;
-    default: return (const void *)k_pcg_cluster<double, 1, false, false, true>;
+    default: return one ? (const void *)k_pcg_cluster<double, 1, true, false> : (const void *)k_pcg_cluster<double, 1, false, false>;
     }
 }
 
@@ -649,15 +551,15 @@ cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jo
     cluster_config(&cfg, at, n_jobs * p.ctas, p.ctas, threads, smem_bytes, st);
     ClusterParams copy = p;
     void *args[] = { &copy };
-    const int kind = fp32 ? 0 : batch ? 1 : p.gather ? 3 : 2;
-    if (kind > 1 && rows_per_thread != 1) return cudaErrorInvalidValue;
+    const int kind = fp32 ? 0 : batch ? 1 : 2;
+    if (kind == 2 && rows_per_thread != 1) return cudaErrorInvalidValue;
     return cudaLaunchKernelExC(&cfg, cluster_fn(kind, rows_per_thread, p.ctas == 1), args);
 }
 
 int pcg_cluster_max_ctas(int device, size_t smem_bytes) {
     (void)device;
     int best = 0;
-    for (int v = 0; v < 16; v++) {
+    for (int v = 0; v < 12; v++) {
         const void *fn = cluster_fn(v >> 2, 1 + (v & 1), (v & 2) != 0);
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess ||
             cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {

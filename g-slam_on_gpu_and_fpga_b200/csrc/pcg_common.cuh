@@ -8,8 +8,11 @@
 #include "gslam.h"
 #include "kernels.cuh"
 
-/* largest dynamic shared memory the resident solver asks for (sm_100: 227 KB per block) */
+/* largest dynamic shared memory a solver's CTA asks for (sm_100: 227 KB per block with the
+ * static part): the cluster solver's, and the grid-wide ones', whose reductions keep up to
+ * 5 KB of static shared memory */
 #define GSLAM_RES_SMEM_MAX (225 * 1024)
+#define GSLAM_GRID_SMEM_MAX (222 * 1024)
 
 __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned *p) {
     unsigned v;
@@ -155,39 +158,6 @@ __device__ __forceinline__ bool grid_reduce_arrive(const double (&v)[NV], double
     return *s_ok != 0;
 }
 
-/* the partial loads of grid_reduce_sum alone (warps < NV), so a caller can issue them
- * ahead of its own loads and finish with grid_reduce_sum_finish */
-template <int NV>
-__device__ __forceinline__ void grid_reduce_sum_issue(const double *partials_base, int epoch,
-                                                      double (&t)[GSLAM_SUM_UNROLL]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp >= NV) return;
-    const int G = (int)gridDim.x;
-    const double *pp = partials_base + ((epoch - 1) & 1) * 4 * G + warp * G;
-#pragma unroll
-    for (int u = 0; u < GSLAM_SUM_UNROLL; u++) {
-        const int c = lane + 32 * u;
-        t[u] = c < G ? __ldcg(pp + c) : 0.0;
-    }
-}
-
-template <int NV>
-__device__ __forceinline__ void grid_reduce_sum_finish(const double *partials_base, int epoch,
-                                                       const double (&t)[GSLAM_SUM_UNROLL], double *s_bc) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp >= NV) return;
-    const int G = (int)gridDim.x;
-    const double *pp = partials_base + ((epoch - 1) & 1) * 4 * G + warp * G;
-    double s = t[0];
-#pragma unroll
-    for (int u = 1; u < GSLAM_SUM_UNROLL; u++) s = s + t[u];
-    for (int c = lane + 32 * GSLAM_SUM_UNROLL; c < G; c += 32) s = s + __ldcg(pp + c);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s = s + __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) s_bc[warp] = s;
-    if (NV > 1) asm volatile("bar.sync 1, %0;" ::"r"(NV * 32) : "memory");
-}
-
 template <int NV>
 __device__ __forceinline__ void grid_reduce_sum(const double *partials_base, int epoch, double *s_bc) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -228,6 +198,142 @@ __device__ __forceinline__ bool grid_allreduce(double (&v)[NV], double *partials
     return true;
 }
 
+/*
+ * The same all-reduce without a barrier counter and without fences. Every value travels with
+ * its reduction's number: 16 bytes holding the two halves of a double, each beside the
+ * number, written by one 128-bit exchange and polled with 128-bit loads, so a reader that
+ * sees the number has the data, and one trip through L2 replaces the counter's three (the
+ * release that waits for the partials, the counter, the partials). 148 CTAs x 768 threads,
+ * two doubles: 2.40 us with grid_reduce_*, 1.41 with this (one double 1.27; x 384 threads
+ * 1.25). Plain stores instead of the exchange, or a mailbox per reader, take 2.1 to 4.6 us:
+ * many readers of a line slow the writes to it. That also holds for readers that poll
+ * before the data can be there (1.69 us when they poll at once), so the first poll waits
+ * TAG_DELAY cycles after the CTA's own value left: the trip's length and part of the CTAs'
+ * skew. Resident FP64 solver, us per iteration at 20,000 / 50,000 / 100,000 poses: no wait
+ * 4.40 / 5.07 / 6.95, 400 cycles 4.12 / 4.76 / 6.80, 600 3.78 / 4.45 / 6.53, 700 3.70 / 4.37
+ * / 6.39, 800 3.82 / 4.36 / 6.31, 1000 4.04 / 4.52 / 6.49. Later polls follow at once (a gap
+ * of 150 cycles between them costs 0.1 us).
+ *
+ * The slots are zeroed before every launch; number 1 is the first reduction. Two buffers
+ * alternate: a CTA writes number n + 2 only after it has read every CTA's n + 1, which each
+ * of them sent after it had read every n.
+ *
+ * Sums are those of grid_reduce_*, bit for bit: the warps' tree, then the CTAs lane-strided,
+ * then the tree over the lanes.
+ */
+#define TAG_DELAY 750
+#define TAG_VALUES 4 /* values of one reduction */
+
+struct TagWord {
+    unsigned long long a, b;
+};
+
+__device__ __forceinline__ void tag_exch(TagWord *p, double v, unsigned tag) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
+    const unsigned long long a = (bits & 0xffffffffull) | t, b = (bits >> 32) | t;
+    asm volatile("{\n .reg .b128 q, r;\n mov.b128 q, {%1, %2};\n atom.relaxed.gpu.global.exch.b128 r, [%0], q;\n}\n" ::"l"(p),
+                 "l"(a), "l"(b)
+                 : "memory");
+}
+__device__ __forceinline__ void tag_store(TagWord *p, unsigned long long a, unsigned long long b) {
+    asm volatile("{\n .reg .b128 q;\n mov.b128 q, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], q;\n}\n" ::"l"(p), "l"(a), "l"(b)
+                 : "memory");
+}
+__device__ __forceinline__ TagWord tag_load(const TagWord *p) {
+    TagWord r;
+    asm volatile("{\n .reg .b128 q;\n ld.relaxed.gpu.global.b128 q, [%2];\n mov.b128 {%0, %1}, q;\n}\n"
+                 : "=l"(r.a), "=l"(r.b)
+                 : "l"(p)
+                 : "memory");
+    return r;
+}
+
+/* whether a poll that has failed `n` times must be given up: this wait's time is over (then
+ * every other wait's is too), or another wait gave up */
+__device__ __forceinline__ bool tag_give_up(GridSync *gs, int n, long long t0, long long limit) {
+    if ((n & 15) != 15) return false;
+    if (ld_relaxed_s32(&gs->abort)) return true;
+    if (clock64() - t0 <= limit) return false;
+    atomicExch(&gs->abort, 1);
+    return true;
+}
+
+/* sums of v[][] over the CTA and their way to the slots: by warps 0 .. NV - 1, one value
+ * each, after a CTA barrier. v[i][j]: value i of the thread's j-th row; the warp's rows are
+ * slices warp and warp + BS / 32, and the CTA's tree runs over its slices. tag: the
+ * reduction's number. */
+template <int NV, int R, int BS>
+__device__ __forceinline__ void tag_reduce_send(const double (&v)[NV][R], TagWord *slots, unsigned tag,
+                                                double (*s_red)[32]) {
+    static_assert(NV <= TAG_VALUES && R * BS / 32 <= 32, "reduction shape");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double a[NV][R];
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+#pragma unroll
+        for (int j = 0; j < R; j++) a[i][j] = v[i][j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < NV; i++)
+#pragma unroll
+            for (int j = 0; j < R; j++) a[i][j] = a[i][j] + __shfl_down_sync(0xffffffffu, a[i][j], o);
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < NV; i++)
+#pragma unroll
+            for (int j = 0; j < R; j++) s_red[i][warp + j * (BS / 32)] = a[i][j];
+    }
+    __syncthreads();
+    if (warp < NV) {
+        double t = lane < R * BS / 32 ? s_red[warp][lane] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t = t + __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) tag_exch(slots + ((tag & 1) * TAG_VALUES + warp) * gridDim.x + blockIdx.x, t, tag);
+    }
+}
+
+/* the totals into s_bc[], for thread 0 (and whoever passes a CTA barrier after it); *s_ok = 0
+ * when a wait gave up. Five warps per value poll one slot a lane (a grid of more than 160
+ * CTAs: several in turn) into s_slot, and the value's first warp adds them. (One warp per
+ * value with five slots a lane needs 30 registers in every thread of the kernel: 400 bytes
+ * of spills in a 768-thread CTA.) */
+#define TAG_WARPS 5
+#define TAG_LANES (32 * TAG_WARPS)
+
+template <int NV, int BS>
+__device__ __forceinline__ void tag_reduce_sum(const TagWord *slots, unsigned tag, GridSync *gs, long long spin_limit,
+                                               double (*s_slot)[TAG_LANES], double *s_bc, int *s_ok) {
+    static_assert(TAG_WARPS * NV <= BS / 32, "polling warps");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp >= TAG_WARPS * NV) return;
+    const int G = (int)gridDim.x, v = warp / TAG_WARPS, l = threadIdx.x - v * TAG_LANES;
+    const TagWord *p = slots + ((tag & 1) * TAG_VALUES + v) * G;
+    const long long t0 = clock64();
+    while (clock64() - t0 < TAG_DELAY) {}
+    double sum = 0.0;
+    for (int c = l; c < G; c += TAG_LANES) {
+        TagWord w = tag_load(p + c);
+        for (int n = 0; (unsigned)(w.a >> 32) != tag || (unsigned)(w.b >> 32) != tag; n++) {
+            if (tag_give_up(gs, n, t0, spin_limit)) { *s_ok = 0; break; }
+            w = tag_load(p + c);
+        }
+        const double d = __longlong_as_double((long long)((w.a & 0xffffffffull) | w.b << 32));
+        sum = c == l ? d : sum + d;
+    }
+    s_slot[v][l] = sum;
+    asm volatile("bar.sync 1, %0;" ::"r"(NV * TAG_LANES) : "memory");
+    if (warp < NV) {
+        double t = s_slot[warp][lane];
+#pragma unroll
+        for (int u = 1; u < TAG_WARPS; u++) t = t + s_slot[warp][lane + 32 * u];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t = t + __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) s_bc[warp] = t;
+        if (NV > 1) asm volatile("bar.sync 2, %0;" ::"r"(NV * 32) : "memory");
+    }
+}
+
 struct V3 { double a, b, c; };
 
 __device__ __forceinline__ V3 ld3(const double *v4, int row) {
@@ -254,6 +360,42 @@ __device__ __forceinline__ V3 ldg3(const double *v4, int row) {
 __device__ __forceinline__ void st3(double *v4, int row, V3 v) {
     *reinterpret_cast<double2 *>(v4 + 4 * (size_t)row) = make_double2(v.a, v.b);
     v4[4 * (size_t)row + 2] = v.c;
+}
+
+/* a row of three doubles published for the CTAs that read it, with the number of the
+ * iteration it belongs to in both halves (32 bytes: a double, the next one's low word and
+ * the number; its high word and the number, a double) */
+__device__ __forceinline__ void tag_row_store(double *v4, int row, V3 v, unsigned tag) {
+    TagWord *p = reinterpret_cast<TagWord *>(v4 + 4 * (size_t)row);
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v.b), t = (unsigned long long)tag << 32;
+    tag_store(p, (unsigned long long)__double_as_longlong(v.a), (b & 0xffffffffull) | t);
+    tag_store(p + 1, (b >> 32) | t, (unsigned long long)__double_as_longlong(v.c));
+}
+/* reads such a row, waiting for the number; false (the row unknown) when the wait gave up */
+__device__ __forceinline__ bool tag_row_load(const double *v4, int row, unsigned tag, GridSync *gs, long long spin_limit,
+                                             V3 *v) {
+    const TagWord *p = reinterpret_cast<const TagWord *>(v4 + 4 * (size_t)row);
+    const long long t0 = clock64();
+    for (int n = 0;; n++) {
+        const TagWord a = tag_load(p), b = tag_load(p + 1);
+        if ((unsigned)(a.b >> 32) == tag && (unsigned)(b.a >> 32) == tag) {
+            *v = V3{ __longlong_as_double((long long)a.a),
+                     __longlong_as_double((long long)((a.b & 0xffffffffull) | b.a << 32)), __longlong_as_double((long long)b.b) };
+            return true;
+        }
+        if (tag_give_up(gs, n, t0, spin_limit)) return false;
+    }
+}
+
+/* the smallest number whose rounded square root is not below tol, so that
+ * rr < square_limit(tol) decides as sqrt(rr) < tol does (sqrt is monotonic and correctly
+ * rounded) without a square root on the critical path */
+__device__ __forceinline__ double square_limit(double tol) {
+    double y = tol * tol;
+    for (int i = 0; i < 8 && sqrt(y) < tol; i++) y = __longlong_as_double(__double_as_longlong(y) + 1);
+    for (int i = 0; i < 8 && y > 0.0 && sqrt(__longlong_as_double(__double_as_longlong(y) - 1)) >= tol; i++)
+        y = __longlong_as_double(__double_as_longlong(y) - 1);
+    return y;
 }
 
 /* p_new = z + beta * p_old exactly as MatrixOps.c:382 (first iteration: p = z). */

@@ -1,6 +1,7 @@
 """The solver of a graph inside one thread-block cluster (pcg_cluster.cu) against the
 grid-wide solvers on the same graphs, at the sizes where its split changes: one CTA (up to
-13 slices of 32 rows), 2 to 16 CTAs, one and two rows per thread, graphs that do not fit.
+13 slices of 32 rows), 2 to 16 CTAs, 144 slices and one more, and in a batch one and two
+rows per thread and graphs that do not fit.
 
 test_absent_cta beyond every grid is no CTA at all, but it names a CTA that no cluster has,
 so such a handle runs the grid-wide solver. Both solvers take the same PCG iterates; above
@@ -59,7 +60,7 @@ def test_one_cta_gives_the_grid_solvers_bits(pkg, synth, kind, n):
     assert_bitwise(xa, xb, f"{kind} n={n}")
 
 
-@pytest.mark.parametrize("n", [417, 449, 1025, 2049, 5000, 10240, 10241])
+@pytest.mark.parametrize("n", [417, 449, 1025, 2049, 4608, 4609])
 @pytest.mark.parametrize("kind", ["se2", "far", "log"])
 def test_cluster_takes_the_grid_solvers_iterates(pkg, synth, kind, n):
     opts = dict(tol=0.0, max_iter=60)
@@ -141,7 +142,7 @@ def test_batch_options_still_shape_the_solve(pkg, synth):
         b.close()
 
 
-@pytest.mark.parametrize("n", [450, 2500, 10240])
+@pytest.mark.parametrize("n", [300, 450, 2500])
 def test_adjoint_keeps_the_grid_solvers_bits(pkg, synth, n):
     """The exact Hessian can be indefinite, where two orders of the sums end far apart (4e-3
     of mu measured at 800 poses): the adjoint's sums keep the grid-wide solver's order."""
