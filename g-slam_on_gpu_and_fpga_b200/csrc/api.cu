@@ -210,16 +210,15 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
     L->n_sm = n_sm;
     L->partial_capacity = std::max(L->grid, maxg);
     /* resident solvers: contiguous slice ranges per CTA balanced by slot count, at most
-     * one slice per warp; the FP64 solver stages FP64 values, the mixed solver FP32
-     * values plus its own rows' D^-1 and halo, each up to the shared-memory budget */
+     * two slices per warp; the FP64 solvers stage FP64 values, the mixed solver FP32
+     * values, each up to the shared-memory budget */
     L->resident = false;
     L->mixed_ok = false;
     L->cg_ok = false;
-    const int rgrid = std::min(pcg_resident_max_grid(device, GSLAM_GRID_SMEM_MAX),
-                               pcg_mixed_max_grid(device, GSLAM_RES_SMEM_MAX));
+    const int rgrid = std::min({ pcg_resident_max_grid(device, GSLAM_GRID_SMEM_MAX), pcg_mixed_max_grid(device, GSLAM_GRID_SMEM_MAX),
+                                 TAG_LANES });
     if (!batch && rgrid > 0 && S.n_slices <= 32 * rgrid) {
-        const int block = (S.n_slices <= 24 * rgrid) ? 768 : 1024;
-        const int cap_sl = block / 32;          /* one slice per warp */
+        const int cap_sl = S.n_slices <= 24 * rgrid ? 24 : 32;
         /* contiguous slice ranges of at most cap_sl slices that minimise the largest
          * slot count of any CTA (the slowest CTA sets the pace of every iteration):
          * binary search on that bound, each probe a greedy fill; feasible at the
@@ -257,7 +256,6 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
             if (cs[i + 1] < cs[i] || cs[i + 1] - cs[i] > cap_sl) ok = false;
         if (ok) {
             L->res_grid = rgrid;
-            L->res_block = block;
             for (int i = 0; i < rgrid; i++) L->res_slices = std::max(L->res_slices, cs[i + 1] - cs[i]);
             CK(dupload(m, st, &L->cta_slice, cs));
             L->partial_capacity = std::max(L->partial_capacity, rgrid);
@@ -265,8 +263,22 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
             std::vector<int> lcol(S.n_slots, 0), hptr(rgrid + 1, 0), hrows;
             /* mixed / FP64 one-reduction solvers: every CTA's own layout must fit */
             bool fit32 = true, fit64 = true, fit_res = true;
-            std::vector<int> keep(S.n_slices, 0), pos(S.n_slices, 0);
-            int64_t cap32_min = INT64_MAX, cap64_min = INT64_MAX, cap_res_min = INT64_MAX;
+            std::vector<int> keep[3], pos[3]; /* FP64 resident, mixed, one-reduction */
+            for (int v = 0; v < 3; v++) {
+                keep[v].assign(S.n_slices, 0);
+                pos[v].assign(S.n_slices, 0);
+            }
+            /* block positions (288 values of a slice) that do not fit are left out evenly: the
+             * last one of every slice of the CTA, then of every slice that still has one */
+            auto share = [&](int v, int i, int64_t val_cap) {
+                int64_t out = std::max<int64_t>(0, (9 * (S.slice_ptr[cs[i + 1]] - S.slice_ptr[cs[i]]) -
+                                                    std::max<int64_t>(val_cap, 0)) / 288);
+                for (int sl = cs[i]; sl < cs[i + 1]; sl++) keep[v][sl] = (int)((S.slice_ptr[sl + 1] - S.slice_ptr[sl]) / 32);
+                while (out > 0)
+                    for (int sl = cs[i]; sl < cs[i + 1] && out > 0; sl++)
+                        if (keep[v][sl] > 0) { keep[v][sl]--; out--; }
+                for (int sl = cs[i] + 1; sl < cs[i + 1]; sl++) pos[v][sl] = pos[v][sl - 1] + keep[v][sl - 1];
+            };
             /* the largest CTA's layout end: the launch asks for no more shared memory than
              * that (shared memory and L1 share the SM's SRAM, and these kernels read D^-1 and
              * row data through L1) */
@@ -289,56 +301,43 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 }
                 hptr[i + 1] = hptr[i] + (int)rem.size();
                 hrows.insert(hrows.end(), rem.begin(), rem.end());
-                const MixedSmem l32 = mixed_smem_layout(4, false, a1 - a0, cs[i + 1] - cs[i], (int64_t)rem.size(), block,
-                                                        GSLAM_RES_SMEM_MAX);
-                const MixedSmem l64 = mixed_smem_layout(8, true, a1 - a0, cs[i + 1] - cs[i], (int64_t)rem.size(), block,
-                                                        GSLAM_RES_SMEM_MAX);
-                const ResidentSmem lr = resident_smem_layout(a1 - a0, cs[i + 1] - cs[i], (int64_t)rem.size(),
-                                                             GSLAM_GRID_SMEM_MAX);
+                const int64_t nh = (int64_t)rem.size(), nsl = cs[i + 1] - cs[i];
+                const MixedSmem l32 = mixed_smem_layout(4, a1 - a0, nsl, nh, GSLAM_GRID_SMEM_MAX);
+                const MixedSmem l64 = mixed_smem_layout(8, a1 - a0, nsl, nh, GSLAM_GRID_SMEM_MAX);
+                const ResidentSmem lr = resident_smem_layout(a1 - a0, nsl, nh, GSLAM_GRID_SMEM_MAX);
                 fit_res = fit_res && lr.val_cap >= 0;
-                /* positions that do not fit are left out evenly: the last one of every slice,
-                 * then of every slice that still has one, and so on */
-                int64_t out = std::max<int64_t>(0, (9 * (a1 - a0) - std::max<int64_t>(lr.val_cap, 0)) / 288);
-                for (int sl = cs[i]; sl < cs[i + 1]; sl++) keep[sl] = (int)((S.slice_ptr[sl + 1] - S.slice_ptr[sl]) / 32);
-                while (out > 0)
-                    for (int sl = cs[i]; sl < cs[i + 1] && out > 0; sl++)
-                        if (keep[sl] > 0) { keep[sl]--; out--; }
-                for (int sl = cs[i] + 1; sl < cs[i + 1]; sl++) pos[sl] = pos[sl - 1] + keep[sl - 1];
-                cap_res_min = std::min(cap_res_min, std::min<int64_t>(lr.val_cap, 9 * (a1 - a0)));
                 fit32 = fit32 && l32.val_cap >= 0;
                 fit64 = fit64 && l64.val_cap >= 0;
+                share(0, i, lr.val_cap);
+                share(1, i, l32.val_cap);
+                share(2, i, l64.val_cap);
                 end_res = std::max(end_res, lr.end);
                 end32 = std::max(end32, l32.end);
                 end64 = std::max(end64, l64.end);
-                cap32_min = std::min(cap32_min, std::min<int64_t>(l32.val_cap, 9 * (a1 - a0)));
-                cap64_min = std::min(cap64_min, std::min<int64_t>(l64.val_cap, 9 * (a1 - a0)));
             }
-            /* FP64: values | local columns | staged p (32 B per own or halo row), each CTA's
+            /* FP64: values | local columns | staged p (24 B per own or halo row), each CTA's
              * from its own sizes (resident_smem_layout) */
             if (fit_res && !o.disable_resident) {
                 L->resident = true;
-                L->smem_val_cap = cap_res_min; /* the smallest CTA's share (statistics only) */
                 L->smem_bytes = (size_t)end_res;
-                CK(dupload(m, st, &L->res_keep, keep));
-                CK(dupload(m, st, &L->res_pos, pos));
+                CK(dupload(m, st, &L->res_keep, keep[0]));
+                CK(dupload(m, st, &L->res_pos, pos[0]));
                 const int rc = cluster_upload(L, S, st, device, cs);
                 if (rc != GSLAM_OK) return rc;
             }
-            /* mixed: FP32 values | local columns | D^-1 of own rows (2304 B per slice) | z of
-             * own and halo rows (16 B each) | u, v of the first `block` halo rows (32 B each,
-             * copied in asynchronously); FP64 one-reduction solver: FP64 values | local
-             * columns | z (32 B per row) | u, v (64 B per halo row), D^-1 in global memory
-             * (L2). Each CTA lays its share out from its own sizes (mixed_smem_layout), so a
-             * CTA with a short halo keeps more of its values on chip. */
+            /* mixed and one-reduction: values | local columns | z of own and halo rows | v of
+             * halo rows, each CTA's from its own sizes (mixed_smem_layout) */
             if (fit32) {
                 L->mixed_ok = true;
-                L->mixed_val_cap = cap32_min; /* the smallest CTA's share (statistics only) */
                 L->mixed_smem_bytes = (size_t)end32;
+                CK(dupload(m, st, &L->mixed_keep, keep[1]));
+                CK(dupload(m, st, &L->mixed_pos, pos[1]));
             }
             if (fit64) {
                 L->cg_ok = true;
-                L->cg_val_cap = cap64_min;
                 L->cg_smem_bytes = (size_t)end64;
+                CK(dupload(m, st, &L->cg_keep, keep[2]));
+                CK(dupload(m, st, &L->cg_pos, pos[2]));
             }
             if (L->resident || L->mixed_ok || L->cg_ok) {
                 CK(dupload(m, st, &L->lcol, lcol));
@@ -438,12 +437,6 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
         return GSLAM_ERR_TOO_LARGE;
     }
     if (cg) {
-        if (!L->w4) {
-            const size_t nvec = 4 * 32 * (size_t)L->n_slices;
-            CK(dalloc(L->mem, &L->w4, nvec));
-            CK(cudaMemsetAsync(L->w4, 0, nvec * sizeof(double), st));
-        }
-        P.w4 = L->w4;
         /* one inner solve to the outer tolerance and iteration cap, no refinement */
         P.inner_tol = o.tol;
         P.inner_max_iter = o.max_iter;
@@ -464,19 +457,27 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
         }
     }
     P.cta_slice = L->cta_slice;
-    P.smem_val_cap = L->smem_val_cap;
     /* every CTA lays its share out against the full budget, as the host's check did; the
      * launch asks for the largest resulting layout */
-    P.smem_budget = resident ? GSLAM_GRID_SMEM_MAX : GSLAM_RES_SMEM_MAX;
+    P.smem_budget = GSLAM_GRID_SMEM_MAX;
     P.lcol = L->lcol;
     P.halo_ptr = L->halo_ptr;
     P.halo_rows = L->halo_rows;
     P.row_export = L->row_export;
     P.res_keep = L->res_keep;
     P.res_pos = L->res_pos;
+    P.mixed_keep = L->mixed_keep;
+    P.mixed_pos = L->mixed_pos;
+    P.cg_keep = L->cg_keep;
+    P.cg_pos = L->cg_pos;
     tr.step("memsets");
     /* published rows carry their iteration's number: none may be left from an earlier solve */
-    if (resident && !cluster) CK(cudaMemsetAsync(L->z4, 0, 4 * 32 * (size_t)L->n_slices * sizeof(double), st));
+    const size_t vec = 4 * 32 * (size_t)L->n_slices;
+    if (resident && !cluster) CK(cudaMemsetAsync(L->z4, 0, vec * sizeof(double), st));
+    if (mixed || cg) {
+        void *u[2] = { mixed ? (void *)P.zf4 : (void *)P.p4b, mixed ? (void *)P.pfa4 : (void *)P.p4a };
+        for (void *q : u) CK(cudaMemsetAsync(q, 0, vec * (mixed ? sizeof(float) : sizeof(double)), st));
+    }
     CK(record_event(L->ev0, st));
     if (cluster) {
         ClusterParams Q;
@@ -504,8 +505,8 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
         Q.smem_budget = GSLAM_RES_SMEM_MAX;
         Q.res = L->res;
         CK(launch_pcg_cluster(st, Q, 1, L->cluster_threads, L->cluster_rows, L->cluster_smem, false, false));
-    } else if (mixed) CK(launch_pcg_mixed(st, P, grid, L->res_block, L->mixed_smem_bytes, false));
-    else if (cg) CK(launch_pcg_mixed(st, P, grid, L->res_block, L->cg_smem_bytes, true));
+    } else if (mixed) CK(launch_pcg_mixed(st, P, grid, L->res_slices, L->mixed_smem_bytes, false));
+    else if (cg) CK(launch_pcg_mixed(st, P, grid, L->res_slices, L->cg_smem_bytes, true));
     else if (resident) CK(launch_pcg_resident(st, P, grid, L->res_slices, L->smem_bytes));
     else CK(launch_pcg(st, P, fused_prec, grid, L->block));
     tr.step("solver launch");

@@ -41,19 +41,18 @@ struct DevLayout {
     int partial_capacity = 0;
     /* shared-memory-resident solver (pcg_resident.cu), when the layout fits */
     bool resident = false;
-    int res_grid = 0, res_block = 0;
+    int res_grid = 0;
     int res_slices = 0;            /* slices of the CTA that owns most */
-    int *res_keep = nullptr, *res_pos = nullptr; /* per slice: block positions in shared memory, and where */
+    /* per slice: block positions in shared memory, and where (FP64 resident, mixed, one-reduction) */
+    int *res_keep = nullptr, *res_pos = nullptr, *mixed_keep = nullptr, *mixed_pos = nullptr, *cg_keep = nullptr,
+        *cg_pos = nullptr;
     int *cta_slice = nullptr;      /* [res_grid + 1] */
-    int64_t smem_val_cap = 0;      /* doubles staged by the CTA that stages fewest */
     int *lcol = nullptr, *halo_ptr = nullptr, *halo_rows = nullptr; /* CTA-local columns, halo lists */
     unsigned char *row_export = nullptr; /* rows some other CTA's halo lists */
     size_t smem_bytes = 0;
     bool mixed_ok = false;          /* the mixed solver's shared-memory layout fits */
-    int64_t mixed_val_cap = 0;     /* floats staged by the CTA that stages fewest */
     size_t mixed_smem_bytes = 0;   /* dynamic shared memory per launch: the largest CTA layout (mixed_smem_layout) */
     bool cg_ok = false;             /* the FP64 one-reduction solver's layout fits */
-    int64_t cg_val_cap = 0;        /* doubles staged by the CTA that stages fewest */
     size_t cg_smem_bytes = 0;
     /* cluster solver (pcg_cluster.cu), when the graph fits one thread-block cluster */
     bool cluster_ok = false;
@@ -62,7 +61,6 @@ struct DevLayout {
     ClusterJob *cluster_job = nullptr;
     int *cluster_bounds = nullptr, *cluster_halo = nullptr, *cluster_lcol = nullptr, *cluster_exp_ptr = nullptr;
     unsigned *cluster_exp = nullptr;
-    double *w4 = nullptr;          /* its sixth published vector (made on first use) */
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;   /* brackets the solver launch */
     int max_grid_alloc() const { return partial_capacity; }
 };

@@ -65,7 +65,6 @@ struct PcgParams {
     const double *dinv;    /* block-Jacobi inverses (slot layout) */
     const double *b4;      /* right-hand side, padded new order */
     double *x4, *r4, *z4, *p4a, *p4b, *q4;  /* FP64 work vectors */
-    double *w4;            /* FP64 one-reduction solver: its sixth published vector */
     float *xf4, *rf4, *zf4, *pfa4, *pfb4, *qf4; /* FP32 work vectors (mixed) */
     double tol_rel;
     int max_iter;
@@ -79,11 +78,11 @@ struct PcgParams {
     long long spin_limit;  /* clock cycles a barrier may wait */
     int absent_cta;        /* test hook: CTA that leaves before its first barrier, -1 = none */
     const int *cta_slice;  /* resident solver: [grid + 1] first slice of each CTA */
-    int64_t smem_val_cap;  /* resident solvers: the smallest CTA's staged values (statistics only) */
     const int *lcol;       /* resident solver: per slot, CTA-local column index (own rows, then halo) */
     const int *halo_ptr;   /* resident solver: [grid + 1] halo list bounds per CTA */
     const int *halo_rows;  /* resident solver: halo rows (new row indices) */
     const unsigned char *row_export; /* 1 for rows in another CTA's halo: only those are published */
+    const int *mixed_keep, *mixed_pos, *cg_keep, *cg_pos; /* the same for the mixed and the one-reduction solver */
     const int *res_keep, *res_pos; /* resident solver, per slice: block positions kept in shared memory, and the
                             * first one's place there (in positions of 288 values) */
     int64_t smem_budget;   /* resident, mixed and FP64 one-reduction solvers: dynamic shared memory per CTA */
@@ -110,29 +109,26 @@ __host__ __device__ inline ResidentSmem resident_smem_layout(int64_t n_slots, in
 }
 
 /* Shared-memory layout of one CTA of the mixed / FP64 one-reduction solver, from its own
- * sizes: the fixed parts (local columns, D^-1 of own rows when staged, z of own and halo
- * rows, the halo's u and v for the first `block` halo rows) after the values, and as many
- * values (whole multiples of 288, one block position of a slice) as the budget leaves.
- * val_cap < 0: the fixed parts alone exceed the budget. */
+ * sizes: the fixed parts (local columns, z of own and halo rows, v of halo rows: 16 bytes a
+ * row in FP32, 24 in FP64) after the values, and as many values (whole multiples of 288, one
+ * block position of a slice) as the budget leaves. val_cap < 0: the fixed parts alone exceed
+ * the budget. */
 struct MixedSmem {
-    int64_t val_cap, col_off, dinv_off, halo_off, stage_off, end;
+    int64_t val_cap, col_off, z_off, v_off, end;
 };
-__host__ __device__ inline MixedSmem mixed_smem_layout(int64_t elem, bool fp64, int64_t n_slots, int64_t n_slices,
-                                                       int64_t n_halo, int64_t block, int64_t budget) {
+__host__ __device__ inline MixedSmem mixed_smem_layout(int64_t elem, int64_t n_slots, int64_t n_slices, int64_t n_halo,
+                                                       int64_t budget) {
     auto up = [](int64_t b) { return (b + 127) / 128 * 128; };
-    const int64_t col_b = up(4 * n_slots);
-    const int64_t dinv_b = fp64 ? 0 : 2304 * n_slices;
-    const int64_t z_b = up(4 * elem * (32 * n_slices + n_halo));
-    const int64_t stage_b = up(8 * elem * (n_halo < block ? n_halo : block));
+    const int64_t row_b = elem == 8 ? 24 : 16;
+    const int64_t col_b = up(4 * n_slots), z_b = up(row_b * (32 * n_slices + n_halo)), v_b = up(row_b * n_halo);
     MixedSmem m;
-    const int64_t fixed = col_b + dinv_b + z_b + stage_b;
+    const int64_t fixed = col_b + z_b + v_b;
     m.val_cap = budget >= fixed ? (budget - fixed) / elem / 288 * 288 : -1;
     const int64_t nv = m.val_cap > 9 * n_slots ? 9 * n_slots : m.val_cap;
     m.col_off = up(elem * (nv > 0 ? nv : 0));
-    m.dinv_off = m.col_off + col_b;
-    m.halo_off = m.dinv_off + dinv_b;
-    m.stage_off = m.halo_off + z_b;
-    m.end = m.stage_off + stage_b;
+    m.z_off = m.col_off + col_b;
+    m.v_off = m.z_off + z_b;
+    m.end = m.v_off + v_b;
     return m;
 }
 
@@ -278,7 +274,7 @@ int pcg_cluster_max_ctas(int device, size_t smem_bytes);
 
 /* Mixed-precision solver (pcg_mixed.cu); fp64: the same kernel as the FP64 one-reduction
  * solver. */
-cudaError_t launch_pcg_mixed(cudaStream_t st, const PcgParams &p, int grid, int block, size_t smem_bytes,
+cudaError_t launch_pcg_mixed(cudaStream_t st, const PcgParams &p, int grid, int max_slices, size_t smem_bytes,
                              bool fp64);
 int pcg_mixed_max_grid(int device, size_t smem_bytes);
 

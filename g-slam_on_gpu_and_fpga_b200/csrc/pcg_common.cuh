@@ -198,6 +198,42 @@ __device__ __forceinline__ bool grid_allreduce(double (&v)[NV], double *partials
     return true;
 }
 
+/* grid_allreduce of R values per thread: the warp's rows are slices warp and warp + BS / 32,
+ * and the CTA's tree runs over its slices (the same sums as one row per thread) */
+template <int NV, int R, int BS>
+__device__ __forceinline__ bool grid_allreduce_rows(const double (&v)[NV][R], double (&tot)[NV], double *partials_base,
+                                                    int &epoch, GridSync *gs, long long spin_limit, double (*s_red)[32],
+                                                    double *s_bc, int *s_ok) {
+    static_assert(NV <= 4 && R * BS / 32 <= 32, "reduction shape");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *partials = partials_base + (epoch & 1) * 4 * gridDim.x;
+    epoch++;
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            double a = v[i][j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a = a + __shfl_down_sync(0xffffffffu, a, o);
+            if (lane == 0) s_red[i][warp + j * (BS / 32)] = a;
+        }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            double a = lane < R * BS / 32 ? s_red[i][lane] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a = a + __shfl_down_sync(0xffffffffu, a, o);
+            if (lane == 0) partials[i * gridDim.x + blockIdx.x] = a;
+        }
+        if (lane == 0) grid_barrier_t0(gs, (unsigned)epoch, spin_limit, s_ok);
+    }
+    __syncthreads();
+    if (!*s_ok) return false;
+    grid_reduce_collect<NV, BS>(tot, partials_base, epoch, s_bc);
+    return true;
+}
+
 /*
  * The same all-reduce without a barrier counter and without fences. Every value travels with
  * its reduction's number: 16 bytes holding the two halves of a double, each beside the
@@ -294,35 +330,39 @@ __device__ __forceinline__ void tag_reduce_send(const double (&v)[NV][R], TagWor
 }
 
 /* the totals into s_bc[], for thread 0 (and whoever passes a CTA barrier after it); *s_ok = 0
- * when a wait gave up. Five warps per value poll one slot a lane (a grid of more than 160
- * CTAs: several in turn) into s_slot, and the value's first warp adds them. (One warp per
- * value with five slots a lane needs 30 registers in every thread of the kernel: 400 bytes
- * of spills in a 768-thread CTA.) */
+ * when a wait gave up. Every slot is polled by a thread of its own, into s_slot, and then one
+ * warp per value adds them: by the first TAG_WARPS * NV warps, which leave the others to the
+ * caller, where the CTA has that many (call it with all threads), else by all. (One warp per
+ * value with five slots a lane needs 30 registers in every thread of the kernel: 400 bytes of
+ * spills in a 768-thread CTA.) A grid has at most TAG_LANES CTAs. */
 #define TAG_WARPS 5
 #define TAG_LANES (32 * TAG_WARPS)
 
 template <int NV, int BS>
 __device__ __forceinline__ void tag_reduce_sum(const TagWord *slots, unsigned tag, GridSync *gs, long long spin_limit,
                                                double (*s_slot)[TAG_LANES], double *s_bc, int *s_ok) {
-    static_assert(TAG_WARPS * NV <= BS / 32, "polling warps");
+    constexpr bool SOME = TAG_WARPS * NV <= BS / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp >= TAG_WARPS * NV) return;
-    const int G = (int)gridDim.x, v = warp / TAG_WARPS, l = threadIdx.x - v * TAG_LANES;
-    const TagWord *p = slots + ((tag & 1) * TAG_VALUES + v) * G;
+    if (SOME && warp >= TAG_WARPS * NV) return;
+    const int G = (int)gridDim.x;
+    const TagWord *p = slots + (tag & 1) * TAG_VALUES * G;
     const long long t0 = clock64();
     while (clock64() - t0 < TAG_DELAY) {}
-    double sum = 0.0;
-    for (int c = l; c < G; c += TAG_LANES) {
-        TagWord w = tag_load(p + c);
-        for (int n = 0; (unsigned)(w.a >> 32) != tag || (unsigned)(w.b >> 32) != tag; n++) {
-            if (tag_give_up(gs, n, t0, spin_limit)) { *s_ok = 0; break; }
-            w = tag_load(p + c);
+    for (int c = threadIdx.x; c < NV * TAG_LANES; c += BS) {
+        const int v = c / TAG_LANES, l = c - v * TAG_LANES;
+        double d = 0.0;
+        if (l < G) {
+            TagWord w = tag_load(p + v * G + l);
+            for (int n = 0; (unsigned)(w.a >> 32) != tag || (unsigned)(w.b >> 32) != tag; n++) {
+                if (tag_give_up(gs, n, t0, spin_limit)) { *s_ok = 0; break; }
+                w = tag_load(p + v * G + l);
+            }
+            d = __longlong_as_double((long long)((w.a & 0xffffffffull) | w.b << 32));
         }
-        const double d = __longlong_as_double((long long)((w.a & 0xffffffffull) | w.b << 32));
-        sum = c == l ? d : sum + d;
+        s_slot[v][l] = d;
     }
-    s_slot[v][l] = sum;
-    asm volatile("bar.sync 1, %0;" ::"r"(NV * TAG_LANES) : "memory");
+    if (SOME) asm volatile("bar.sync 1, %0;" ::"r"(NV * TAG_LANES) : "memory");
+    else __syncthreads();
     if (warp < NV) {
         double t = s_slot[warp][lane];
 #pragma unroll

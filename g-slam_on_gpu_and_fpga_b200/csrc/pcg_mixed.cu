@@ -22,20 +22,28 @@
  *     beta_k = gamma_k / gamma_{k-1};  alpha_k = gamma_k / (delta_k - beta_k gamma_k / alpha_{k-1})
  * (alpha, beta = those of the previous reduction). The SpMV needs z_k of rows
  * other CTAs own, which is only final after the reduction; instead of a second
- * grid barrier every row publishes (z_k, u_k, v_{k-1}) before the reduction and
- * a reader forms v_k and z_{k+1} from them with the same two FP32 FMAs per
- * component the owner uses, so the copies are bit-identical and no reader needs
- * the owner's D^-1.
+ * grid barrier every row that another CTA reads publishes u_k before the
+ * reduction, and its readers keep their own copies of its z and v and take the
+ * owner's two FMAs per component, so the copies are bit-identical and no reader
+ * needs the owner's D^-1. u is published with the iteration's number in the same
+ * 16-byte words, and the sums travel the same way (tag_reduce_*): no fence, no
+ * barrier counter. Two buffers of u alternate: an owner writes u_{k+2} after
+ * reduction k + 1, which every reader enters after it has read u_k.
  *
- * Shared memory holds, per CTA: its FP32 matrix share, CTA-local column indices
- * (own rows first, then the CTA's halo: the other CTAs' rows its blocks touch, a
- * list fixed at setup), its own rows' D^-1, and z of its own and halo rows. Each
- * thread owns one row and keeps r, z, s, v, w, u, p, d in registers; every thread
- * also advances z of (at least) one halo row per iteration. The halo's published
- * values are loaded right after the grid barrier, while warps 0-2 sum the
- * reduction partials, so the two L2 round trips overlap; thread 0 alone then
- * advances the scalar recurrence. The SpMV reads values, columns and z from
- * shared memory only.
+ * Shared memory holds, per CTA: its matrix share (of a share that does not fit
+ * every slice leaves out its last block positions, read from L2), CTA-local column
+ * indices (own rows first, then the CTA's halo: the other CTAs' rows its blocks
+ * touch, a list fixed at setup), z of its own and halo rows and the halo's v. Each
+ * thread owns one or two rows and keeps r, z, s, v, w, u, p, d in registers, and
+ * D^-1 where they suffice. Thread 0 alone advances the scalar recurrence while the
+ * others fetch the halo's u. The SpMV reads values, columns and z from shared
+ * memory only.
+ *
+ * Measured, us per iteration (before: a barrier counter with a release fence and z, u, v
+ * of every row published), same bits. FP32: 2.7 (4.5) at N = 20,000, 2.9 (4.8) at 50,000,
+ * 4.45 (5.9) at 100,000. FP64: 2.9 (6.2), 3.8 (7.6), 6.3 (11.8). Up to 50,000 the
+ * all-reduce of three doubles (1.5 us) bounds it, at 100,000 the SpMV from shared memory
+ * and, in FP64, D^-1 from L2.
  *
  * Outer step: x += d (FP64), grid barrier, r = xi - Omega x with the FP64 matrix,
  * ||r|| -> stop at tol * ||xi||, else restart the inner solve from r; a step that
@@ -43,9 +51,8 @@
  * solves in FP64).
  *
  * The same kernel with T = double is the FP64 one-reduction solver (GSLAM_PREC_FP64_CG):
- * one inner solve in FP64 (FP64 values staged in shared memory as far as they fit, the
- * rest read from L2; D^-1 read from global memory, where it stays in L2) to the outer
- * tolerance and iteration cap, no refinement. It stops on the recurrence residual, as the
+ * one inner solve in FP64 to the outer tolerance and iteration cap, no refinement. It stops
+ * on the recurrence residual, as the
  * reference's loop does (MatrixOps.c:345-347), and reports the true residual; its
  * iterates are the reference's PCG in exact arithmetic, with other rounding (20
  * Gauss-Newton rounds of a 100k-pose graph at 1e-6 / 500: 9.5e-10 from the reference
@@ -65,14 +72,6 @@
  * (16 B in FP32, 32 B in FP64) */
 template <typename T> struct T3 { T a, b, c; };
 
-__device__ __forceinline__ T3<float> ldt3(const float *v4, int row) {
-    const float4 v = *reinterpret_cast<const float4 *>(v4 + 4 * (size_t)row);
-    return { v.x, v.y, v.z };
-}
-__device__ __forceinline__ T3<double> ldt3(const double *v4, int row) {
-    const V3 v = ld3(v4, row);
-    return { v.a, v.b, v.c };
-}
 __device__ __forceinline__ T3<float> ldcgt3(const float *v4, int row) {
     const float4 v = __ldcg(reinterpret_cast<const float4 *>(v4 + 4 * (size_t)row));
     return { v.x, v.y, v.z };
@@ -86,35 +85,62 @@ __device__ __forceinline__ void stt3(float *v4, int row, T3<float> v) {
 }
 __device__ __forceinline__ void stt3(double *v4, int row, T3<double> v) { st3(v4, row, V3{ v.a, v.b, v.c }); }
 
-/* 16-byte asynchronous global -> shared copy through L2 (no registers), and its wait */
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
+/* a row published for the CTAs that read it, with the iteration's number: FP64 as
+ * tag_row_store, FP32 as one 16-byte word */
+__device__ __forceinline__ void put_row(double *v4, int row, T3<double> v, unsigned tag) {
+    tag_row_store(v4, row, V3{ v.a, v.b, v.c }, tag);
+}
+__device__ __forceinline__ void put_row(float *v4, int row, T3<float> v, unsigned tag) {
+    tag_store(reinterpret_cast<TagWord *>(v4 + 4 * (size_t)row),
+              (unsigned long long)__float_as_uint(v.a) | (unsigned long long)__float_as_uint(v.b) << 32,
+              (unsigned long long)__float_as_uint(v.c) | (unsigned long long)tag << 32);
+}
+__device__ __forceinline__ bool get_row(const double *v4, int row, unsigned tag, GridSync *gs, long long limit, T3<double> *v) {
+    V3 t;
+    if (!tag_row_load(v4, row, tag, gs, limit, &t)) return false;
+    *v = T3<double>{ t.a, t.b, t.c };
+    return true;
+}
+__device__ __forceinline__ bool get_row(const float *v4, int row, unsigned tag, GridSync *gs, long long limit, T3<float> *v) {
+    const long long t0 = clock64();
+    for (int n = 0;; n++) {
+        const TagWord w = tag_load(reinterpret_cast<const TagWord *>(v4 + 4 * (size_t)row));
+        if ((unsigned)(w.b >> 32) == tag) {
+            *v = T3<float>{ __uint_as_float((unsigned)w.a), __uint_as_float((unsigned)(w.a >> 32)), __uint_as_float((unsigned)w.b) };
+            return true;
+        }
+        if (tag_give_up(gs, n, t0, limit)) return false;
+    }
 }
 
-__device__ __forceinline__ void cp_async_commit_wait_later() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-/* one padded row of T (4 elements) global -> shared, asynchronously */
-template <typename T>
-__device__ __forceinline__ void cp_async_row(T *smem_dst, const T *gsrc) {
-#pragma unroll
-    for (int c = 0; c < (int)(4 * sizeof(T)) / 16; c++) cp_async16(smem_dst + c * (16 / sizeof(T)), gsrc + c * (16 / sizeof(T)));
-}
+/* z (and v) of own and halo rows in shared memory: FP32 one float4 per row, FP64 three arrays
+ * (a gather of 8 bytes at stride 8 meets fewer bank conflicts than 16 + 8 bytes at stride 32) */
+template <typename T> struct Rows;
+template <> struct Rows<float> {
+    float4 *p;
+    __device__ Rows(unsigned char *at, int) : p(reinterpret_cast<float4 *>(at)) {}
+    __device__ T3<float> get(int i) const { const float4 v = p[i]; return { v.x, v.y, v.z }; }
+    __device__ void put(int i, T3<float> v) const { p[i] = make_float4(v.a, v.b, v.c, 0.f); }
+};
+template <> struct Rows<double> {
+    double *a, *b, *c;
+    __device__ Rows(unsigned char *at, int n) : a(reinterpret_cast<double *>(at)), b(a + n), c(b + n) {}
+    __device__ T3<double> get(int i) const { return { a[i], b[i], c[i] }; }
+    __device__ void put(int i, T3<double> v) const { a[i] = v.a; b[i] = v.b; c[i] = v.c; }
+};
 
 /* a * b + c in one rounding */
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-/* y = D^-1 x in FP64 (the 9 entries of D^-1 at stride 32 doubles), rounded to T. */
+/* y = D^-1 x in FP64 (the nine entries of D^-1), rounded to T. */
 template <typename T>
-__device__ __forceinline__ T3<T> dinv_apply_t(const double *d, T3<T> x) {
+__device__ __forceinline__ T3<T> dinv_apply_t(const double (&d)[9], T3<T> x) {
     const double x0 = x.a, x1 = x.b, x2 = x.c;
     double y0 = 0.0, y1 = 0.0, y2 = 0.0;
-    y0 = y0 + d[0] * x0;   y0 = y0 + d[32] * x1;  y0 = y0 + d[64] * x2;
-    y1 = y1 + d[96] * x0;  y1 = y1 + d[128] * x1; y1 = y1 + d[160] * x2;
-    y2 = y2 + d[192] * x0; y2 = y2 + d[224] * x1; y2 = y2 + d[256] * x2;
+    y0 = y0 + d[0] * x0; y0 = y0 + d[1] * x1; y0 = y0 + d[2] * x2;
+    y1 = y1 + d[3] * x0; y1 = y1 + d[4] * x1; y1 = y1 + d[5] * x2;
+    y2 = y2 + d[6] * x0; y2 = y2 + d[7] * x1; y2 = y2 + d[8] * x2;
     return T3<T>{ (T)y0, (T)y1, (T)y2 };
 }
 
@@ -139,30 +165,53 @@ __device__ __forceinline__ void blk_acc_t(const T *v, T3<T> p, T &q0, T &q1, T &
     q2 = fma_t(v[192], p.a, q2); q2 = fma_t(v[224], p.b, q2); q2 = fma_t(v[256], p.c, q2);
 }
 
-/* the inner solve's buffers for T: the matrix copy and the published (z, u, v) of both
- * iteration parities. FP32: the FP32 copy and six FP32 vectors. FP64: the FP64 matrix and
- * six FP64 vectors (r4 .. q4 and w4; x4 holds the solution). */
+/* U blocks of one row with values in shared memory: every load is issued before the first
+ * sum (a shorter row's lane leaves its sums alone) */
+template <int U, typename T>
+__device__ __forceinline__ void mix_blocks(const int *cb, const T *sv, const Rows<T> &sz, int left, T &q0, T &q1, T &q2) {
+    int c[U];
+    T3<T> z[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) c[u] = cb[32 * u];
+#pragma unroll
+    for (int u = 0; u < U; u++) z[u] = sz.get(c[u]);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        T n0 = q0, n1 = q1, n2 = q2;
+        blk_acc_t(sv + 288 * u, z[u], n0, n1, n2);
+        if (u < left) {
+            q0 = n0;
+            q1 = n1;
+            q2 = n2;
+        }
+    }
+}
+
+/* the inner solve's buffers for T: the matrix copy, z at the start of an inner solve, and the
+ * published u of both iteration parities */
 template <typename T> struct Inner;
 template <> struct Inner<float> {
     static __device__ const float *val(const PcgParams &P) { return P.val32; }
-    static __device__ float *pz(const PcgParams &P, int par) { return par ? P.rf4 : P.xf4; }
-    static __device__ float *pu(const PcgParams &P, int par) { return par ? P.pfa4 : P.zf4; }
-    static __device__ float *pv(const PcgParams &P, int par) { return par ? P.qf4 : P.pfb4; }
+    static __device__ float *z0(const PcgParams &P) { return P.rf4; }
+    static __device__ float *u(const PcgParams &P, unsigned par) { return par ? P.pfa4 : P.zf4; }
 };
 template <> struct Inner<double> {
     static __device__ const double *val(const PcgParams &P) { return P.val; }
-    static __device__ double *pz(const PcgParams &P, int par) { return par ? P.r4 : P.z4; }
-    static __device__ double *pu(const PcgParams &P, int par) { return par ? P.p4a : P.p4b; }
-    static __device__ double *pv(const PcgParams &P, int par) { return par ? P.q4 : P.w4; }
+    static __device__ double *z0(const PcgParams &P) { return P.r4; }
+    static __device__ double *u(const PcgParams &P, unsigned par) { return par ? P.p4a : P.p4b; }
 };
 
-/* T = float: the mixed solver; T = double: the FP64 one-reduction solver (one inner
- * solve, D^-1 from global memory) */
-template <int BS, typename T>
+/* T = float: the mixed solver; T = double: the FP64 one-reduction solver (one inner solve).
+ * R: slices per warp (warp w owns slices w and w + BS / 32); DREGS: the rows' D^-1 stay in
+ * registers for the whole solve, else they are read from L2 in every iteration; U: blocks
+ * whose loads are issued together */
+template <int BS, int R, typename T, bool DREGS, int U>
 __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
     constexpr bool F64 = sizeof(T) == 8;
+    constexpr int W = BS / 32;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ double s_red[3][BS / 32];
+    __shared__ double s_red[3][32];
+    __shared__ double s_slot[3][TAG_LANES];
     __shared__ double s_bc[4];
     __shared__ int s_ok;
     __shared__ __align__(8) uint64_t s_bar;
@@ -170,47 +219,54 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
      * other threads): gamma_{k-1}, alpha_{k-1}, rho_0 of the inner solve, tol, ||xi|| */
     __shared__ double s_sc[5];
     __shared__ T s_ab[2];      /* alpha, beta for the next iteration */
-    __shared__ int s_flag;     /* 0 continue, 1 inner solve done, 2 breakdown */
+    __shared__ int s_flag;     /* 0 continue, 1 inner solve done, 2 breakdown, 3 a wait gave up */
     __shared__ int s_conv;     /* the inner solve ended on its residual tolerance */
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int epoch = 0;
+    unsigned seq = 0;          /* inner iterations so far: the number of their reduction and of u */
     if ((int)blockIdx.x == P.absent_cta) return; /* test hook, see pcg.cu */
 
     const int s0 = __ldg(P.cta_slice + blockIdx.x), s1 = __ldg(P.cta_slice + blockIdx.x + 1);
     const int row0 = 32 * s0, n_loc = 32 * (s1 - s0);
     const int64_t slot0 = __ldg(P.slice_ptr + s0), slot1 = __ldg(P.slice_ptr + s1);
     const int64_t nval = 9 * (slot1 - slot0);
-    const int h0 = __ldg(P.halo_ptr + blockIdx.x), h1 = __ldg(P.halo_ptr + blockIdx.x + 1);
+    const int h0 = __ldg(P.halo_ptr + blockIdx.x), n_halo = __ldg(P.halo_ptr + blockIdx.x + 1) - h0;
     /* dynamic shared memory, laid out per CTA from its own sizes (mixed_smem_layout, the
      * host's feasibility check uses the same function): T values as far as they fit |
-     * local columns | D^-1 of own rows (FP32 only) | z of own + halo rows | halo u, v
-     * (8 T per row, the first BS halo rows) */
-    const MixedSmem ml = mixed_smem_layout(sizeof(T), F64, slot1 - slot0, s1 - s0, h1 - h0, BS, P.smem_budget);
+     * local columns | z of own + halo rows | v of halo rows */
+    const MixedSmem ml = mixed_smem_layout(sizeof(T), slot1 - slot0, s1 - s0, n_halo, P.smem_budget);
     const int64_t nsm = nval < ml.val_cap ? nval : ml.val_cap;
     T *sval = reinterpret_cast<T *>(smem);
     int *scol = reinterpret_cast<int *>(smem + ml.col_off);
-    double *sdinv = reinterpret_cast<double *>(smem + ml.dinv_off);
-    T *sz = reinterpret_cast<T *>(smem + ml.halo_off);
-    T *sstage = reinterpret_cast<T *>(smem + ml.stage_off);
+    const Rows<T> sz(smem + ml.z_off, n_loc + n_halo), shv(smem + ml.v_off, n_halo);
 
     if (threadIdx.x == 0) {
         tma_mbar_init(&s_bar, 1);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        s_ok = 1;
     }
     __syncthreads();
+    const int *keep = F64 ? P.cg_keep : P.mixed_keep, *pos = F64 ? P.cg_pos : P.mixed_pos;
     if (threadIdx.x == 0) {
+        /* one copy when every value fits, else one per slice (its kept positions) */
         const unsigned vbytes = (unsigned)(sizeof(T) * nsm), cbytes = (unsigned)(4 * (slot1 - slot0));
-        const unsigned dbytes = F64 ? 0u : (unsigned)(2304 * (s1 - s0));
-        tma_mbar_expect_tx(&s_bar, vbytes + cbytes + dbytes);
-        if (vbytes) tma_bulk_g2s(sval, Inner<T>::val(P) + 9 * slot0, vbytes, &s_bar);
+        tma_mbar_expect_tx(&s_bar, vbytes + cbytes);
         if (cbytes) tma_bulk_g2s(scol, P.lcol + slot0, cbytes, &s_bar);
-        if (dbytes) tma_bulk_g2s(sdinv, P.dinv + 288 * (size_t)s0, dbytes, &s_bar);
-        int ok = tma_wait(&s_bar, 0, P.spin_limit);
-        if (!ok) {
-            atomicExch(&P.gs->abort, 1);
-            tma_wait(&s_bar, 0, P.spin_limit);
+        if (nsm == nval) {
+            if (vbytes) tma_bulk_g2s(sval, Inner<T>::val(P) + 9 * slot0, vbytes, &s_bar);
+        } else {
+            for (int t = s0; t < s1; t++) {
+                const int n = __ldg(keep + t);
+                if (n)
+                    tma_bulk_g2s(sval + 288 * __ldg(pos + t), Inner<T>::val(P) + 9 * __ldg(P.slice_ptr + t),
+                                 (unsigned)(288 * sizeof(T)) * n, &s_bar);
+            }
         }
-        s_ok = ok;
+    }
+    if (!tma_wait(&s_bar, 0, P.spin_limit)) {
+        atomicExch(&P.gs->abort, 1);
+        s_ok = 0;
+        tma_wait(&s_bar, 0, P.spin_limit); /* let the copy finish before the CTA leaves */
     }
     __syncthreads();
     if (!s_ok) {
@@ -218,39 +274,65 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
         return;
     }
 
-    const int s = s0 + warp;
-    const bool own_slice = s < s1;
-    const int row = 32 * s + lane;
-    const bool mine = own_slice && row < P.n_rows;
-    const int len = mine ? __ldg(P.row_len + row) : 0;
-    /* 32-bit offsets into this CTA's share: local slot of (j = 0), and how many of the
-     * row's blocks have their values in shared memory (the rest are read from L2) */
-    const int lslot = own_slice ? (int)(__ldg(P.slice_ptr + s) - slot0) : 0;
-    const int j_sm = min(len, max(0, ((int)nsm - 9 * lslot) / 288));
-    /* the halo row this thread advances every iteration (more, in a loop, only when
-     * the halo has more rows than the CTA has threads) */
-    const bool has_h = (int)threadIdx.x < h1 - h0;
-    const int hrow = has_h ? __ldg(P.halo_rows + h0 + threadIdx.x) : 0;
-    const bool h_extra = h1 - h0 > BS;  /* CTA-uniform */
-
-    /* published (z_k, u_k, v_{k-1}) in global memory, double-buffered by iteration
-     * parity (selected with ?: so no local-memory array is needed) */
-#define PUB_Z(par) Inner<T>::pz(P, par)
-#define PUB_U(par) Inner<T>::pu(P, par)
-#define PUB_V(par) Inner<T>::pv(P, par)
-    /* this thread's own row's D^-1 (stride 32 doubles): staged in shared memory (FP32), or
-     * in global memory, where it stays in L2 (FP64: the shared memory holds values) */
-    const double *my_dinv = F64 ? P.dinv + 288 * (size_t)s + lane : sdinv + 288 * warp + lane;
+    /* ---- this thread's rows ---- */
+    int row[R], len[R], kept[R], lslot[R], spos[R];
+    bool mine[R], pub[R];
+    double d9[DREGS ? R : 1][9];
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int s = s0 + warp + i * W;
+        const bool own = s < s1;
+        row[i] = 32 * s + lane;
+        mine[i] = own && row[i] < P.n_rows;
+        pub[i] = mine[i] && __ldg(P.row_export + row[i]); /* another CTA reads this row */
+        len[i] = mine[i] ? __ldg(P.row_len + row[i]) : 0;
+        lslot[i] = own ? (int)(__ldg(P.slice_ptr + s) - slot0) : 0;
+        /* the slice's block positions with values in shared memory, and where; the last ones,
+         * if they do not all fit, are read from L2 */
+        kept[i] = own ? __ldg(keep + s) : 0;
+        spos[i] = own ? 288 * __ldg(pos + s) : 0;
+        if (DREGS && mine[i]) {
+            const double *g = P.dinv + 288 * (size_t)(row[i] >> 5) + lane;
+#pragma unroll
+            for (int e = 0; e < 9; e++) d9[DREGS ? i : 0][e] = __ldg(g + 32 * e);
+        }
+    }
+    auto precond = [&](int i, T3<T> v) {
+        if (DREGS) return dinv_apply_t<T>(d9[DREGS ? i : 0], v);
+        double d[9];
+        const double *g = P.dinv + 288 * (size_t)(row[i] >> 5) + lane;
+#pragma unroll
+        for (int e = 0; e < 9; e++) d[e] = __ldg(g + 32 * e);
+        return dinv_apply_t<T>(d, v);
+    };
+    /* the halo rows this thread advances, the last threads first (the first warps poll the
+     * sums); further ones, when the halo has more rows than that, at the top of the iteration */
+    const int hh = BS - 1 - (int)threadIdx.x;
+    int hrow[R];
+    T3<T> hu[R];
+    const T3<T> zero = { (T)0, (T)0, (T)0 };
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        hrow[i] = hh + i * BS < n_halo ? __ldg(P.halo_rows + h0 + hh + i * BS) : -1;
+        hu[i] = zero;
+    }
 
     /* ---- ||xi|| ---- */
     double bb[1] = { 0.0 };
-    if (mine) {
-        const V3 b = ldg3(P.b4, row);
-        bb[0] = bb[0] + b.a * b.a; bb[0] = bb[0] + b.b * b.b; bb[0] = bb[0] + b.c * b.c;
-    }
-    if (!grid_allreduce<1, BS>(bb, P.partials, epoch, P.gs, P.spin_limit, s_red, s_bc, &s_ok)) {
-        if (threadIdx.x == 0) res_mark_timeout(P.res);
-        return;
+    {
+        double acc[1][R];
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            acc[0][i] = 0.0;
+            if (mine[i]) {
+                const V3 b = ldg3(P.b4, row[i]);
+                acc[0][i] = acc[0][i] + b.a * b.a; acc[0][i] = acc[0][i] + b.b * b.b; acc[0][i] = acc[0][i] + b.c * b.c;
+            }
+        }
+        if (!grid_allreduce_rows<1, R, BS>(acc, bb, P.partials, epoch, P.gs, P.spin_limit, s_red, s_bc, &s_ok)) {
+            if (threadIdx.x == 0) res_mark_timeout(P.res);
+            return;
+        }
     }
     if (threadIdx.x == 0) {
         const double tol = P.tol_rel * sqrt(bb[0]);
@@ -262,8 +344,8 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
      * other warps waiting for it at a barrier that counts warps */
     __syncthreads();
 
-    V3 x = { 0.0, 0.0, 0.0 };   /* FP64 solution (P.x4 holds it during an inner solve) */
-    V3 r64 = mine ? ldg3(P.b4, row) : V3{ 0.0, 0.0, 0.0 }; /* FP64 residual, = xi for x = 0 */
+    /* FP64 solution (P.x4 holds it during an inner solve) and FP64 residual, = xi for x = 0;
+     * the residual of the row is kept in P.q4 between refinement steps */
     double rnorm = sqrt(bb[0]);
     int total = 0, outer = 0, reason = GSLAM_STOP_MAXIT;
     bool timed_out = false;
@@ -272,135 +354,99 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
         if (rnorm < P.tol_rel * s_sc[4]) { reason = GSLAM_STOP_TOL; break; }
         if (total >= P.max_iter || outer >= P.max_refine) { reason = GSLAM_STOP_MAXIT; break; }
         outer++;
-        /* ---- inner FP32 solve of A d = r64; x += d in FP64 afterwards ---- */
-        if (mine) st3(P.x4, row, x);  /* x is not held in registers during the inner solve */
-        T3<T> r = { (T)r64.a, (T)r64.b, (T)r64.c };
-        const T3<T> zero = { (T)0, (T)0, (T)0 };
-        /* state "k = -1": z_{-1} = D^-1 r_0, and w, u, s, v, p of earlier steps 0, so
-         * with alpha = beta = 0 the first step leaves r and z unchanged; readers of
-         * iteration 0 use parity (0 - 1) & 1 = 1 */
-        T3<T> z = mine ? dinv_apply_t<T>(my_dinv, r) : zero;
-        T3<T> w = zero, u = zero, sv = zero, v = zero, p = zero, d = zero;
-        if (mine) {
-            stt3(PUB_Z(1), row, z);
-            stt3(PUB_U(1), row, zero);
-            stt3(PUB_V(1), row, zero);
+        /* ---- inner solve of A d = r64 in T; x += d in FP64 afterwards ---- */
+        T3<T> r[R], z[R], w[R], u[R], sv[R], v[R], p[R], d[R];
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            r[i] = z[i] = w[i] = u[i] = sv[i] = v[i] = p[i] = d[i] = zero;
+            /* state "k = -1": z_{-1} = D^-1 r_0, and w, u, s, v, p of earlier steps 0, so with
+             * alpha = beta = 0 the first step leaves r and z unchanged */
+            if (mine[i]) {
+                const V3 r64 = outer == 1 ? ldg3(P.b4, row[i]) : ld3(P.q4, row[i]);
+                if (outer == 1) st3(P.x4, row[i], V3{ 0.0, 0.0, 0.0 });
+                r[i] = T3<T>{ (T)r64.a, (T)r64.b, (T)r64.c };
+                z[i] = precond(i, r[i]);
+                if (pub[i]) stt3(Inner<T>::z0(P), row[i], z[i]);
+            }
         }
         if (!grid_barrier(P.gs, (unsigned)(++epoch), P.spin_limit, &s_ok)) { timed_out = true; break; }
-        /* the halo's published (z, u, v) go straight into shared memory (no registers held
-         * across the reduction): z into the halo row's z slot, u and v into staging */
-        if (has_h) {
-            cp_async_row(sz + 4 * (n_loc + threadIdx.x), PUB_Z(1) + 4 * (size_t)hrow);
-            cp_async_row(sstage + 8 * threadIdx.x, PUB_U(1) + 4 * (size_t)hrow);
-            cp_async_row(sstage + 8 * threadIdx.x + 4, PUB_V(1) + 4 * (size_t)hrow);
-            cp_async_commit_wait_later();
+        for (int h = hh; h < n_halo; h += BS) {
+            sz.put(n_loc + h, ldcgt3(Inner<T>::z0(P), __ldg(P.halo_rows + h0 + h)));
+            shv.put(h, zero);
         }
+#pragma unroll
+        for (int i = 0; i < R; i++) hu[i] = zero;
         T alpha = (T)0, beta = (T)0;
         int k = 0;
         while (true) {
-            const int pr = (k - 1) & 1, pw = k & 1;
-            /* z_k of the halo rows (first: frees the prefetched registers) */
-            if (has_h) {
-                cp_async_wait_all();
+            /* z_k of the halo rows, from the owners' u_{k-1} and this CTA's copies of v and z:
+             * the owners' own step, bit for bit */
+            auto halo_step = [&](int h, T3<T> uh) {
                 T3<T> zn, vn;
-                step_zv(ldt3(sz, n_loc + threadIdx.x), ldt3(sstage, 2 * threadIdx.x), ldt3(sstage, 2 * threadIdx.x + 1),
-                        alpha, beta, zn, vn);
-                stt3(sz, n_loc + (int)threadIdx.x, zn);
+                step_zv(sz.get(n_loc + h), uh, shv.get(h), alpha, beta, zn, vn);
+                sz.put(n_loc + h, zn);
+                shv.put(h, vn);
+            };
+#pragma unroll
+            for (int i = 0; i < R; i++)
+                if (hrow[i] >= 0) halo_step(hh + i * BS, hu[i]);
+            for (int h = hh + R * BS; h < n_halo; h += BS) {
+                T3<T> uh = zero;
+                if (k > 0 && !get_row(Inner<T>::u(P, seq & 1), __ldg(P.halo_rows + h0 + h), seq, P.gs, P.spin_limit, &uh)) s_ok = 0;
+                halo_step(h, uh);
             }
-            if (h_extra) {
-                /* halo rows beyond the CTA's thread count (bounds re-read: rare path) */
-                const int e0 = __ldg(P.halo_ptr + blockIdx.x), e1 = __ldg(P.halo_ptr + blockIdx.x + 1);
-                for (int h = e0 + (int)threadIdx.x + BS; h < e1; h += BS) {
-                    const int c = __ldg(P.halo_rows + h);
-                    T3<T> zn, vn;
-                    step_zv(ldcgt3(PUB_Z(pr), c), ldcgt3(PUB_U(pr), c), ldcgt3(PUB_V(pr), c), alpha, beta, zn, vn);
-                    stt3(sz, n_loc + (h - e0), zn);
-                }
-            }
-            /* own row: s_{k-1}, r_k, p_{k-1}, d, then v_{k-1}, z_k */
-            sv = axpy_t(beta, sv, w);
-            r = axpy_t(-alpha, sv, r);
-            p = axpy_t(beta, p, z);
-            if (k > 0) d = axpy_t(alpha, p, d);
-            step_zv(z, u, v, alpha, beta, z, v);
-            if (mine) {
-                stt3(sz, row - row0, z);
-                /* z_k and v_{k-1} are final here: publish them now, so only u_k's stores
-                 * are still in flight when the CTA arrives at the barrier */
-                stt3(PUB_Z(pw), row, z);
-                stt3(PUB_V(pw), row, v);
+            /* own rows: s_{k-1}, r_k, p_{k-1}, d, then v_{k-1}, z_k */
+#pragma unroll
+            for (int i = 0; i < R; i++) {
+                sv[i] = axpy_t(beta, sv[i], w[i]);
+                r[i] = axpy_t(-alpha, sv[i], r[i]);
+                p[i] = axpy_t(beta, p[i], z[i]);
+                if (k > 0) d[i] = axpy_t(alpha, p[i], d[i]);
+                step_zv(z[i], u[i], v[i], alpha, beta, z[i], v[i]);
+                if (mine[i]) sz.put(row[i] - row0, z[i]);
             }
             __syncthreads();
+            seq++;
             /* w_k = A z_k from shared memory, u_k = D^-1 w_k */
-            double part[3] = { 0.0, 0.0, 0.0 };
-            T q0 = (T)0, q1 = (T)0, q2 = (T)0;
-            if (mine) {
-                const int *cb = scol + lslot + lane;
-                const int jend = len;
-                const int jsm = j_sm;
+            double part[3][R];
+#pragma unroll
+            for (int i = 0; i < R; i++) {
+                T q0 = (T)0, q1 = (T)0, q2 = (T)0;
+                const int *cb = scol + lslot[i] + lane;
+                const T *sv0 = sval + spos[i] + lane;
                 int j = 0;
-                /* four blocks at a time: their column and z loads are in flight together
-                 * (a row's blocks are still added in ascending column order) */
-                const T *sv0 = sval + 9 * lslot + lane;
-                /* the diagonal block's z is this thread's own (no shared-memory load) */
-                const int lrow = row - row0;
-                for (; j + 3 < jsm; j += 4) {
-                    const int c0 = cb[32 * j], c1 = cb[32 * (j + 1)], c2 = cb[32 * (j + 2)], c3 = cb[32 * (j + 3)];
-                    const T3<T> z0 = c0 == lrow ? z : ldt3(sz, c0), z1 = c1 == lrow ? z : ldt3(sz, c1);
-                    const T3<T> z2 = c2 == lrow ? z : ldt3(sz, c2), z3 = c3 == lrow ? z : ldt3(sz, c3);
-                    blk_acc_t(sv0 + 288 * j, z0, q0, q1, q2);
-                    blk_acc_t(sv0 + 288 * (j + 1), z1, q0, q1, q2);
-                    blk_acc_t(sv0 + 288 * (j + 2), z2, q0, q1, q2);
-                    blk_acc_t(sv0 + 288 * (j + 3), z3, q0, q1, q2);
+                for (; j + U <= kept[i]; j += U) mix_blocks<U, T>(cb + 32 * j, sv0 + 288 * j, sz, len[i] - j, q0, q1, q2);
+                if (U > 2 && kept[i] - j >= 2) {
+                    mix_blocks<2, T>(cb + 32 * j, sv0 + 288 * j, sz, len[i] - j, q0, q1, q2);
+                    j += 2;
                 }
-                for (; j < jsm; j++) {
-                    const int c0 = cb[32 * j];
-                    blk_acc_t(sv0 + 288 * j, c0 == lrow ? z : ldt3(sz, c0), q0, q1, q2);
-                }
-                if (j < jend) {
-                    /* blocks beyond the shared-memory share: values from L2, four blocks' loads
-                     * in flight together (still added in ascending column order) */
-                    const T *gv = Inner<T>::val(P) + 9 * __ldg(P.slice_ptr + s) + lane;
-                    for (; j + 3 < jend; j += 4) {
-                        T vb[4][9];
+                if (U > 1 && kept[i] - j >= 1) mix_blocks<1, T>(cb + 32 * j, sv0 + 288 * j, sz, len[i] - j, q0, q1, q2);
+                if (len[i] > kept[i]) {
+                    /* the row's last blocks, from L2 */
+                    const T *gv = Inner<T>::val(P) + 9 * (slot0 + lslot[i]) + lane;
+                    for (j = kept[i]; j < len[i]; j++) {
+                        T vb[9];
 #pragma unroll
-                        for (int u4 = 0; u4 < 4; u4++)
-#pragma unroll
-                            for (int e = 0; e < 9; e++) vb[u4][e] = __ldg(gv + 288 * (j + u4) + 32 * e);
-#pragma unroll
-                        for (int u4 = 0; u4 < 4; u4++) {
-                            const T3<T> zc = ldt3(sz, cb[32 * (j + u4)]);
-                            q0 = fma_t(vb[u4][0], zc.a, q0); q0 = fma_t(vb[u4][1], zc.b, q0); q0 = fma_t(vb[u4][2], zc.c, q0);
-                            q1 = fma_t(vb[u4][3], zc.a, q1); q1 = fma_t(vb[u4][4], zc.b, q1); q1 = fma_t(vb[u4][5], zc.c, q1);
-                            q2 = fma_t(vb[u4][6], zc.a, q2); q2 = fma_t(vb[u4][7], zc.b, q2); q2 = fma_t(vb[u4][8], zc.c, q2);
-                        }
+                        for (int e = 0; e < 9; e++) vb[e] = __ldg(gv + 288 * j + 32 * e);
+                        const T3<T> zc = sz.get(cb[32 * j]);
+                        q0 = fma_t(vb[0], zc.a, q0); q0 = fma_t(vb[1], zc.b, q0); q0 = fma_t(vb[2], zc.c, q0);
+                        q1 = fma_t(vb[3], zc.a, q1); q1 = fma_t(vb[4], zc.b, q1); q1 = fma_t(vb[5], zc.c, q1);
+                        q2 = fma_t(vb[6], zc.a, q2); q2 = fma_t(vb[7], zc.b, q2); q2 = fma_t(vb[8], zc.c, q2);
                     }
-                    for (; j < jend; j++) blk_acc_t(gv + 288 * j, ldt3(sz, cb[32 * j]), q0, q1, q2);
+                }
+                part[0][i] = part[1][i] = part[2][i] = 0.0;
+                if (mine[i]) {
+                    w[i] = T3<T>{ q0, q1, q2 };
+                    u[i] = precond(i, w[i]);
+                    if (pub[i]) put_row(Inner<T>::u(P, seq & 1), row[i], u[i], seq);
+                    const double r0 = r[i].a, r1 = r[i].b, r2 = r[i].c, z0 = z[i].a, z1 = z[i].b, z2 = z[i].c;
+                    part[0][i] = r0 * z0 + r1 * z1 + r2 * z2;                                           /* gamma */
+                    part[1][i] = (double)w[i].a * z0 + (double)w[i].b * z1 + (double)w[i].c * z2;       /* delta */
+                    part[2][i] = r0 * r0 + r1 * r1 + r2 * r2;                                           /* rho */
                 }
             }
-            if (mine) {
-                w = T3<T>{ q0, q1, q2 };
-                u = dinv_apply_t<T>(my_dinv, w); /* own row's D^-1 (stride 32) */
-                const double r0 = r.a, r1 = r.b, r2 = r.c, z0 = z.a, z1 = z.b, z2 = z.c;
-                part[0] = r0 * z0 + r1 * z1 + r2 * z2;                            /* gamma */
-                part[1] = (double)w.a * z0 + (double)w.b * z1 + (double)w.c * z2; /* delta */
-                part[2] = r0 * r0 + r1 * r1 + r2 * r2;                            /* rho */
-                /* publish u_k for iteration k + 1 (z_k and v_{k-1} went out before the SpMV) */
-                stt3(PUB_U(pw), row, u);
-            }
-            if (!grid_reduce_arrive<3, BS>(part, P.partials, epoch, P.gs, P.spin_limit, s_red, &s_ok)) {
-                timed_out = true;
-                break;
-            }
-            /* the halo's values for iteration k + 1, in flight while the partials are summed
-             * (every read of the halo z slots in this iteration's SpMV precedes the barrier) */
-            if (has_h) {
-                cp_async_row(sz + 4 * (n_loc + threadIdx.x), PUB_Z(pw) + 4 * (size_t)hrow);
-                cp_async_row(sstage + 8 * threadIdx.x, PUB_U(pw) + 4 * (size_t)hrow);
-                cp_async_row(sstage + 8 * threadIdx.x + 4, PUB_V(pw) + 4 * (size_t)hrow);
-                cp_async_commit_wait_later();
-            }
-            grid_reduce_sum<3>(P.partials, epoch, s_bc);
+            tag_reduce_send<3, R, BS>(part, P.tags, seq, s_red);
+            tag_reduce_sum<3, BS>(P.tags, seq, P.gs, P.spin_limit, s_slot, s_bc, &s_ok);
             total++;
             k++;
             if (threadIdx.x == 0) {
@@ -417,7 +463,8 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
                     a = (gamma * g) / (delta * g - gamma * gamma);
                 }
                 int flag = 0, conv = 0;
-                if (!(delta != 0.0) || !(a == a) || isinf(a)) flag = 2;
+                if (!s_ok) flag = 3;
+                else if (!(delta != 0.0) || !(a == a) || isinf(a)) flag = 2;
                 else if (rho <= P.inner_tol * P.inner_tol * s_sc[2] || rho < s_sc[3])
                     flag = conv = 1;
                 else if (k >= P.inner_max_iter || total >= P.max_iter)
@@ -429,8 +476,13 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
                 s_ab[1] = (T)bt;
                 s_flag = flag;
             }
+            /* the halo's u_k, while the sums are made */
+#pragma unroll
+            for (int i = 0; i < R; i++)
+                if (hrow[i] >= 0 && !get_row(Inner<T>::u(P, seq & 1), hrow[i], seq, P.gs, P.spin_limit, &hu[i])) s_ok = 0;
             __syncthreads();
             const int flag = s_flag;
+            if (flag == 3) { timed_out = true; break; }
             if (flag == 2) { reason = GSLAM_STOP_PQ_ZERO; break; }
             alpha = s_ab[0];
             beta = s_ab[1];
@@ -442,29 +494,38 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
                 if (F64 && s_conv) {
                     total--;
                 } else {
-                    p = axpy_t(beta, p, z);
-                    d = axpy_t(alpha, p, d);
+#pragma unroll
+                    for (int i = 0; i < R; i++) {
+                        p[i] = axpy_t(beta, p[i], z[i]);
+                        d[i] = axpy_t(alpha, p[i], d[i]);
+                    }
                 }
                 break;
             }
         }
         if (timed_out) break;
         /* ---- x += d in FP64, then the outer FP64 residual r64 = xi - A x ---- */
-        if (mine) {
-            x = ld3(P.x4, row);
-            x = V3{ x.a + (double)d.a, x.b + (double)d.b, x.c + (double)d.c };
-            st3(P.x4, row, x);
-        }
+#pragma unroll
+        for (int i = 0; i < R; i++)
+            if (mine[i]) {
+                const V3 x = ld3(P.x4, row[i]);
+                st3(P.x4, row[i], V3{ x.a + (double)d[i].a, x.b + (double)d[i].b, x.c + (double)d[i].c });
+            }
         if (!grid_barrier(P.gs, (unsigned)(++epoch), P.spin_limit, &s_ok)) { timed_out = true; break; }
-        double rr[1] = { 0.0 };
-        if (mine) {
-            const int64_t sb = __ldg(P.slice_ptr + s);
-            const V3 ax = spmv_row(P.val + 9 * sb + lane, P.col + sb + lane, len, P.x4, P.x4, 0.0, true);
-            const V3 b = ldg3(P.b4, row);
-            r64 = V3{ b.a - ax.a, b.b - ax.b, b.c - ax.c };
-            rr[0] = rr[0] + r64.a * r64.a; rr[0] = rr[0] + r64.b * r64.b; rr[0] = rr[0] + r64.c * r64.c;
+        double acc[1][R], rr[1] = { 0.0 };
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            acc[0][i] = 0.0;
+            if (mine[i]) {
+                const int64_t sb = slot0 + lslot[i];
+                const V3 ax = spmv_row(P.val + 9 * sb + lane, P.col + sb + lane, len[i], P.x4, P.x4, 0.0, true);
+                const V3 b = ldg3(P.b4, row[i]);
+                const V3 r64 = V3{ b.a - ax.a, b.b - ax.b, b.c - ax.c };
+                if (!F64) st3(P.q4, row[i], r64);
+                acc[0][i] = acc[0][i] + r64.a * r64.a; acc[0][i] = acc[0][i] + r64.b * r64.b; acc[0][i] = acc[0][i] + r64.c * r64.c;
+            }
         }
-        if (!grid_allreduce<1, BS>(rr, P.partials, epoch, P.gs, P.spin_limit, s_red, s_bc, &s_ok)) {
+        if (!grid_allreduce_rows<1, R, BS>(acc, rr, P.partials, epoch, P.gs, P.spin_limit, s_red, s_bc, &s_ok)) {
             timed_out = true;
             break;
         }
@@ -485,10 +546,12 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
             break;
         }
     }
-#undef PUB_Z
-#undef PUB_U
-#undef PUB_V
-    /* P.x4 already holds x: stored at the start of every refinement step and after it */
+    /* P.x4 already holds x: stored at the start of the first refinement step and after each; a
+     * solve that needs none stores its zeros here */
+    if (outer == 0)
+#pragma unroll
+        for (int i = 0; i < R; i++)
+            if (mine[i]) st3(P.x4, row[i], V3{ 0.0, 0.0, 0.0 });
     if (timed_out && threadIdx.x == 0) {
         res_mark_timeout(P.res);
     }
@@ -497,35 +560,58 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
     }
 }
 
-template <int BS, typename T>
-static cudaError_t set_attr_mixed() {
-    return cudaFuncSetAttribute((const void *)k_pcg_mixed<BS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                GSLAM_RES_SMEM_MAX);
+/* The kernel by precision and by the slices of the CTA that owns most: one or two per warp, as
+ * leaves registers for the rows' state. Us per iteration: FP32 at 56,000 poses (18 slices)
+ * 3.27 with one row per thread, 3.76 with two; at 70,000 (22) 4.40 (768 threads, spills) and
+ * 4.33; at 140,000 (32) 5.75 (1024 threads) and 5.24. FP64 at 56,000 5.26 (768 threads) and
+ * 4.52, at 100,000 6.88 and 6.31; D^-1 loaded ahead of the product instead of after it
+ * spills: 8.1. */
+struct MixKernel {
+    const void *fn;
+    int block, max_slices;
+};
+static const MixKernel *mix_kernels(bool fp64, int *n) {
+    static const MixKernel f[] = {
+        { (const void *)k_pcg_mixed<384, 1, float, true, 4>, 384, 12 },
+        { (const void *)k_pcg_mixed<512, 1, float, true, 4>, 512, 16 },
+        { (const void *)k_pcg_mixed<640, 1, float, true, 4>, 640, 20 },
+        { (const void *)k_pcg_mixed<384, 2, float, true, 4>, 384, 24 },
+        { (const void *)k_pcg_mixed<512, 2, float, false, 2>, 512, 32 },
+    };
+    static const MixKernel d[] = {
+        { (const void *)k_pcg_mixed<384, 1, double, true, 4>, 384, 12 },
+        { (const void *)k_pcg_mixed<512, 1, double, true, 2>, 512, 16 },
+        { (const void *)k_pcg_mixed<384, 2, double, false, 4>, 384, 24 },
+        { (const void *)k_pcg_mixed<512, 2, double, false, 1>, 512, 32 },
+    };
+    *n = (int)(fp64 ? sizeof d / sizeof d[0] : sizeof f / sizeof f[0]);
+    return fp64 ? d : f;
 }
 
-cudaError_t launch_pcg_mixed(cudaStream_t st, const PcgParams &p, int grid, int block, size_t smem_bytes, bool fp64) {
-    if (block != 768 && block != 1024) return cudaErrorInvalidValue;
-    PcgParams copy = p;
-    void *args[] = { &copy };
-    const void *fn = fp64 ? (block == 768 ? (const void *)k_pcg_mixed<768, double> : (const void *)k_pcg_mixed<1024, double>)
-                          : (block == 768 ? (const void *)k_pcg_mixed<768, float> : (const void *)k_pcg_mixed<1024, float>);
-    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, smem_bytes, st);
+cudaError_t launch_pcg_mixed(cudaStream_t st, const PcgParams &p, int grid, int max_slices, size_t smem_bytes, bool fp64) {
+    int n;
+    const MixKernel *k = mix_kernels(fp64, &n);
+    for (int i = 0; i < n; i++)
+        if (max_slices <= k[i].max_slices) {
+            PcgParams copy = p;
+            void *args[] = { &copy };
+            return cudaLaunchCooperativeKernel(k[i].fn, dim3(grid), dim3(k[i].block), args, smem_bytes, st);
+        }
+    return cudaErrorInvalidValue;
 }
 
 int pcg_mixed_max_grid(int device, size_t smem_bytes) {
-    int n_sm = 0, a = 0, b = 0, c = 0, d = 0;
+    int n_sm = 0, best = 0, n;
     if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-    if (set_attr_mixed<768, float>() != cudaSuccess || set_attr_mixed<1024, float>() != cudaSuccess ||
-        set_attr_mixed<768, double>() != cudaSuccess || set_attr_mixed<1024, double>() != cudaSuccess)
-        return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (const void *)k_pcg_mixed<768, float>, 768, smem_bytes) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void *)k_pcg_mixed<1024, float>, 1024, smem_bytes) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, (const void *)k_pcg_mixed<768, double>, 768, smem_bytes) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, (const void *)k_pcg_mixed<1024, double>, 1024, smem_bytes) !=
-            cudaSuccess)
-        return 0;
-    return std::min(std::min(a, b), std::min(c, d)) * n_sm;
+    for (int f = 0; f < 2; f++) {
+        const MixKernel *k = mix_kernels(f != 0, &n);
+        for (int i = 0; i < n; i++) {
+            int a = 0;
+            if (cudaFuncSetAttribute(k[i].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, GSLAM_GRID_SMEM_MAX) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k[i].fn, k[i].block, smem_bytes) != cudaSuccess)
+                return 0;
+            best = f == 0 && i == 0 ? a : std::min(best, a);
+        }
+    }
+    return best * n_sm;
 }

@@ -1,8 +1,11 @@
-"""The grid-wide resident FP64 solver (pcg_resident.cu) at the sizes where its kernel or its
-shared-memory split changes, against the streaming solver of the same graph
+"""The grid-wide resident solvers (pcg_resident.cu; pcg_mixed.cu in FP64 and FP32) at the sizes
+where the kernel or its shared-memory split changes, against the streaming solver of the same graph
 (disable_resident): 12, 16, 24 and 32 slices in the largest CTA, values that do not all fit,
 halos longer than the CTA's threads. The two add the dot products in other orders (relative
-1e-15 per sum), which 60 iterations amplify by far less than the 1e-9 allowed."""
+1e-15 per sum), which 60 iterations amplify by far less than the 1e-9 allowed. The
+one-reduction solver takes the same steps in another recurrence (1e-6 allowed after 40), the
+mixed one in FP32 (6e-8 per operation; 5e-2 allowed after 40: a row or block read from the
+wrong place shows as a step of another direction altogether)."""
 import importlib
 
 import numpy as np
@@ -13,22 +16,27 @@ from conftest import assert_bitwise
 pytestmark = pytest.mark.gpu
 
 
-def _dx(pkg, cg, i, j, meas, lw, **opts):
-    with pkg.PoseGraph.from_se2(cg.init, i, j, meas, lw, lam=0.1, tol=0.0, max_iter=60, **opts) as g:
+def _dx(pkg, cg, i, j, meas, lw, its=60, **opts):
+    with pkg.PoseGraph.from_se2(cg.init, i, j, meas, lw, lam=0.1, tol=0.0, max_iter=its, **opts) as g:
         g.linearise()
         g.assemble()
         out = []
         for _ in range(2):      # a second solve on the same buffers: the same bits
-            assert g.solve().iterations == 60
+            assert g.solve().iterations == its
             out.append(g.dx())
     assert_bitwise(out[1], out[0], "the same solve again")
     return out[0]
 
 
 def _check(pkg, cg, i, j, meas, lw):
-    a = _dx(pkg, cg, i, j, meas, lw)
     b = _dx(pkg, cg, i, j, meas, lw, disable_resident=1)
+    a = _dx(pkg, cg, i, j, meas, lw)
     assert np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(b)
+    if (cg.n_poses + 31) // 32 <= 32 * 148:
+        b = _dx(pkg, cg, i, j, meas, lw, its=40, disable_resident=1)
+        for prec, bound in ((2, 1e-6), (1, 5e-2)):
+            a = _dx(pkg, cg, i, j, meas, lw, its=40, precision=prec, inner_tol=0.0)
+            assert np.linalg.norm(a - b) <= bound * np.linalg.norm(b)
 
 
 @pytest.mark.parametrize("n", [4700, 33000, 45000, 60001, 90000, 120000, 151552, 151553])
