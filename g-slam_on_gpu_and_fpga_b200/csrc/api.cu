@@ -130,8 +130,8 @@ static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t s
     if (S.n_slices > CLUSTER_ONE_SLICES)
         while (ctas < max_ctas && CLUSTER_CTA_SLICES * ctas < S.n_slices) ctas *= 2;
     gslam_cluster_part part;
-    std::vector<int> lcol(S.n_slots, 0);
-    if (max_ctas == 0 || !gslam_cluster_plan(S, 0, S.n_slices, ctas, 8, GSLAM_RES_SMEM_MAX, &part, &lcol) || part.rows > 1)
+    std::vector<int> lcol(S.n_slots, 0), keep(S.n_slices, 0), pos(S.n_slices, 0);
+    if (max_ctas == 0 || !gslam_cluster_plan(S, 0, S.n_slices, ctas, 8, GSLAM_RES_SMEM_MAX, &part, &lcol, &keep, &pos))
         return GSLAM_OK;
     /* the grid-wide solver's CTAs that own slices (the order of its sums) */
     int vctas = 0;
@@ -145,11 +145,13 @@ static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t s
     CK(dupload(m, st, &L->cluster_bounds, part.bounds));
     CK(dupload(m, st, &L->cluster_halo, part.n_halo));
     CK(dupload(m, st, &L->cluster_lcol, lcol));
+    CK(dupload(m, st, &L->cluster_keep, keep));
+    CK(dupload(m, st, &L->cluster_pos, pos));
     CK(dupload(m, st, &L->cluster_exp_ptr, part.exp_ptr));
     CK(dupload(m, st, &L->cluster_exp, part.exp));
     L->cluster_ctas = part.ctas;
     L->cluster_threads = part.threads;
-    L->cluster_rows = part.rows;
+    L->cluster_shape = part.shape;
     L->cluster_smem = part.smem;
     L->cluster_vctas = vctas;
     L->cluster_ok = true;
@@ -487,6 +489,8 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
         Q.cta_slice = L->cluster_bounds;
         Q.n_halo = L->cluster_halo;
         Q.lcol = L->cluster_lcol;
+        Q.keep = L->cluster_keep;
+        Q.pos = L->cluster_pos;
         Q.exp_ptr = L->cluster_exp_ptr;
         Q.exp = L->cluster_exp;
         Q.slice_ptr = L->slice_ptr;
@@ -504,7 +508,7 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
         Q.absent_cta = o.test_absent_cta;
         Q.smem_budget = GSLAM_RES_SMEM_MAX;
         Q.res = L->res;
-        CK(launch_pcg_cluster(st, Q, 1, L->cluster_threads, L->cluster_rows, L->cluster_smem, false, false));
+        CK(launch_pcg_cluster(st, Q, 1, L->cluster_threads, L->cluster_shape, L->cluster_smem, false, false));
     } else if (mixed) CK(launch_pcg_mixed(st, P, grid, L->res_slices, L->mixed_smem_bytes, false));
     else if (cg) CK(launch_pcg_mixed(st, P, grid, L->res_slices, L->cg_smem_bytes, true));
     else if (resident) CK(launch_pcg_resident(st, P, grid, L->res_slices, L->smem_bytes));

@@ -210,15 +210,16 @@ int gslam_create_se2_batch(const gslam_se2_graph *graphs, uint32_t n_graphs, con
 
 /*
  * The graphs of a batch that get a thread-block cluster each (pcg_cluster.cu): those that
- * fit 16 CTAs (20,480 rows). Each takes the smallest cluster whose shared memory holds all
- * its values, or 16 CTAs: the GPU is shared by all graphs at once, and few full CTAs use it
- * better than many sparse ones (64 graphs of 500 to 17,000 poses: 11.1 ms of solve per
- * round; with clusters twice that size, two CTAs to an SM, 14.3; cluster sizes that are no
- * power of two, 11.2; the grid-wide batch solver 23.8). While twice as many CTAs still run
- * at once, every cluster is doubled, down to four slices per CTA. Launches of equal cluster
- * shape run side by side on their own streams, the largest clusters first, and the GPU starts
- * the next cluster as one ends; the graphs of a launch come in order of falling size, so the
- * last to start are short.
+ * fit 16 CTAs (20,480 rows). The GPU is shared by all graphs at once, and few full CTAs use it
+ * better than many sparse ones, so each takes the smallest cluster with 20 slices per CTA in
+ * FP64, 40 in FP32 (about what shared memory holds), or 16 CTAs. Ms of solve per round, 64
+ * graphs of 500 to 17,000 poses, 10 / 20 / 30 / 40 slices: FP64 14.3 / 10.3 / 11.4 / 11.9, FP32
+ * - / 8.4 / 8.1 / 7.7; the grid-wide batch solver takes 23.8 and 15.8; cluster sizes that are no
+ * power of two, or higher stream priorities for larger graphs, gain nothing. While twice as
+ * many CTAs still run at once, every cluster is doubled, down to four slices per CTA. Launches
+ * of equal cluster shape run side by side on their own streams, the largest clusters first,
+ * and the GPU starts the next cluster as one ends; the graphs of a launch come in order of
+ * falling size, so the last to start are short.
  */
 static int batch_clusters_build(gslam_graph *g, bool fp32) {
     BatchState &B = *g->batch;
@@ -230,20 +231,19 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
     K.launches.clear();
     const int max_ctas = pcg_cluster_max_ctas(g->device, GSLAM_RES_SMEM_MAX);
     std::vector<gslam_cluster_part> part(G);
-    std::vector<int> lcol(S.n_slots, 0), ctas(G, 0);
+    std::vector<int> lcol(S.n_slots, 0), keep(S.n_slices, 0), pos(S.n_slices, 0), ctas(G, 0);
     auto first = [&](int q) { return B.pose_off[q] / 32; };
     auto plan = [&](int q, int c) {
-        return gslam_cluster_plan(S, first(q), first(q + 1), c, elem, GSLAM_RES_SMEM_MAX, &part[q], &lcol);
+        return gslam_cluster_plan(S, first(q), first(q + 1), c, elem, GSLAM_RES_SMEM_MAX, &part[q], &lcol, &keep, &pos);
     };
     int64_t used = 0;
     for (int q = 0; q < G; q++) {
-        /* how many CTAs the values alone fill, then one that fits */
         const int ns = first(q + 1) - first(q);
-        const int64_t bytes = 9 * elem * (S.slice_ptr[first(q + 1)] - S.slice_ptr[first(q)]);
         int c = 1;
-        while (c < max_ctas && (c * (int64_t)GSLAM_RES_SMEM_MAX < bytes || c * (GSLAM_CLUSTER_THREADS / 32) < ns)) c *= 2;
+        const int per = fp32 ? GSLAM_CLUSTER_SLICES : GSLAM_CLUSTER_SLICES / 2;
+        while (c < max_ctas && c * per < ns) c *= 2;
         for (; c <= max_ctas; c *= 2)
-            if (plan(q, c) && (part[q].on_chip || 2 * c > max_ctas)) { ctas[q] = c; break; }
+            if (plan(q, c)) { ctas[q] = c; break; }
         used += ctas[q];
     }
     for (bool more = true; more && 2 * used <= g->L.n_sm;) {
@@ -262,12 +262,10 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
         K.in_cluster[q] = 1;
         order.push_back(q);
     }
-    /* launches: cluster size, rows per thread and CTA size (8 warps or 20) */
-    auto wide = [&](int q) { return part[q].threads > 256 ? 1 : 0; };
+    /* launches: cluster size and CTA shape */
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         if (part[a].ctas != part[b].ctas) return part[a].ctas > part[b].ctas;
-        if (part[a].rows != part[b].rows) return part[a].rows > part[b].rows;
-        if (wide(a) != wide(b)) return wide(a) > wide(b);
+        if (part[a].shape != part[b].shape) return part[a].shape > part[b].shape;
         return first(a + 1) - first(a) > first(b + 1) - first(b);
     });
     std::vector<ClusterJob> jobs;
@@ -277,8 +275,8 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
         const int q = order[i];
         const gslam_cluster_part &p = part[q];
         const int prev = i ? order[i - 1] : -1;
-        if (prev < 0 || part[prev].ctas != p.ctas || part[prev].rows != p.rows || wide(prev) != wide(q))
-            K.launches.push_back({ (int)i, 0, p.ctas, 0, p.rows, 0 });
+        if (prev < 0 || part[prev].ctas != p.ctas || part[prev].shape != p.shape)
+            K.launches.push_back({ (int)i, 0, p.ctas, 0, p.shape, 0 });
         BatchClusters::Launch &l = K.launches.back();
         l.n_jobs++;
         l.threads = std::max(l.threads, p.threads);
@@ -296,11 +294,13 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
         CK(dupload(m, g->st, &K.d_bounds, bounds));
         CK(dupload(m, g->st, &K.d_halo, halo));
         CK(dupload(m, g->st, &K.d_lcol, lcol));
+        CK(dupload(m, g->st, &K.d_keep, keep));
+        CK(dupload(m, g->st, &K.d_pos, pos));
         CK(dupload(m, g->st, &K.d_exp_ptr, exp_ptr));
         CK(dupload(m, g->st, &K.d_exp, exp));
         if (!K.all) CK(dupload(m, g->st, &K.d_rest_skip, K.in_cluster)); /* graphs the grid-wide solver leaves alone */
         if (!B.fork) CK(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming));
-        while (B.side.size() + 1 < K.launches.size()) {
+        while (B.side.size() < K.launches.size()) {
             cudaStream_t t;
             cudaEvent_t e;
             CK(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
@@ -346,6 +346,8 @@ static int batch_launch(gslam_graph *g, const PcgParams &P, BatchParams BP, bool
     Q.cta_slice = K.d_bounds;
     Q.n_halo = K.d_halo;
     Q.lcol = K.d_lcol;
+    Q.keep = K.d_keep;
+    Q.pos = K.d_pos;
     Q.exp_ptr = K.d_exp_ptr;
     Q.exp = K.d_exp;
     Q.slice_ptr = P.slice_ptr;
@@ -370,14 +372,13 @@ static int batch_launch(gslam_graph *g, const PcgParams &P, BatchParams BP, bool
     CK(cudaEventRecord(B.fork, st));
     for (size_t i = 0; i < K.launches.size(); i++) {
         const BatchClusters::Launch &l = K.launches[i];
-        cudaStream_t on = i == 0 ? st : B.side[i - 1];
-        if (i > 0) CK(cudaStreamWaitEvent(on, B.fork, 0));
+        CK(cudaStreamWaitEvent(B.side[i], B.fork, 0));
         Q.job0 = l.job0;
         Q.ctas = l.ctas;
-        CK(launch_pcg_cluster(on, Q, l.n_jobs, l.threads, l.rows, l.smem, fp32, true));
-        if (i > 0) CK(cudaEventRecord(B.side_done[i - 1], on));
+        CK(launch_pcg_cluster(B.side[i], Q, l.n_jobs, l.threads, l.shape, l.smem, fp32, true));
+        CK(cudaEventRecord(B.side_done[i], B.side[i]));
     }
-    for (size_t i = 1; i < K.launches.size(); i++) CK(cudaStreamWaitEvent(st, B.side_done[i - 1], 0));
+    for (size_t i = 0; i < K.launches.size(); i++) CK(cudaStreamWaitEvent(st, B.side_done[i], 0));
     if (!K.all) {
         BP.skip = rest_skip;
         CK(launch_pcg_batch(st, P, BP, B.grid, B.block, B.smem_bytes, fp32));

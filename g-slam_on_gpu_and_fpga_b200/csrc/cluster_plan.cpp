@@ -35,13 +35,12 @@ bool fill(const gslam_structure &S, int sl0, int sl1, int ctas, int cap, int64_t
 }  // namespace
 
 bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, int elem, int64_t budget,
-                        gslam_cluster_part *part, std::vector<int> *lcol) {
+                        gslam_cluster_part *part, std::vector<int> *lcol, std::vector<int> *keep, std::vector<int> *pos) {
     const int ns = sl1 - sl0;
-    const int warps = GSLAM_CLUSTER_THREADS / 32;
-    if (ns < ctas || ns > ctas * warps * GSLAM_CLUSTER_ROWS) return false;
+    if (ns < ctas || ns > ctas * GSLAM_CLUSTER_SLICES) return false;
     part->ctas = ctas;
-    part->rows = ns <= ctas * warps ? 1 : 2;
-    const int cap = warps * part->rows;
+    part->shape = ns <= 10 * ctas ? 0 : ns <= 20 * ctas ? 1 : 2;
+    const int cap = 10 << part->shape;
     int64_t lo = 0, hi = S.slice_ptr[sl1] - S.slice_ptr[sl0];
     for (int sl = sl0; sl < sl1; sl++) lo = std::max(lo, S.slice_ptr[sl + 1] - S.slice_ptr[sl]);
     while (lo < hi) {
@@ -52,7 +51,7 @@ bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, in
     if (!fill(S, sl0, sl1, ctas, cap, lo, &part->bounds)) return false;
     int most = 0;
     for (int r = 0; r < ctas; r++) most = std::max(most, part->bounds[r + 1] - part->bounds[r]);
-    part->threads = 32 * ((most + part->rows - 1) / part->rows);
+    part->threads = 32 * (part->shape == 2 ? (most + 1) / 2 : most);
     /* local columns and halos; the rows each CTA reads from others */
     part->n_halo.assign(ctas, 0);
     std::vector<std::vector<int>> halo(ctas);
@@ -90,13 +89,21 @@ bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, in
             part->exp[at[halo[r][h] - row_base]++] = (unsigned)r << 20 | (unsigned)h;
     /* shared memory */
     part->smem = 0;
-    part->on_chip = true;
     for (int r = 0; r < ctas; r++) {
         const int64_t n_slots = S.slice_ptr[part->bounds[r + 1]] - S.slice_ptr[part->bounds[r]];
         const ClusterSmem m = cluster_smem_layout(elem, n_slots, part->bounds[r + 1] - part->bounds[r], part->n_halo[r],
                                                   part->halo_max, budget);
         if (m.val_cap < 0) return false;
-        if (m.val_cap < 9 * n_slots) part->on_chip = false;
+        /* block positions that do not fit are left out evenly: the last one of every slice,
+         * then of every slice that still has one, and so on */
+        const int a = part->bounds[r], b = part->bounds[r + 1];
+        int64_t out = std::max<int64_t>(0, (9 * n_slots - m.val_cap) / 288);
+        for (int sl = a; sl < b; sl++) (*keep)[sl] = (int)((S.slice_ptr[sl + 1] - S.slice_ptr[sl]) / 32);
+        while (out > 0)
+            for (int sl = a; sl < b && out > 0; sl++)
+                if ((*keep)[sl] > 0) { (*keep)[sl]--; out--; }
+        (*pos)[a] = 0;
+        for (int sl = a + 1; sl < b; sl++) (*pos)[sl] = (*pos)[sl - 1] + (*keep)[sl - 1];
         part->smem = std::max(part->smem, (size_t)m.end);
     }
     /* one mbarrier phase counts at most 2^20 - 1 bytes; halo slots are 20-bit */

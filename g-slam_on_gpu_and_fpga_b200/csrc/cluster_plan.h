@@ -10,9 +10,8 @@
 
 /* one graph's split over a cluster */
 struct gslam_cluster_part {
-    int ctas = 0, threads = 0, rows = 1; /* rows: block rows per thread */
+    int ctas = 0, threads = 0, shape = 0; /* shape: launch_pcg_cluster */
     int halo_max = 0;
-    bool on_chip = false;                /* every value is in shared memory */
     size_t smem = 0;                     /* dynamic shared memory of the largest CTA */
     std::vector<int> bounds;             /* [ctas + 1] slices */
     std::vector<int> n_halo;             /* [ctas] */
@@ -21,10 +20,11 @@ struct gslam_cluster_part {
 };
 
 /* Splits the slices [sl0, sl1) over a cluster of `ctas` CTAs for values of `elem` bytes;
- * lcol (all slots of the layout) gets the graph's CTA-local columns. False when the graph
+ * lcol (all slots of the layout) gets the graph's CTA-local columns, keep and pos (all its
+ * slices) the block positions in shared memory and where they start. False when the graph
  * does not fit (more rows than the threads own, or the fixed parts of a CTA's shared
- * memory exceed the budget); *part and the graph's part of lcol are then undefined. */
+ * memory exceed the budget); *part and the graph's part of the arrays are then undefined. */
 bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, int elem, int64_t budget,
-                        gslam_cluster_part *part, std::vector<int> *lcol);
+                        gslam_cluster_part *part, std::vector<int> *lcol, std::vector<int> *keep, std::vector<int> *pos);
 
 #endif

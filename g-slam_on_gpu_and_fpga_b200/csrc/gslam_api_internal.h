@@ -56,10 +56,11 @@ struct DevLayout {
     size_t cg_smem_bytes = 0;
     /* cluster solver (pcg_cluster.cu), when the graph fits one thread-block cluster */
     bool cluster_ok = false;
-    int cluster_ctas = 0, cluster_threads = 0, cluster_rows = 1, cluster_vctas = 0;
+    int cluster_ctas = 0, cluster_threads = 0, cluster_shape = 0, cluster_vctas = 0;
     size_t cluster_smem = 0;
     ClusterJob *cluster_job = nullptr;
     int *cluster_bounds = nullptr, *cluster_halo = nullptr, *cluster_lcol = nullptr, *cluster_exp_ptr = nullptr;
+    int *cluster_keep = nullptr, *cluster_pos = nullptr;
     unsigned *cluster_exp = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;   /* brackets the solver launch */
     int max_grid_alloc() const { return partial_capacity; }
@@ -69,7 +70,7 @@ struct DevLayout {
  * launches of equal cluster shape, largest clusters first. */
 struct BatchClusters {
     struct Launch {
-        int job0, n_jobs, ctas, threads, rows;
+        int job0, n_jobs, ctas, threads, shape;
         size_t smem;
     };
     bool built = false;
@@ -78,6 +79,7 @@ struct BatchClusters {
     bool all = false;            /* every graph has one */
     ClusterJob *d_jobs = nullptr;
     int *d_bounds = nullptr, *d_halo = nullptr, *d_lcol = nullptr, *d_exp_ptr = nullptr;
+    int *d_keep = nullptr, *d_pos = nullptr;
     unsigned *d_exp = nullptr;
     int *d_rest_skip = nullptr;  /* [n_graphs] graphs that the grid-wide solver leaves alone */
 };

@@ -204,8 +204,7 @@ int pcg_resident_max_grid(int device, size_t smem_bytes);
 
 /* Solver of a graph inside one thread-block cluster (pcg_cluster.cu). */
 #define GSLAM_CLUSTER_CTAS 16    /* largest cluster (non-portable size) */
-#define GSLAM_CLUSTER_THREADS 640 /* largest CTA: 20 warps, up to 96 registers a thread */
-#define GSLAM_CLUSTER_ROWS 2     /* block rows a thread may own */
+#define GSLAM_CLUSTER_SLICES 40  /* most slices of a CTA */
 
 /* one graph for one cluster: the range of its slices and where its per-CTA data lie */
 struct ClusterJob {
@@ -224,6 +223,8 @@ struct ClusterParams {
     const int *cta_slice; /* slice bounds of every job's CTAs */
     const int *n_halo;    /* halo rows of every job's CTAs */
     const int *lcol;      /* per slot, CTA-local column index (own rows, then halo) */
+    const int *keep, *pos; /* per slice: block positions kept in shared memory, and the first one's
+                           * place there (in positions of 288 values) */
     const int *exp_ptr;   /* per row of a job, bounds in exp */
     const unsigned *exp;  /* the CTAs that read a row and the halo slot there: rank << 20 | slot */
     const int64_t *slice_ptr;
@@ -266,8 +267,9 @@ __host__ __device__ inline ClusterSmem cluster_smem_layout(int64_t elem, int64_t
     return m;
 }
 
-cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jobs, int threads, int rows_per_thread,
+cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jobs, int threads, int shape,
                                size_t smem_bytes, bool fp32, bool batch);
+/* shape: 0 up to 10 slices per CTA, 1 up to 20, 2 up to 40 (two per warp) */
 /* Largest cluster the solver's kernels can be launched with (0: none), with this much
  * dynamic shared memory per CTA; also sets their attributes. */
 int pcg_cluster_max_ctas(int device, size_t smem_bytes);

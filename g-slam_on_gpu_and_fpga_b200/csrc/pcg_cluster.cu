@@ -11,10 +11,12 @@
  * cluster per graph, as many at a time as the GPU holds.
  *
  * Layout: CTA r of a graph's cluster owns a contiguous range of its slices (balanced by
- * slot count), one thread per block row (R slices per warp). Values (as far as they fit),
+ * slot count), one thread per block row (two above 20 slices per CTA). Values (as far as they
+ * fit; every slice leaves out its last block positions, so that no warp is much slower than
+ * the others: 8.2 us per iteration at 16,000 poses against 9.5 with whole slices left out),
  * CTA-local column indices and p of own and halo rows are in shared memory; x, r, z, p, q
- * and, for R = 1, the row's D^-1 are in registers. Nothing but the values that do not fit
- * (and D^-1 for R = 2) is read from L2 during the solve.
+ * and, with one row per thread, the row's D^-1 are in registers. Nothing but the values that
+ * do not fit (and D^-1 of two rows) is read from L2 during the solve.
  *
  * Exchange: warp 0 adds its CTA's partials and stores the sum into every CTA of the cluster
  * (st.async: the data and the count on the receiver's mbarrier in one message, no fence and
@@ -175,10 +177,12 @@ __device__ __forceinline__ void cl_bar_arrive(int id, int threads) {
 }
 
 /* ONE: the cluster is one CTA (its partials stay in its shared memory) */
-template <typename T, int R, bool ONE, bool BATCH>
-__global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const ClusterParams P) {
+template <typename T, int BS, int R, bool ONE, bool BATCH>
+__global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int MAXS = GSLAM_CLUSTER_THREADS / 32 * R; /* slices of a CTA */
+    constexpr int MAXS = BS / 32 * R; /* slices of a CTA */
+    constexpr bool DREGS = R == 1;    /* the rows' D^-1 stay in registers, else L2 */
+    constexpr int U = R == 1 ? 4 : 2; /* blocks whose loads are issued together */
     __shared__ __align__(8) uint64_t s_mb[3];            /* staging; p.q; r.z, r.r and halo z */
     __shared__ __align__(16) double s_part[MAXS];        /* the slices' p.q */
     __shared__ __align__(16) double2 s_part2[MAXS];      /* the slices' (r.z, r.r) */
@@ -235,16 +239,26 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
     if (!absent && threadIdx.x == 0) {
         const unsigned vbytes = (unsigned)(sizeof(T) * nsm), cbytes = (unsigned)(4 * (slot1 - slot0));
         tma_mbar_expect_tx(&s_mb[0], vbytes + cbytes);
-        if (vbytes) tma_bulk_g2s(sval, ClVec<T>::val(P) + 9 * slot0, vbytes, &s_mb[0]);
+        /* one copy when every value fits, else one per slice (its kept positions) */
+        if (nsm == nval) {
+            if (vbytes) tma_bulk_g2s(sval, ClVec<T>::val(P) + 9 * slot0, vbytes, &s_mb[0]);
+        } else {
+            for (int t = s0; t < s1; t++) {
+                const int n = __ldg(P.keep + t);
+                if (n)
+                    tma_bulk_g2s(sval + 288 * __ldg(P.pos + t), ClVec<T>::val(P) + 9 * __ldg(P.slice_ptr + t),
+                                 (unsigned)(288 * sizeof(T)) * n, &s_mb[0]);
+            }
+        }
         if (cbytes) tma_bulk_g2s(scol, P.lcol + slot0, cbytes, &s_mb[0]);
         /* waited for by every thread below, after its first rows are read */
     }
 
     /* ---- this thread's rows ---- */
-    int row[R], len[R], wsm[R], width[R], voff[R], e0[R], ecnt[R];
+    int row[R], len[R], kept[R], spos[R], voff[R], e0[R], ecnt[R];
     bool mine[R];
     C3<T> x[R], r[R], z[R], p[R];
-    double d[R == 1 ? 9 : 1];
+    double d[DREGS ? R : 1][9];
 #pragma unroll
     for (int i = 0; i < R; i++) {
         const int s = s0 + warp + i * W;
@@ -253,21 +267,22 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
         mine[i] = own && row[i] < P.n_rows;
         len[i] = mine[i] ? __ldg(P.row_len + row[i]) : 0;
         voff[i] = own ? (int)(__ldg(P.slice_ptr + s) - slot0) : 0;
-        width[i] = own ? (int)(__ldg(P.slice_ptr + s + 1) - slot0 - voff[i]) >> 5 : 0;
-        /* the slice's block positions with values in shared memory (the rest are in L2) */
-        wsm[i] = min(width[i], max(0, ((int)nsm - 9 * voff[i]) / 288));
+        /* the slice's block positions with values in shared memory, and where; the last ones,
+         * if they do not all fit, are read from L2 */
+        kept[i] = own ? __ldg(P.keep + s) : 0;
+        spos[i] = own ? 288 * __ldg(P.pos + s) : 0;
         const int er = J.exp0 + row[i] - 32 * J.slice0;
         e0[i] = mine[i] && !ONE ? __ldg(P.exp_ptr + er) : 0;
         ecnt[i] = mine[i] && !ONE ? __ldg(P.exp_ptr + er + 1) - e0[i] : 0;
         x[i] = r[i] = z[i] = p[i] = C3<T>{ 0, 0, 0 };
-        if (R == 1 && mine[i]) {
+        if (DREGS && mine[i]) {
             const double *g = P.dinv + 288 * (size_t)s + lane;
 #pragma unroll
-            for (int e = 0; e < 9; e++) d[e] = __ldg(g + 32 * e);
+            for (int e = 0; e < 9; e++) d[DREGS ? i : 0][e] = __ldg(g + 32 * e);
         }
     }
     auto dinv_row = [&](int i, C3<T> rv) {
-        if (R == 1) return cl_dinv<T>([&](int e) { return d[R == 1 ? e : 0]; }, rv);
+        if (DREGS) return cl_dinv<T>([&](int e) { return d[DREGS ? i : 0][e]; }, rv);
         const double *g = P.dinv + 288 * (size_t)(row[i] >> 5) + lane;
         return cl_dinv<T>([&](int e) { return __ldg(g + 32 * e); }, rv);
     };
@@ -392,27 +407,28 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
             for (int i = 0; i < R; i++) {
                 T q0 = 0, q1 = 0, q2 = 0;
                 const int *cb = scol + voff[i] + lane;
-                const T *sv = sval + 9 * voff[i] + lane;
+                const T *sv = sval + spos[i] + lane;
                 int j = 0;
-                for (; j + 4 <= wsm[i]; j += 4)
-                    cl_blocks<4>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2);
-                switch (wsm[i] - j) {
-                case 1: cl_blocks<1>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2); break;
-                case 2: cl_blocks<2>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2); break;
-                case 3: cl_blocks<3>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2); break;
-                default: break;
+                for (; j + U <= kept[i]; j += U)
+                    cl_blocks<U>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2);
+                if (U > 2 && kept[i] - j >= 2) {
+                    cl_blocks<2>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2);
+                    j += 2;
                 }
-                /* the share's tail, from L2 */
-                for (j = wsm[i]; j < len[i]; j++) {
-                    const T *gv = ClVec<T>::val(P) + 9 * (slot0 + voff[i]) + lane + 288 * j;
-                    T vb[9];
+                if (kept[i] - j >= 1) cl_blocks<1>(cb + 32 * j, sv + 288 * j, sp0, sp1, sp2, len[i] - j, q0, q1, q2);
+                if (len[i] > kept[i]) {
+                    /* the row's last blocks, from L2 */
+                    const T *gv = ClVec<T>::val(P) + 9 * (slot0 + voff[i]) + lane;
+                    for (j = kept[i]; j < len[i]; j++) {
+                        T vb[9];
 #pragma unroll
-                    for (int e = 0; e < 9; e++) vb[e] = __ldg(gv + 32 * e);
-                    const int c = cb[32 * j];
-                    const C3<T> pc = { sp0[c], sp1[c], sp2[c] };
-                    q0 = q0 + vb[0] * pc.a; q0 = q0 + vb[1] * pc.b; q0 = q0 + vb[2] * pc.c;
-                    q1 = q1 + vb[3] * pc.a; q1 = q1 + vb[4] * pc.b; q1 = q1 + vb[5] * pc.c;
-                    q2 = q2 + vb[6] * pc.a; q2 = q2 + vb[7] * pc.b; q2 = q2 + vb[8] * pc.c;
+                        for (int e = 0; e < 9; e++) vb[e] = __ldg(gv + 288 * j + 32 * e);
+                        const int c = cb[32 * j];
+                        const C3<T> pc = { sp0[c], sp1[c], sp2[c] };
+                        q0 = q0 + vb[0] * pc.a; q0 = q0 + vb[1] * pc.b; q0 = q0 + vb[2] * pc.c;
+                        q1 = q1 + vb[3] * pc.a; q1 = q1 + vb[4] * pc.b; q1 = q1 + vb[5] * pc.c;
+                        q2 = q2 + vb[6] * pc.a; q2 = q2 + vb[7] * pc.b; q2 = q2 + vb[8] * pc.c;
+                    }
                 }
                 q[i] = C3<T>{ q0, q1, q2 };
                 double pq = 0.0;
@@ -512,19 +528,25 @@ __global__ void __launch_bounds__(GSLAM_CLUSTER_THREADS, 1) k_pcg_cluster(const 
     }
 }
 
-template <typename T, bool BATCH>
-static const void *fn_of(int rows, bool one) {
-    if (rows == 1)
-        return one ? (const void *)k_pcg_cluster<T, 1, true, BATCH> : (const void *)k_pcg_cluster<T, 1, false, BATCH>;
-    return one ? (const void *)k_pcg_cluster<T, 2, true, BATCH> : (const void *)k_pcg_cluster<T, 2, false, BATCH>;
+/* The kernel's shapes: up to 10, 20 and 40 slices per CTA. One row per thread and 10 warps have
+ * the registers for everything; 20 warps (96 registers) hide more latency than 10 warps of
+ * two rows each (64-graph batch: 11.1 ms of solve per round against 12.9). */
+template <typename T, bool ONE, bool BATCH>
+static const void *fn_of(int shape) {
+    switch (shape) {
+    case 0: return (const void *)k_pcg_cluster<T, 320, 1, ONE, BATCH>;
+    case 1: return (const void *)k_pcg_cluster<T, 640, 1, ONE, BATCH>;
+    default: return (const void *)k_pcg_cluster<T, 640, 2, ONE, BATCH>;
+    }
 }
 
-/* kinds of launches: FP32 batches, FP64 batches, single graphs (one row per thread) */
-static const void *cluster_fn(int kind, int rows, bool one) {
+/* kinds of launches: FP32 batches, FP64 batches, single graphs */
+#define CLUSTER_KINDS 3
+static const void *cluster_fn(int kind, int shape, bool one) {
     switch (kind) {
-    case 0: return fn_of<float, true>(rows, one);
-    case 1: return fn_of<double, true>(rows, one);
-    default: return one ? (const void *)k_pcg_cluster<double, 1, true, false> : (const void *)k_pcg_cluster<double, 1, false, false>;
+    case 0: return one ? fn_of<float, true, true>(shape) : fn_of<float, false, true>(shape);
+    case 1: return one ? fn_of<double, true, true>(shape) : fn_of<double, false, true>(shape);
+    default: return one ? fn_of<double, true, false>(shape) : fn_of<double, false, false>(shape);
     }
 }
 
@@ -543,7 +565,7 @@ static void cluster_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *at, int
     cfg->numAttrs = 1;
 }
 
-cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jobs, int threads, int rows_per_thread,
+cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jobs, int threads, int shape,
                                size_t smem_bytes, bool fp32, bool batch) {
     if (n_jobs <= 0) return cudaSuccess;
     cudaLaunchConfig_t cfg;
@@ -552,26 +574,27 @@ cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jo
     ClusterParams copy = p;
     void *args[] = { &copy };
     const int kind = fp32 ? 0 : batch ? 1 : 2;
-    if (kind == 2 && rows_per_thread != 1) return cudaErrorInvalidValue;
-    return cudaLaunchKernelExC(&cfg, cluster_fn(kind, rows_per_thread, p.ctas == 1), args);
+    return cudaLaunchKernelExC(&cfg, cluster_fn(kind, shape, p.ctas == 1), args);
 }
 
 int pcg_cluster_max_ctas(int device, size_t smem_bytes) {
     (void)device;
     int best = 0;
-    for (int v = 0; v < 12; v++) {
-        const void *fn = cluster_fn(v >> 2, 1 + (v & 1), (v & 2) != 0);
+    for (int v = 0; v < CLUSTER_KINDS * 6; v++) {
+        const bool one = v % 2 != 0;
+        const int shape = v / 2 % 3, threads = shape == 0 ? 320 : 640;
+        const void *fn = cluster_fn(v / 6, shape, one);
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess ||
             cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
-        if (v & 2) continue; /* one CTA needs no cluster */
+        if (one) continue; /* one CTA needs no cluster */
         int can = 0;
         for (int c = GSLAM_CLUSTER_CTAS; c > 1; c /= 2) {
             cudaLaunchConfig_t cfg;
             cudaLaunchAttribute at[1];
-            cluster_config(&cfg, at, c, c, GSLAM_CLUSTER_THREADS, smem_bytes, nullptr);
+            cluster_config(&cfg, at, c, c, threads, smem_bytes, nullptr);
             int n = 0;
             if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) { can = c; break; }
             cudaGetLastError();

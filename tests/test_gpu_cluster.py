@@ -103,7 +103,7 @@ def test_absent_cta_of_the_cluster_times_out(pkg, synth):
     g.close()
 
 
-SIZES = (37, 600, 640, 5000, 10240, 10250, 20480, 20500)   # the last one fits no cluster
+SIZES = (37, 320, 330, 640, 650, 5000, 10240, 10250, 20480, 20500)   # the last one fits no cluster
 
 
 @pytest.mark.parametrize("prec", [PREC_FP64, PREC_MIXED], ids=["fp64", "mixed"])
