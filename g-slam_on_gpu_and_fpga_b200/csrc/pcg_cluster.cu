@@ -120,17 +120,46 @@ __device__ __forceinline__ double cl_warp_sum(double a) {
     return a;
 }
 
-/* the sum of the partials v(a) .. v(a + n - 1), n <= 32, as the grid-wide solver's warp
- * tree adds a CTA's warps (offsets 16, 8, 4, 2, 1; missing warps are 0) */
-template <typename F>
-__device__ __forceinline__ double cl_tree(F v, int a, int n) {
-    auto at = [&](int i) { return i < n ? v(a + i) : 0.0; };
-    if (n <= 1) return at(0);
-    if (n <= 4) return (at(0) + at(2)) + (at(1) + at(3));
+__device__ __forceinline__ double cl_add(double a, double b) { return a + b; }
+__device__ __forceinline__ double2 cl_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double cl_xor(double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+__device__ __forceinline__ double2 cl_xor(double2 a, int o) { return make_double2(cl_xor(a.x, o), cl_xor(a.y, o)); }
+
+/* the sum of the partials v[a] .. v[a + n - 1], n <= most <= 32 (most: the warp's largest n),
+ * as the grid-wide solver's warp tree adds a CTA's warps (offsets 16, 8, 4, 2, 1; missing
+ * warps are 0) */
+template <int STRIDE>
+__device__ __forceinline__ double cl_tree(const double *v, int a, int n, int most) {
+    auto at = [&](int i) { return i < n ? v[STRIDE * (a + i)] : 0.0; };
+    if (most <= 4) return (at(0) + at(2)) + (at(1) + at(3));
     double b[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) b[i] = n <= 8 ? at(i) : (at(i) + at(i + 16)) + (at(i + 8) + at(i + 24));
+    for (int i = 0; i < 8; i++) b[i] = most <= 8 ? at(i) : (at(i) + at(i + 16)) + (at(i + 8) + at(i + 24));
     return ((b[0] + b[4]) + (b[2] + b[6])) + ((b[1] + b[5]) + (b[3] + b[7]));
+}
+__device__ __forceinline__ double cl_tree(const double *v, int a, int n, int most) { return cl_tree<1>(v, a, n, most); }
+__device__ __forceinline__ double2 cl_tree(const double2 *v, int a, int n, int most) {
+    if (most <= 1) return n > 0 ? v[a] : make_double2(0.0, 0.0);
+    return make_double2(cl_tree<2>(&v->x, a, n, most), cl_tree<2>(&v->y, a, n, most));
+}
+
+/* The sum of 16 values that every lane can read, on every lane, in the order of the butterfly
+ * over 16 lanes: a lane adds the even or the odd ones in registers, and of double2 one
+ * component (one or three shuffles instead of four or eight). */
+__device__ __forceinline__ double cl_sum8(const double *v, int stride) {
+    double b[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) b[i] = v[2 * i * stride];
+    return ((b[0] + b[4]) + (b[2] + b[6])) + ((b[1] + b[5]) + (b[3] + b[7]));
+}
+__device__ __forceinline__ double cl_sum16(const double *v) {
+    const double s = cl_sum8(v + (threadIdx.x & 1), 1);
+    return s + cl_xor(s, 1);
+}
+__device__ __forceinline__ double2 cl_sum16(const double2 *v) {
+    double s = cl_sum8(&v[threadIdx.x & 1].x + (threadIdx.x >> 1 & 1), 2);
+    s = s + cl_xor(s, 1);
+    return make_double2(__shfl_sync(0xffffffffu, s, 0), __shfl_sync(0xffffffffu, s, 2));
 }
 
 template <typename T> struct ClVec;
@@ -180,12 +209,13 @@ __device__ __forceinline__ void cl_bar_arrive(int id, int threads) {
 template <typename T, int BS, int R, bool ONE, bool BATCH>
 __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int MAXS = BS / 32 * R; /* slices of a CTA */
+    constexpr int MAXS = BS / 32 * R;                           /* slices of a CTA */
+    constexpr int MAXP = MAXS <= 16 ? 16 : MAXS <= 32 ? 32 : 64; /* their partials, 0 beyond its slices */
     constexpr bool DREGS = R == 1;    /* the rows' D^-1 stay in registers, else L2 */
     constexpr int U = R == 1 ? 4 : 2; /* blocks whose loads are issued together */
     __shared__ __align__(8) uint64_t s_mb[3];            /* staging; p.q; r.z, r.r and halo z */
-    __shared__ __align__(16) double s_part[MAXS];        /* the slices' p.q */
-    __shared__ __align__(16) double2 s_part2[MAXS];      /* the slices' (r.z, r.r) */
+    __shared__ __align__(16) double s_part[MAXP];        /* the slices' p.q */
+    __shared__ __align__(16) double2 s_part2[MAXP];      /* the slices' (r.z, r.r) */
     __shared__ __align__(16) double s_all[GSLAM_CLUSTER_CTAS];   /* the CTAs' p.q */
     __shared__ __align__(16) double2 s_all2[GSLAM_CLUSTER_CTAS]; /* the CTAs' (r.z, r.r) */
     __shared__ double s_bn, s_alpha, s_beta;
@@ -224,6 +254,14 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
             arm(b_rz, bytes_rz);
         }
         s_flag = s_flag_pq = 0;
+    }
+    for (int i = threadIdx.x; i < MAXP; i += blockDim.x) {
+        s_part[i] = 0.0;
+        s_part2[i] = make_double2(0.0, 0.0);
+    }
+    if (threadIdx.x < GSLAM_CLUSTER_CTAS) {
+        s_all[threadIdx.x] = 0.0; /* stay 0 beyond the cluster's CTAs */
+        s_all2[threadIdx.x] = make_double2(0.0, 0.0);
     }
     /* every CTA's barriers are ready before anything is stored to it */
     if (ONE) __syncthreads();
@@ -292,36 +330,34 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
     };
     /* The sum over this CTA's slices, on every lane of the calling warp. ONE single graphs: in
      * the grid-wide solver's order, per CTA of its partition (lane c: its first slice and how
-     * many), then over its CTAs. Butterflies run over the next power of two of the summands
+     * many), then over its CTAs; that butterfly runs over the next power of two of the CTAs
      * only: the steps left out would add zeros. */
-    const int n_sum = ONE && !BATCH ? P.n_vcta : ns;
-    int p2 = 1, c2 = 1;
-    while (p2 < n_sum && p2 < 32) p2 *= 2;
-    while (c2 < C) c2 *= 2;
-    const int sl = lane & (p2 - 1), cl = lane & (c2 - 1);
-    int vt0 = 0, vtn = 0;
-    if (ONE && !BATCH && sl < n_sum) {
-        vt0 = __ldg(P.vcta_slice + sl);
-        vtn = __ldg(P.vcta_slice + sl + 1) - vt0;
-    }
-    auto sum_slices = [&](auto v) {
-        double s = 0.0;
-        if (ONE && !BATCH) {
-            s = cl_tree(v, vt0, vtn);
-        } else {
-            for (int c = sl; c < ns; c += 32) s = s + v(c);
+    int p2 = 1, vt0 = 0, vtn = 0, vt_most = 0;
+    if (ONE && !BATCH) {
+        while (p2 < P.n_vcta) p2 *= 2;
+        const int c = lane & (p2 - 1);
+        if (c < P.n_vcta) {
+            vt0 = __ldg(P.vcta_slice + c);
+            vtn = __ldg(P.vcta_slice + c + 1) - vt0;
         }
+        vt_most = __reduce_max_sync(0xffffffffu, vtn);
+    }
+    auto sum_slices = [&](const auto *v) {
+        if constexpr (ONE && !BATCH) {
+            auto s = cl_tree(v, vt0, vtn, vt_most);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            if (o < p2) s = s + __shfl_xor_sync(0xffffffffu, s, o);
-        return s;
-    };
-    /* the sum over the cluster's CTAs, on every lane */
-    auto sum_ctas = [&](double s) {
+            for (int o = 16; o > 0; o >>= 1)
+                if (o < p2) s = cl_add(s, cl_xor(s, o));
+            return s;
+        } else if constexpr (MAXP == 16) {
+            return cl_sum16(v);
+        } else {
+            auto s = v[lane];
+            if (MAXP > 32) s = cl_add(s, v[(lane + 32) % MAXP]);
 #pragma unroll
-        for (int o = GSLAM_CLUSTER_CTAS / 2; o > 0; o >>= 1)
-            if (o < c2) s = s + __shfl_xor_sync(0xffffffffu, s, o);
-        return s;
+            for (int o = 16; o > 0; o >>= 1) s = cl_add(s, cl_xor(s, o));
+            return s;
+        }
     };
 
     bool ok = true;
@@ -330,37 +366,35 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
      * s_part or s_part2. ONE: on every lane of every warp, which then makes the scalars for
      * itself: one barrier per sum instead of three, 2.08 -> 1.57 us per iteration at 100 poses.
      * Else on the lanes of warp 0 only, because a wait that gives up has to be the whole CTA's:
-     * one warp decides. `between` is the caller's work while the sums travel. */
+     * one warp decides (and arms the barrier again, before it next stores to another CTA:
+     * none can send the next sums earlier). `between` is the caller's work while the sums travel. */
     auto total_pq = [&]() {
         if (ONE) {
             __syncthreads();
-            return sum_slices([&](int c) { return s_part[c]; });
+            return sum_slices(s_part);
         }
         if (warp == 0) {
             cl_bar_sync(1, blockDim.x);
-            const double s = sum_slices([&](int c) { return s_part[c]; });
+            const double s = sum_slices(s_part);
             if (lane < C) cl_st_async(cl_mapa(cl_smem_u32(&s_all[rank]), lane), s, cl_mapa(b_pq, lane));
         } else {
             cl_bar_arrive(1, blockDim.x);
         }
         if (warp != 0) return 0.0;
         ok = cl_wait(b_pq, k & 1, P.spin_limit);
-        if (threadIdx.x == 0 && ok) arm(b_pq, bytes_pq);
-        return sum_ctas(cl < C ? s_all[cl] : 0.0);
+        return cl_sum16(s_all);
     };
     auto total_rz = [&](auto between) {
         double2 t = make_double2(0.0, 0.0);
         if (ONE) {
             __syncthreads();
-            t.x = sum_slices([&](int c) { return s_part2[c].x; });
-            t.y = sum_slices([&](int c) { return s_part2[c].y; });
+            t = sum_slices(s_part2);
             between();
             return t;
         }
         if (warp == 0) {
             cl_bar_sync(2, blockDim.x);
-            t.x = sum_slices([&](int c) { return s_part2[c].x; });
-            t.y = sum_slices([&](int c) { return s_part2[c].y; });
+            t = sum_slices(s_part2);
             if (lane < C) cl_st_async2(cl_mapa(cl_smem_u32(&s_all2[rank]), lane), t.x, t.y, cl_mapa(b_rz, lane));
         } else {
             cl_bar_arrive(2, blockDim.x);
@@ -368,9 +402,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
         between();
         if (warp != 0) return t;
         ok = cl_wait(b_rz, k & 1, P.spin_limit);
-        if (threadIdx.x == 0 && ok) arm(b_rz, bytes_rz);
-        const double2 v = cl < C ? s_all2[cl] : make_double2(0.0, 0.0);
-        return make_double2(sum_ctas(v.x), sum_ctas(v.y));
+        return cl_sum16(s_all2);
     };
     double rz_cur = 0.0, rr_cur = 0.0, limit = 0.0; /* ONE: in every thread; else in thread 0 */
     if (!absent) {
@@ -400,6 +432,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
                 if (BATCH && t.y == 0.0) s_flag = 1 + GSLAM_STOP_TOL; /* zero right-hand side: x = 0 */
             }
             if (!ok) s_flag = 1 + GSLAM_STOP_TIMEOUT;
+            else if (!ONE && threadIdx.x == 0) arm(b_rz, bytes_rz);
         }
         if (!tma_wait(&s_mb[0], 0, P.spin_limit)) {
             s_flag = 1 + GSLAM_STOP_TIMEOUT;
@@ -479,6 +512,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
                     if (!ok) s_flag_pq = 1 + GSLAM_STOP_TIMEOUT;
                     else if (pq == 0.0) s_flag_pq = 1 + GSLAM_STOP_PQ_ZERO;
                     s_alpha = rz_cur / pq;
+                    if (ok) arm(b_pq, bytes_pq);
                 }
                 __syncthreads();
                 flag = s_flag_pq;
@@ -521,6 +555,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
                     s_beta = t.x / rz_cur;
                     rz_cur = t.x;
                     rr_cur = t.y;
+                    if (ok) arm(b_rz, bytes_rz);
                 }
                 __syncthreads();
                 flag = s_flag;
