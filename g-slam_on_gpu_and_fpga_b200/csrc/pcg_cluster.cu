@@ -530,9 +530,9 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
                     rr = rr + r0 * r0; rr = rr + r1 * r1; rr = rr + r2 * r2;
                     rz = rz + r0 * (double)z[i].a; rz = rz + r1 * (double)z[i].b; rz = rz + r2 * (double)z[i].c;
                 }
-                rr = cl_warp_sum(rr);
-                rz = cl_warp_sum(rz);
-                if (lane == 0 && warp + i * W < ns) s_part2[warp + i * W] = make_double2(rz, rr);
+                double sums[2] = { rz, rr };
+                const double sum = warp_sums<2>(sums);
+                if ((lane & 15) == 0 && warp + i * W < ns) (&s_part2[warp + i * W].x)[lane >> 4] = sum;
             }
             k++;
             /* while the sums travel: the halo's z, and x */
