@@ -110,17 +110,18 @@ void DevMem::release() {
 }
 
 /* The cluster solver's plan of a single graph, where it is the faster one. Us per iteration,
- * cluster / grid-wide solver: 1.5 / 3.4 at 100 poses, 2.7 / 3.35 at 800, 2.85 / 3.4 at 2,001,
- * 3.2 / 3.5 at 4,000, 3.45 / 3.47 at 5,000 (city walks); landmark logs, with longer rows,
- * 3.4 / 4.0 at 2,001, 3.8 / 4.1 at 4,000, 4.2 / 3.9 at 5,000: up to 144 slices (4,608 rows).
+ * cluster / grid-wide solver: 1.5 / 3.1 at 100 poses, 2.0 / 3.1 at 800, 2.1 / 3.15 at 2,001,
+ * 2.3 / 3.3 at 4,000, 3.0 / 3.4 at 7,120, 3.4 / 3.4 at 8,000 (city walks; with twice the
+ * closures, some far, 3.4 / 3.6 at 7,120 and 4.0 / 3.6 at 8,000); landmark logs, with longer
+ * rows, 2.6 / 3.7 at 2,001, 2.9 / 3.8 at 4,000, 3.4 / 3.9 at 7,120: up to 224 slices (7,168 rows),
+ * 14 per CTA.
  * One CTA up to 13 slices: such a solve can go past convergence within its 500 iterations,
- * where rounding decides the iterates, and one CTA adds in the grid-wide solver's order (2.1
- * at 100 poses, where 2 and 4 CTAs take 2.7). Then four slices per CTA (a warp per SM
- * sub-partition) up to 16 CTAs: 2.7 at 800 poses with 8 CTAs (4: 2.9, 2: 3.4), 2.85 at
- * 2,001 with 16 (8: 3.1, 4: 3.8). */
+ * where rounding decides the iterates, and one CTA adds in the grid-wide solver's order (1.5
+ * at 100 poses). Then four slices per CTA (a warp per SM sub-partition) up to 16 CTAs: 2.55 at
+ * 1,000 poses of a log with 8 CTAs, 2.74 with 16. */
 #define CLUSTER_ONE_SLICES 13
 #define CLUSTER_CTA_SLICES 4
-#define CLUSTER_MAX_SLICES 144
+#define CLUSTER_MAX_SLICES 224
 
 static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, int device,
                           const std::vector<int> &grid_slices) {
@@ -129,9 +130,13 @@ static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t s
     int ctas = 1;
     if (S.n_slices > CLUSTER_ONE_SLICES)
         while (ctas < max_ctas && CLUSTER_CTA_SLICES * ctas < S.n_slices) ctas *= 2;
+    /* a shape with an eighth of its slices to spare, so that the CTAs can be balanced by slots
+     * (log of 6,000 poses, 11.75 slices per CTA: 3.84 us per iteration in 12-slice CTAs, 3.32 in
+     * 16-slice ones) */
+    const unsigned shapes = 8 * S.n_slices <= 7 * 12 * ctas ? 15 : 8 * S.n_slices <= 7 * 16 * ctas ? 14 : 12;
     gslam_cluster_part part;
     std::vector<int> lcol(S.n_slots, 0), keep(S.n_slices, 0), pos(S.n_slices, 0);
-    if (max_ctas == 0 || !gslam_cluster_plan(S, 0, S.n_slices, ctas, 8, GSLAM_RES_SMEM_MAX, &part, &lcol, &keep, &pos))
+    if (max_ctas == 0 || !gslam_cluster_plan(S, 0, S.n_slices, ctas, shapes, 8, GSLAM_RES_SMEM_MAX, &part, &lcol, &keep, &pos))
         return GSLAM_OK;
     /* the grid-wide solver's CTAs that own slices (the order of its sums) */
     int vctas = 0;

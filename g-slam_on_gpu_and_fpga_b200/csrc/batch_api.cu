@@ -28,6 +28,10 @@
 
 static int batch_clusters_build(gslam_graph *g, bool fp32);
 
+/* CTA shapes of 12, 20 and 40 slices: the 16-slice one would only split the launches further
+ * (solve of the 64 graphs below, ms: 8.9 without it, 9.6 with it; 9.1 without the 12-slice one) */
+#define GSLAM_BATCH_SHAPES 13u
+
 static int batch_partition(gslam_graph *g) {
     BatchState &B = *g->batch;
     const gslam_structure &S = g->S;
@@ -214,7 +218,8 @@ int gslam_create_se2_batch(const gslam_se2_graph *graphs, uint32_t n_graphs, con
  * better than many sparse ones, so each takes the smallest cluster with 20 slices per CTA in
  * FP64, 40 in FP32 (about what shared memory holds), or 16 CTAs. Ms of solve per round, 64
  * graphs of 500 to 17,000 poses, 10 / 20 / 30 / 40 slices: FP64 14.3 / 10.3 / 11.4 / 11.9, FP32
- * - / 8.4 / 8.1 / 7.7; the grid-wide batch solver takes 23.8 and 15.8; cluster sizes that are no
+ * - / 8.4 / 8.1 / 7.7 (8.9 and 6.7 since the sums are shorter); the grid-wide batch solver takes
+ * 23.8 and 15.8; cluster sizes that are no
  * power of two, or higher stream priorities for larger graphs, gain nothing. While twice as
  * many CTAs still run at once, every cluster is doubled, down to four slices per CTA. Launches
  * of equal cluster shape run side by side on their own streams, the largest clusters first,
@@ -234,7 +239,7 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
     std::vector<int> lcol(S.n_slots, 0), keep(S.n_slices, 0), pos(S.n_slices, 0), ctas(G, 0);
     auto first = [&](int q) { return B.pose_off[q] / 32; };
     auto plan = [&](int q, int c) {
-        return gslam_cluster_plan(S, first(q), first(q + 1), c, elem, GSLAM_RES_SMEM_MAX, &part[q], &lcol, &keep, &pos);
+        return gslam_cluster_plan(S, first(q), first(q + 1), c, GSLAM_BATCH_SHAPES, elem, GSLAM_RES_SMEM_MAX, &part[q], &lcol, &keep, &pos);
     };
     int64_t used = 0;
     for (int q = 0; q < G; q++) {

@@ -34,13 +34,15 @@ bool fill(const gslam_structure &S, int sl0, int sl1, int ctas, int cap, int64_t
 
 }  // namespace
 
-bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, int elem, int64_t budget,
+bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, unsigned shapes, int elem, int64_t budget,
                         gslam_cluster_part *part, std::vector<int> *lcol, std::vector<int> *keep, std::vector<int> *pos) {
     const int ns = sl1 - sl0;
     if (ns < ctas || ns > ctas * GSLAM_CLUSTER_SLICES) return false;
     part->ctas = ctas;
-    part->shape = ns <= 10 * ctas ? 0 : ns <= 20 * ctas ? 1 : 2;
-    const int cap = 10 << part->shape;
+    static const int slices[] = { 12, 16, 20, GSLAM_CLUSTER_SLICES };
+    part->shape = 0;
+    while (!(shapes >> part->shape & 1) || ns > slices[part->shape] * ctas) part->shape++;
+    const int cap = slices[part->shape];
     int64_t lo = 0, hi = S.slice_ptr[sl1] - S.slice_ptr[sl0];
     for (int sl = sl0; sl < sl1; sl++) lo = std::max(lo, S.slice_ptr[sl + 1] - S.slice_ptr[sl]);
     while (lo < hi) {
@@ -51,7 +53,7 @@ bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, in
     if (!fill(S, sl0, sl1, ctas, cap, lo, &part->bounds)) return false;
     int most = 0;
     for (int r = 0; r < ctas; r++) most = std::max(most, part->bounds[r + 1] - part->bounds[r]);
-    part->threads = 32 * (part->shape == 2 ? (most + 1) / 2 : most);
+    part->threads = 32 * (part->shape == 3 ? (most + 1) / 2 : most);
     /* local columns and halos; the rows each CTA reads from others */
     part->n_halo.assign(ctas, 0);
     std::vector<std::vector<int>> halo(ctas);

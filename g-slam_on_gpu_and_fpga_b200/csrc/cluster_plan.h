@@ -19,12 +19,13 @@ struct gslam_cluster_part {
     std::vector<unsigned> exp;           /* rank << 20 | halo slot */
 };
 
-/* Splits the slices [sl0, sl1) over a cluster of `ctas` CTAs for values of `elem` bytes;
+/* Splits the slices [sl0, sl1) over a cluster of `ctas` CTAs for values of `elem` bytes, in the
+ * first of the allowed shapes (bits of `shapes`; the last one always is) that has room;
  * lcol (all slots of the layout) gets the graph's CTA-local columns, keep and pos (all its
  * slices) the block positions in shared memory and where they start. False when the graph
  * does not fit (more rows than the threads own, or the fixed parts of a CTA's shared
  * memory exceed the budget); *part and the graph's part of the arrays are then undefined. */
-bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, int elem, int64_t budget,
+bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, unsigned shapes, int elem, int64_t budget,
                         gslam_cluster_part *part, std::vector<int> *lcol, std::vector<int> *keep, std::vector<int> *pos);
 
 #endif

@@ -588,14 +588,17 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
     }
 }
 
-/* The kernel's shapes: up to 10, 20 and 40 slices per CTA. One row per thread and 10 warps have
- * the registers for everything; 20 warps (96 registers) hide more latency than 10 warps of
- * two rows each (64-graph batch: 11.1 ms of solve per round against 12.9). */
+/* The kernel's shapes: up to 12, 16, 20 and 40 slices per CTA. One row per thread and 12 warps
+ * have the registers for everything, 16 warps nearly (us per iteration in 384, 512, 640 threads:
+ * 2.47, -, 2.59 at 5,120 poses; -, 2.99, 3.19 at 7,120); 20 warps (96 registers) hide more
+ * latency than 10 warps of two rows each (64-graph batch: 11.1 ms of solve per round against
+ * 12.9). */
 template <typename T, bool ONE, bool BATCH>
 static const void *fn_of(int shape) {
     switch (shape) {
-    case 0: return (const void *)k_pcg_cluster<T, 320, 1, ONE, BATCH>;
-    case 1: return (const void *)k_pcg_cluster<T, 640, 1, ONE, BATCH>;
+    case 0: return (const void *)k_pcg_cluster<T, 384, 1, ONE, BATCH>;
+    case 1: return (const void *)k_pcg_cluster<T, 512, 1, ONE, BATCH>;
+    case 2: return (const void *)k_pcg_cluster<T, 640, 1, ONE, BATCH>;
     default: return (const void *)k_pcg_cluster<T, 640, 2, ONE, BATCH>;
     }
 }
@@ -640,10 +643,10 @@ cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jo
 int pcg_cluster_max_ctas(int device, size_t smem_bytes) {
     (void)device;
     int best = 0;
-    for (int v = 0; v < CLUSTER_KINDS * 6; v++) {
+    for (int v = 0; v < CLUSTER_KINDS * 8; v++) {
         const bool one = v % 2 != 0;
-        const int shape = v / 2 % 3, threads = shape == 0 ? 320 : 640;
-        const void *fn = cluster_fn(v / 6, shape, one);
+        const int shape = v / 2 % 4, threads = shape == 0 ? 384 : shape == 1 ? 512 : 640;
+        const void *fn = cluster_fn(v / 8, shape, one);
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess ||
             cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();

@@ -60,7 +60,7 @@ def test_one_cta_gives_the_grid_solvers_bits(pkg, synth, kind, n):
     assert_bitwise(xa, xb, f"{kind} n={n}")
 
 
-@pytest.mark.parametrize("n", [417, 449, 1025, 2049, 4608, 4609])
+@pytest.mark.parametrize("n", [417, 449, 1025, 2049, 4608, 4609, 5376, 5377, 7168, 7169])
 @pytest.mark.parametrize("kind", ["se2", "far", "log"])
 def test_cluster_takes_the_grid_solvers_iterates(pkg, synth, kind, n):
     opts = dict(tol=0.0, max_iter=60)
