@@ -83,6 +83,13 @@ __device__ __forceinline__ void load_tile_wait() {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+/* Programmatic launches: the next kernel's CTAs may start as this one's drain, and wait, before
+ * they touch memory, until it has ended and its writes are visible. The row panel lets the
+ * update's CTAs in from its start; the other way round they would take the slots of the
+ * update's last tiles (n = 2,400: 1.73 ms without, 1.57, 1.60 both ways). */
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 /* U = A[:, K] (n x 64, ld 64) */
 __global__ void k_gj_copy_col(int n, const double *__restrict__ A, int k0, double *__restrict__ U) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -111,8 +118,11 @@ __global__ void k_gj_copy_col(int n, const double *__restrict__ A, int k0, doubl
  * 32 shuffles), and forms p = 1 / f_i itself; lane c != i scales its pivot-row entry
  * a = T[i][c] p and subtracts f_r a from its other rows, lane i's column becomes -f_r p
  * with p on the diagonal (the same update, with a = p and the old entries taken as 0, so
- * the warp does not diverge). */
-__device__ __forceinline__ void inv16_warp(double *m, int ld, double *buf) {
+ * the warp does not diverge). One copy for its four calls: the pivot block is inverted once a
+ * launch, and fetching four copies of the straight-line code took 2 us of its 20 (n = 640: 32.1
+ * us a step, 30.8 so). */
+__device__ __noinline__ void inv16_warp(double *m, int ld, double *buf) {
+    __builtin_assume(__isShared(m)); __builtin_assume(__isShared(buf));
     const int lane = threadIdx.x & 31, c = lane & 15;
     double T[16];
 #pragma unroll
@@ -251,6 +261,8 @@ __global__ void __launch_bounds__(128) k_gj_row_panel(int n, double *__restrict_
     extern __shared__ __align__(16) double sm[];
     double *sA = sm, *sB = sm + GJ_B * GJ_LD;
     const int tj = blockIdx.x, c0 = 16 * blockIdx.y;
+    pdl_next();
+    pdl_wait();
     if (64 * tj == k0) return;
     const bool next = (64 * tj == k0 + GJ_B);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
@@ -323,6 +335,7 @@ __global__ void __launch_bounds__(128) k_gj_update(int n, double *__restrict__ A
     const int ti = ((int)blockIdx.y + kn) % nt, tj = ((int)blockIdx.x + kn) % nt;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wm = warp >> 1, wn = warp & 1;
     const int gid = lane >> 2, tig = lane & 3;
+    pdl_wait();
     if (64 * ti == k0) {
         if (64 * tj == k0)
             for (int t = threadIdx.x; t < GJ_B * GJ_B; t += blockDim.x)
@@ -433,21 +446,33 @@ static int gj_run(int m, double *d_a, cudaStream_t st, double *scratch) {
         cudaFuncSetAttribute(k_gj_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
     k_gj_copy_col<<<(m * GJ_B + 255) / 256, 256, 0, st>>>(m, d_a, 0, Ub[0]);
     k_gj_diag<<<1, 128, smem, st>>>(Ub[0], 0, Pb[0]);
     for (int k = 0; k < nt; k++) {
         const int k0 = GJ_B * k;
         double *U = Ub[k & 1], *Un = Ub[(k + 1) & 1];
         double *P = Pb[k & 1], *Pn = Pb[(k + 1) & 1];
-        k_gj_row_panel<<<dim3(nt, 4), 128, smem, st>>>(m, d_a, k0, P, Un);
-        k_gj_update<<<dim3(nt, nt), 128, smem, st>>>(m, d_a, k0, U, P, Un, Pn, ps);
+        cfg.gridDim = dim3(nt, 4);
+        if (cudaLaunchKernelEx(&cfg, k_gj_row_panel, m, d_a, k0, (const double *)P, Un) != cudaSuccess) return GSLAM_ERR_CUDA;
+        cfg.gridDim = dim3(nt, nt);
+        if (cudaLaunchKernelEx(&cfg, k_gj_update, m, d_a, k0, (const double *)U, (const double *)P, Un, Pn, ps) != cudaSuccess)
+            return GSLAM_ERR_CUDA;
     }
     return cudaGetLastError() == cudaSuccess ? GSLAM_OK : GSLAM_ERR_CUDA;
 }
 
 /* The inverse of the padded matrix, handed to `use` (launches on st) before it is freed. One
  * allocation per call holds the matrix and the scratch: allocating and freeing is a large part of
- * a call (n = 2,400: 2.5 ms a solve with one, 3.8 with three). `ms`: the elimination's time. */
+ * a call (n = 2,400: 2.5 ms a solve with one, 3.8 with three; 2.3 with programmatic launches). `ms`: the elimination's time. */
 template <typename F>
 static int gj_padded(int n, const double *d_a, int lda, cudaStream_t st, float *ms, const char *what, F use) {
     const int m = (n + GJ_B - 1) / GJ_B * GJ_B;
