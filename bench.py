@@ -465,7 +465,7 @@ def batch_sample(G, torch, rounds, world, rank, dist):
     val = {name: len(graphs) * rounds / (out[name]["ms"] * 1e-3) for name in out}
     return {"graphs": len(graphs), "poses": int(sum(g.init.shape[0] for g in graphs)),
             "value": round(val["mixed"], 2), "fp64_value": round(val["fp64"], 2),
-            "unit": "graph GN iters/s (all graphs, one persistent launch per PCG pass)",
+            "unit": "graph GN iters/s (all graphs, one thread-block cluster per graph and PCG pass)",
             "ms_per_round": round(out["mixed"]["ms"] / rounds, 3),
             "fp64_ms_per_round": round(out["fp64"]["ms"] / rounds, 3),
             "pcg_iterations_mean": out["mixed"]["its"], "fp64_pcg_iterations_mean": out["fp64"]["its"],

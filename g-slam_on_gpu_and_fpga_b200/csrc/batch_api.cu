@@ -6,7 +6,8 @@
  * No counterpart in the reference, which solves one graph per process and sweeps
  * lambda with a shell loop (README.md:137-160). A batch is one block-diagonal graph:
  * every graph's poses padded to whole 32-row slices, its own lambda and anchor, its own
- * PCG scalars inside one persistent launch of batch.cu's solver.
+ * PCG scalars: in a thread-block cluster of its own (pcg_cluster.cu) if it fits one, else in
+ * one persistent launch of batch.cu's solver.
  */
 #include <cuda_runtime.h>
 
@@ -219,9 +220,9 @@ int gslam_create_se2_batch(const gslam_se2_graph *graphs, uint32_t n_graphs, con
  * FP64, 40 in FP32 (about what shared memory holds), or 16 CTAs. Ms of solve per round, 64
  * graphs of 500 to 17,000 poses, 10 / 20 / 30 / 40 slices: FP64 14.3 / 10.3 / 11.4 / 11.9, FP32
  * - / 8.4 / 8.1 / 7.7 (8.9 and 6.7 since the sums are shorter); the grid-wide batch solver takes
- * 23.8 and 15.8; cluster sizes that are no
- * power of two, or higher stream priorities for larger graphs, gain nothing. While twice as
- * many CTAs still run at once, every cluster is doubled, down to four slices per CTA. Launches
+ * 23.8 and 15.8; cluster sizes that are no power of two, 40 slices per CTA for the smaller
+ * graphs alone, or higher stream priorities for larger graphs, gain nothing. While twice as many
+ * CTAs still run at once, every cluster is doubled, down to four slices per CTA. Launches
  * of equal cluster shape run side by side on their own streams, the largest clusters first,
  * and the GPU starts the next cluster as one ends; the graphs of a launch come in order of
  * falling size, so the last to start are short.

@@ -40,8 +40,8 @@
  * memory only.
  *
  * Measured, us per iteration (before: a barrier counter with a release fence and z, u, v
- * of every row published), same bits. FP32: 2.7 (4.5) at N = 20,000, 2.9 (4.8) at 50,000,
- * 4.45 (5.9) at 100,000. FP64: 2.9 (6.2), 3.8 (7.6), 6.3 (11.8). Up to 50,000 the
+ * of every row published), same bits. FP32: 2.7 (4.5) at N = 20,000, 2.7 (4.8) at 50,000,
+ * 4.3 (5.9) at 100,000. FP64: 2.9 (6.2), 3.6 (7.6), 6.1 (11.8). Up to 50,000 the
  * all-reduce of three doubles (1.5 us) bounds it, at 100,000 the SpMV from shared memory
  * and, in FP64, D^-1 from L2.
  *

@@ -33,8 +33,8 @@
  * p.q, which every reader enters after it has read the old one.
  *
  * Measured, us per iteration (before: a barrier counter with a release fence, p published
- * too, one row per thread): 3.4 (7.6) at N = 2,001, 3.7 (8.3) at 20,000, 4.4 (8.9) at
- * 50,000, 6.4 (12.7) at 100,000, 8.4 (16.6) at 140,000; the two all-reduces take about 2.6
+ * too, one row per thread): 3.15 (7.6) at N = 2,001, 3.5 (8.3) at 20,000, 4.25 (8.9) at
+ * 50,000, 5.95 (12.7) at 100,000, 7.9 (16.6) at 140,000; the two all-reduces take about 2.5
  * of it. Sums and their order are unchanged, and so are the results' bits: each scalar row
  * of q adds its blocks in ascending original column order with separate multiply and add.
  */

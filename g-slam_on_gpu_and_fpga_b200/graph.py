@@ -310,8 +310,8 @@ class PoseGraph:
 
 class PoseGraphBatch(PoseGraph):
     """Many independent SE(2) graphs on one handle (gslam_create_se2_batch): one
-    Gauss-Newton round of every graph per `round()`, their linear solves in one
-    persistent launch with per-graph scalars. Poses of graph q are
+    Gauss-Newton round of every graph per `round()`, each linear solve in a thread-block
+    cluster of its own (graphs above 20,480 rows in one grid-wide launch). Poses of graph q are
     `poses[offsets[q] : offsets[q] + sizes[q]]` of the concatenation."""
 
     @classmethod

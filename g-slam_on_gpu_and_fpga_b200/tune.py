@@ -1,9 +1,10 @@
 """Autotuner for the batched solver's launch and layout shapes.
 
-The batched PCG streams the matrix, so its speed depends on three choices that are
-fixed when a batch is built: threads per CTA (how many slices a CTA works on at
-once), CTAs per SM (latency hiding against barrier cost) and the row-sorting window
-of the sliced block layout (padding vs. how evenly slices fill a warp). The tuner
+Three choices are fixed when a batch is built: the row-sorting window of the sliced
+block layout (padding vs. how evenly slices fill a warp), and, for the graphs that the
+grid-wide solver takes (above 20,480 rows; it streams the matrix), threads per CTA (how
+many slices a CTA works on at once) and CTAs per SM (latency hiding against barrier
+cost); the cluster solver picks its own CTAs. The tuner
 builds the batch for every candidate, times a fixed number of PCG iterations with
 no early stop (CUDA events inside the library), and returns the fastest.
 

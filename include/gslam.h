@@ -58,8 +58,8 @@ typedef struct gslam_opts {
     double tol;           /* relative residual tolerance; reference 1e-6 (MatrixOps.c:345) */
     int max_iter;         /* PCG iteration cap; reference 500 (MatrixOps.c:347) */
     int sell_window;      /* rows sorted by block count inside windows of this size; 0 = auto */
-    int threads_per_cta;  /* persistent PCG block size; 0 = auto */
-    int ctas_per_sm;      /* persistent PCG CTAs per SM; 0 = auto (occupancy) */
+    int threads_per_cta;  /* streamed and grid-wide batch PCG: block size; 0 = auto */
+    int ctas_per_sm;      /* the same solvers' CTAs per SM; 0 = auto (occupancy) */
     int angle_wrap;       /* wrap theta to (-pi, pi] in the pose update; 0 for the reference */
     double inner_tol;     /* mixed: inner FP32 relative tolerance per refinement step */
     int inner_max_iter;   /* mixed: inner iteration cap per refinement step */
@@ -67,7 +67,8 @@ typedef struct gslam_opts {
     int device;           /* CUDA device ordinal; -1 = current */
     double barrier_timeout_ms; /* a solver barrier gives up after this long; 0 = 2000 ms */
     int test_absent_cta;  /* test hook: this solver CTA never arrives at its first barrier, so
-                             the others time out (checks the bounded wait); -1 = off */
+                             the others time out (checks the bounded wait); a number no launch
+                             has: the grid-wide solver, nothing absent; -1 = off */
     int disable_resident; /* 1: never stage the matrix in shared memory (streamed solver only) */
     int round_graph;      /* 1: gslam_round replays the whole round (linearise, assemble,
                              block-Jacobi, solve, pose update, read-backs) as one CUDA graph,
@@ -313,9 +314,10 @@ int gslam_landmark_map(gslam_graph *g, uint32_t *n_landmarks, uint32_t *ids, dou
  * gives the first padded pose of every graph (pose_offset[n_graphs] = total), so
  * gslam_get_poses / gslam_set_poses work on the concatenation.
  *
- * gslam_batch_round: one Gauss-Newton round of every graph; the linear solves run in
- * ONE persistent launch (block-Jacobi PCG with each graph's own alpha, beta and
- * stopping test, tol / max_iter of the handle's options, FP64). per_graph (host,
+ * gslam_batch_round: one Gauss-Newton round of every graph; each linear solve runs in a
+ * thread-block cluster of its own, and what does not fit one in ONE grid-wide launch
+ * (block-Jacobi PCG with each graph's own alpha, beta and stopping test, tol / max_iter of
+ * the handle's options, FP64). per_graph (host,
  * n_graphs entries, may be NULL) receives each graph's iterations, reason, relative
  * residual and update norm diff = ||dx|| / sqrt(3 n_poses). gslam_round on a batch
  * runs the same round and reports the largest iteration count and residual.
