@@ -146,14 +146,10 @@ static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t s
     DevMem &m = L->mem;
     std::vector<ClusterJob> job(1);
     job[0] = ClusterJob{ 0, 0, S.n_slices, 0, 0, 0, part.halo_max };
-    CK(dupload(m, st, &L->cluster_job, job));
-    CK(dupload(m, st, &L->cluster_bounds, part.bounds));
-    CK(dupload(m, st, &L->cluster_halo, part.n_halo));
-    CK(dupload(m, st, &L->cluster_lcol, lcol));
-    CK(dupload(m, st, &L->cluster_keep, keep));
-    CK(dupload(m, st, &L->cluster_pos, pos));
-    CK(dupload(m, st, &L->cluster_exp_ptr, part.exp_ptr));
-    CK(dupload(m, st, &L->cluster_exp, part.exp));
+    CK(dupload_all(m, st, { dpart(&L->cluster_job, job), dpart(&L->cluster_bounds, part.bounds),
+                            dpart(&L->cluster_halo, part.n_halo), dpart(&L->cluster_lcol, lcol),
+                            dpart(&L->cluster_keep, keep), dpart(&L->cluster_pos, pos),
+                            dpart(&L->cluster_exp_ptr, part.exp_ptr), dpart(&L->cluster_exp, part.exp) }));
     L->cluster_ctas = part.ctas;
     L->cluster_threads = part.threads;
     L->cluster_shape = part.shape;
@@ -327,8 +323,6 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
             if (fit_res && !o.disable_resident) {
                 L->resident = true;
                 L->smem_bytes = (size_t)end_res;
-                CK(dupload(m, st, &L->res_keep, keep[0]));
-                CK(dupload(m, st, &L->res_pos, pos[0]));
                 const int rc = cluster_upload(L, S, st, device, cs);
                 if (rc != GSLAM_OK) return rc;
             }
@@ -337,25 +331,22 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
             if (fit32) {
                 L->mixed_ok = true;
                 L->mixed_smem_bytes = (size_t)end32;
-                CK(dupload(m, st, &L->mixed_keep, keep[1]));
-                CK(dupload(m, st, &L->mixed_pos, pos[1]));
             }
             if (fit64) {
                 L->cg_ok = true;
                 L->cg_smem_bytes = (size_t)end64;
-                CK(dupload(m, st, &L->cg_keep, keep[2]));
-                CK(dupload(m, st, &L->cg_pos, pos[2]));
             }
             if (L->resident || L->mixed_ok || L->cg_ok) {
-                CK(dupload(m, st, &L->lcol, lcol));
-                CK(dupload(m, st, &L->halo_ptr, hptr));
                 /* only rows that some CTA reads as halo are published in global memory */
                 std::vector<unsigned char> exported((size_t)std::max(32 * L->n_slices, 1), 0);
                 for (int r : hrows)
                     if (r >= 0 && (size_t)r < exported.size()) exported[(size_t)r] = 1;
-                CK(dupload(m, st, &L->row_export, exported));
                 if (hrows.empty()) hrows.push_back(0);
-                CK(dupload(m, st, &L->halo_rows, hrows));
+                CK(dupload_all(m, st, { dpart(&L->res_keep, keep[0]), dpart(&L->res_pos, pos[0]),
+                                        dpart(&L->mixed_keep, keep[1]), dpart(&L->mixed_pos, pos[1]),
+                                        dpart(&L->cg_keep, keep[2]), dpart(&L->cg_pos, pos[2]), dpart(&L->lcol, lcol),
+                                        dpart(&L->halo_ptr, hptr), dpart(&L->row_export, exported),
+                                        dpart(&L->halo_rows, hrows) }));
             }
         }
     }

@@ -296,15 +296,10 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
     }
     if (!jobs.empty()) {
         DevMem &m = g->mem;
-        CK(dupload(m, g->st, &K.d_jobs, jobs));
-        CK(dupload(m, g->st, &K.d_bounds, bounds));
-        CK(dupload(m, g->st, &K.d_halo, halo));
-        CK(dupload(m, g->st, &K.d_lcol, lcol));
-        CK(dupload(m, g->st, &K.d_keep, keep));
-        CK(dupload(m, g->st, &K.d_pos, pos));
-        CK(dupload(m, g->st, &K.d_exp_ptr, exp_ptr));
-        CK(dupload(m, g->st, &K.d_exp, exp));
-        if (!K.all) CK(dupload(m, g->st, &K.d_rest_skip, K.in_cluster)); /* graphs the grid-wide solver leaves alone */
+        CK(dupload_all(m, g->st, { dpart(&K.d_jobs, jobs), dpart(&K.d_bounds, bounds), dpart(&K.d_halo, halo),
+                                   dpart(&K.d_lcol, lcol), dpart(&K.d_keep, keep), dpart(&K.d_pos, pos),
+                                   dpart(&K.d_exp_ptr, exp_ptr), dpart(&K.d_exp, exp),
+                                   dpart(&K.d_rest_skip, K.in_cluster) })); /* the last: what the grid-wide solver leaves alone */
         if (!B.fork) CK(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming));
         while (B.side.size() < K.launches.size()) {
             cudaStream_t t;

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -216,6 +218,31 @@ inline cudaError_t dupload(DevMem &m, cudaStream_t st, T **p, const std::vector<
     if (e != cudaSuccess) return e;
     if (v.empty()) return cudaSuccess;
     return cudaMemcpyAsync(*p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
+}
+
+/* device copies of several host vectors in one allocation, each from a 256-byte boundary: an
+ * allocation costs 0.1 ms on an idle host and milliseconds on a busy one */
+struct DevPart {
+    void **p;
+    const void *v;
+    size_t bytes;
+};
+template <class T>
+inline DevPart dpart(T **p, const std::vector<T> &v) { return DevPart{ (void **)p, v.data(), v.size() * sizeof(T) }; }
+inline cudaError_t dupload_all(DevMem &m, cudaStream_t st, std::initializer_list<DevPart> parts) {
+    size_t end = 0;
+    for (const DevPart &q : parts) end += (q.bytes + 255) / 256 * 256;
+    std::vector<unsigned char> all(end);
+    unsigned char *base = nullptr;
+    cudaError_t e = dalloc(m, &base, end);
+    if (e != cudaSuccess) return e;
+    end = 0;
+    for (const DevPart &q : parts) {
+        if (q.bytes) memcpy(all.data() + end, q.v, q.bytes);
+        *q.p = base + end;
+        end += (q.bytes + 255) / 256 * 256;
+    }
+    return all.empty() ? cudaSuccess : cudaMemcpyAsync(base, all.data(), all.size(), cudaMemcpyHostToDevice, st);
 }
 
 /* an event record that a stream capture keeps as a node of the graph */
