@@ -266,6 +266,7 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
             std::vector<int> lcol(S.n_slots, 0), hptr(rgrid + 1, 0), hrows;
             /* mixed / FP64 one-reduction solvers: every CTA's own layout must fit */
             bool fit32 = true, fit64 = true, fit_res = true;
+            const int rows32 = pcg_mixed_rows(false, L->res_slices), rows64 = pcg_mixed_rows(true, L->res_slices);
             std::vector<int> keep[3], pos[3]; /* FP64 resident, mixed, one-reduction */
             for (int v = 0; v < 3; v++) {
                 keep[v].assign(S.n_slices, 0);
@@ -305,12 +306,13 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 hptr[i + 1] = hptr[i] + (int)rem.size();
                 hrows.insert(hrows.end(), rem.begin(), rem.end());
                 const int64_t nh = (int64_t)rem.size(), nsl = cs[i + 1] - cs[i];
-                const MixedSmem l32 = mixed_smem_layout(4, a1 - a0, nsl, nh, GSLAM_GRID_SMEM_MAX);
-                const MixedSmem l64 = mixed_smem_layout(8, a1 - a0, nsl, nh, GSLAM_GRID_SMEM_MAX);
+                const MixedSmem l32 = mixed_smem_layout(4, a1 - a0, nsl, nh, rows32, GSLAM_GRID_SMEM_MAX);
+                const MixedSmem l64 = mixed_smem_layout(8, a1 - a0, nsl, nh, rows64, GSLAM_GRID_SMEM_MAX);
                 const ResidentSmem lr = resident_smem_layout(a1 - a0, nsl, nh, GSLAM_GRID_SMEM_MAX);
                 fit_res = fit_res && lr.val_cap >= 0;
                 fit32 = fit32 && l32.val_cap >= 0;
                 fit64 = fit64 && l64.val_cap >= 0;
+                if (l32.v_rows < nh || l64.v_rows < nh) L->long_halo = true;
                 share(0, i, lr.val_cap);
                 share(1, i, l32.val_cap);
                 share(2, i, l64.val_cap);
@@ -327,7 +329,7 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 if (rc != GSLAM_OK) return rc;
             }
             /* mixed and one-reduction: values | local columns | z of own and halo rows | v of
-             * halo rows, each CTA's from its own sizes (mixed_smem_layout) */
+             * halo rows as far as it fits, each CTA's from its own sizes (mixed_smem_layout) */
             if (fit32) {
                 L->mixed_ok = true;
                 L->mixed_smem_bytes = (size_t)end32;
@@ -342,6 +344,7 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 for (int r : hrows)
                     if (r >= 0 && (size_t)r < exported.size()) exported[(size_t)r] = 1;
                 if (hrows.empty()) hrows.push_back(0);
+                L->n_halo = hptr[rgrid];
                 CK(dupload_all(m, st, { dpart(&L->res_keep, keep[0]), dpart(&L->res_pos, pos[0]),
                                         dpart(&L->mixed_keep, keep[1]), dpart(&L->mixed_pos, pos[1]),
                                         dpart(&L->cg_keep, keep[2]), dpart(&L->cg_pos, pos[2]), dpart(&L->lcol, lcol),
@@ -390,6 +393,8 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
             L->val32_fresh = true;
         }
     }
+    if ((fused_prec == GSLAM_PREC_MIXED || fused_prec == GSLAM_PREC_FP64_CG) && L->long_halo && !L->halo_v)
+        CK(dalloc(L->mem, &L->halo_v, 4 * (size_t)L->n_halo));
     HostTrace tr;
     launch_diag_inv(st, L->n_rows, L->diag_slot, L->val, L->dinv);
     CK(cudaGetLastError());
@@ -427,11 +432,11 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
     const bool mixed = fused_prec == GSLAM_PREC_MIXED;
     const bool cg = fused_prec == GSLAM_PREC_FP64_CG;
     if (mixed && !L->mixed_ok) {
-        g_last_error = "mixed precision needs the graph's rows to fit the resident layout (<= 32 slices per SM)";
+        g_last_error = "mixed precision needs the graph to fit the resident layout: at most 32 slices per SM, and each SM's columns and the rows they read in its shared memory";
         return GSLAM_ERR_TOO_LARGE;
     }
     if (cg && !L->cg_ok) {
-        g_last_error = "the one-reduction FP64 solver needs the graph's rows to fit the resident layout (<= 32 slices per SM)";
+        g_last_error = "the one-reduction FP64 solver needs the graph to fit the resident layout: at most 32 slices per SM, and each SM's columns and the rows they read in its shared memory";
         return GSLAM_ERR_TOO_LARGE;
     }
     if (cg) {
@@ -462,6 +467,7 @@ static int layout_solve_enqueue(DevLayout *L, cudaStream_t st, const gslam_opts 
     P.halo_ptr = L->halo_ptr;
     P.halo_rows = L->halo_rows;
     P.row_export = L->row_export;
+    P.halo_v = L->halo_v;
     P.res_keep = L->res_keep;
     P.res_pos = L->res_pos;
     P.mixed_keep = L->mixed_keep;

@@ -51,6 +51,11 @@ struct DevLayout {
     int *cta_slice = nullptr;      /* [res_grid + 1] */
     int *lcol = nullptr, *halo_ptr = nullptr, *halo_rows = nullptr; /* CTA-local columns, halo lists */
     unsigned char *row_export = nullptr; /* rows some other CTA's halo lists */
+    /* mixed and one-reduction: some CTA's halo does not fit its shared memory; v of those rows
+     * (made on first use, n_halo rows) */
+    bool long_halo = false;
+    int n_halo = 0;
+    double *halo_v = nullptr;
     size_t smem_bytes = 0;
     bool mixed_ok = false;          /* the mixed solver's shared-memory layout fits */
     size_t mixed_smem_bytes = 0;   /* dynamic shared memory per launch: the largest CTA layout (mixed_smem_layout) */

@@ -86,6 +86,8 @@ struct PcgParams {
     const int *res_keep, *res_pos; /* resident solver, per slice: block positions kept in shared memory, and the
                             * first one's place there (in positions of 288 values) */
     int64_t smem_budget;   /* resident, mixed and FP64 one-reduction solvers: dynamic shared memory per CTA */
+    void *halo_v;          /* mixed and one-reduction: v of the halo rows that shared memory has no room for
+                            * (4 elements per entry of halo_rows), or null */
 };
 
 /* Shared-memory layout of one CTA of the FP64 resident solver, from its own sizes: local
@@ -111,17 +113,22 @@ __host__ __device__ inline ResidentSmem resident_smem_layout(int64_t n_slots, in
 /* Shared-memory layout of one CTA of the mixed / FP64 one-reduction solver, from its own
  * sizes: the fixed parts (local columns, z of own and halo rows, v of halo rows: 16 bytes a
  * row in FP32, 24 in FP64) after the values, and as many values (whole multiples of 288, one
- * block position of a slice) as the budget leaves. val_cap < 0: the fixed parts alone exceed
- * the budget. */
+ * block position of a slice) as the budget leaves. Of a halo too long for it, v of the rows
+ * beyond the first v_rows is in global memory (read and written by one thread of this CTA
+ * each); v of the first `first` rows (the kernel's rows per CTA) never is. val_cap < 0: the
+ * fixed parts alone exceed the budget. */
 struct MixedSmem {
-    int64_t val_cap, col_off, z_off, v_off, end;
+    int64_t val_cap, col_off, z_off, v_off, v_rows, end;
 };
 __host__ __device__ inline MixedSmem mixed_smem_layout(int64_t elem, int64_t n_slots, int64_t n_slices, int64_t n_halo,
-                                                       int64_t budget) {
+                                                       int64_t first, int64_t budget) {
     auto up = [](int64_t b) { return (b + 127) / 128 * 128; };
     const int64_t row_b = elem == 8 ? 24 : 16;
-    const int64_t col_b = up(4 * n_slots), z_b = up(row_b * (32 * n_slices + n_halo)), v_b = up(row_b * n_halo);
+    const int64_t col_b = up(4 * n_slots), z_b = up(row_b * (32 * n_slices + n_halo));
+    const int64_t room = (budget - col_b - z_b) / 128 * 128 / row_b, least = n_halo < first ? n_halo : first;
     MixedSmem m;
+    m.v_rows = room >= n_halo ? n_halo : room > least ? room : least;
+    const int64_t v_b = up(row_b * m.v_rows);
     const int64_t fixed = col_b + z_b + v_b;
     m.val_cap = budget >= fixed ? (budget - fixed) / elem / 288 * 288 : -1;
     const int64_t nv = m.val_cap > 9 * n_slots ? 9 * n_slots : m.val_cap;
@@ -279,6 +286,8 @@ int pcg_cluster_max_ctas(int device, size_t smem_bytes);
 cudaError_t launch_pcg_mixed(cudaStream_t st, const PcgParams &p, int grid, int max_slices, size_t smem_bytes,
                              bool fp64);
 int pcg_mixed_max_grid(int device, size_t smem_bytes);
+/* rows that a CTA of the launch has threads for, when the largest CTA owns max_slices slices */
+int pcg_mixed_rows(bool fp64, int max_slices);
 
 /* Standalone SpMV y = A x on padded new-order vectors (FP64 or FP32 values). */
 void launch_spmv64(cudaStream_t st, int n_rows, int n_slices, const int64_t *slice_ptr,

@@ -33,7 +33,8 @@
  * Shared memory holds, per CTA: its matrix share (of a share that does not fit
  * every slice leaves out its last block positions, read from L2), CTA-local column
  * indices (own rows first, then the CTA's halo: the other CTAs' rows its blocks
- * touch, a list fixed at setup), z of its own and halo rows and the halo's v. Each
+ * touch, a list fixed at setup), z of its own and halo rows and the halo's v (of a halo
+ * of thousands of rows, as far as it fits; the rest in global memory). Each
  * thread owns one or two rows and keeps r, z, s, v, w, u, p, d in registers, and
  * D^-1 where they suffice. Thread 0 alone advances the scalar recurrence while the
  * others fetch the halo's u. The SpMV reads values, columns and z from shared
@@ -234,11 +235,13 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
     /* dynamic shared memory, laid out per CTA from its own sizes (mixed_smem_layout, the
      * host's feasibility check uses the same function): T values as far as they fit |
      * local columns | z of own + halo rows | v of halo rows */
-    const MixedSmem ml = mixed_smem_layout(sizeof(T), slot1 - slot0, s1 - s0, n_halo, P.smem_budget);
+    const MixedSmem ml = mixed_smem_layout(sizeof(T), slot1 - slot0, s1 - s0, n_halo, R * BS, P.smem_budget);
     const int64_t nsm = nval < ml.val_cap ? nval : ml.val_cap;
     T *sval = reinterpret_cast<T *>(smem);
     int *scol = reinterpret_cast<int *>(smem + ml.col_off);
-    const Rows<T> sz(smem + ml.z_off, n_loc + n_halo), shv(smem + ml.v_off, n_halo);
+    const int n_shv = (int)ml.v_rows;
+    const Rows<T> sz(smem + ml.z_off, n_loc + n_halo), shv(smem + ml.v_off, n_shv);
+    auto far_v = [&]() { return static_cast<T *>(P.halo_v); }; /* v of halo rows n_shv and up, at h0 + row */
 
     if (threadIdx.x == 0) {
         tma_mbar_init(&s_bar, 1);
@@ -372,7 +375,8 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
         if (!grid_barrier(P.gs, (unsigned)(++epoch), P.spin_limit, &s_ok)) { timed_out = true; break; }
         for (int h = hh; h < n_halo; h += BS) {
             sz.put(n_loc + h, ldcgt3(Inner<T>::z0(P), __ldg(P.halo_rows + h0 + h)));
-            shv.put(h, zero);
+            if (h < n_shv) shv.put(h, zero);
+            else stt3(far_v(), h0 + h, zero);
         }
 #pragma unroll
         for (int i = 0; i < R; i++) hu[i] = zero;
@@ -393,7 +397,14 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
             for (int h = hh + R * BS; h < n_halo; h += BS) {
                 T3<T> uh = zero;
                 if (k > 0 && !get_row(Inner<T>::u(P, seq & 1), __ldg(P.halo_rows + h0 + h), seq, P.gs, P.spin_limit, &uh)) s_ok = 0;
-                halo_step(h, uh);
+                if (h < n_shv) {
+                    halo_step(h, uh);
+                } else {
+                    T3<T> zn, vn;
+                    step_zv(sz.get(n_loc + h), uh, ldcgt3(far_v(), h0 + h), alpha, beta, zn, vn);
+                    sz.put(n_loc + h, zn);
+                    stt3(far_v(), h0 + h, vn);
+                }
             }
             /* own rows: s_{k-1}, r_k, p_{k-1}, d, then v_{k-1}, z_k */
 #pragma unroll
@@ -586,6 +597,14 @@ static const MixKernel *mix_kernels(bool fp64, int *n) {
     };
     *n = (int)(fp64 ? sizeof d / sizeof d[0] : sizeof f / sizeof f[0]);
     return fp64 ? d : f;
+}
+
+int pcg_mixed_rows(bool fp64, int max_slices) {
+    int n;
+    const MixKernel *k = mix_kernels(fp64, &n);
+    for (int i = 0; i < n; i++)
+        if (max_slices <= k[i].max_slices) return 32 * k[i].max_slices;
+    return 0;
 }
 
 cudaError_t launch_pcg_mixed(cudaStream_t st, const PcgParams &p, int grid, int max_slices, size_t smem_bytes, bool fp64) {
