@@ -109,12 +109,13 @@ void DevMem::release() {
     ptrs.clear();
 }
 
-/* The cluster solver's plan of a single graph, where it is the faster one. Us per iteration,
- * cluster / grid-wide solver: 1.5 / 3.1 at 100 poses, 2.0 / 3.1 at 800, 2.1 / 3.15 at 2,001,
- * 2.3 / 3.3 at 4,000, 3.0 / 3.4 at 7,120, 3.4 / 3.4 at 8,000 (city walks; with twice the
- * closures, some far, 3.4 / 3.6 at 7,120 and 4.0 / 3.6 at 8,000); landmark logs, with longer
- * rows, 2.6 / 3.7 at 2,001, 2.9 / 3.8 at 4,000, 3.4 / 3.9 at 7,120: up to 224 slices (7,168 rows),
- * 14 per CTA.
+/* The cluster solver's plan of a single graph, unless the grid-wide solver is the faster one by
+ * their estimates (resident_us: the grid-wide one's). Us per iteration, cluster / grid-wide: city walks 1.5 / 3.1 at
+ * 100 poses, 2.0 / 3.1 at 800, 2.3 / 3.3 at 4,000, 3.0 / 3.4 at 7,120, 3.4 / 3.4 at 8,000;
+ * landmark logs 2.7 / 3.7 at 2,001, 3.5 / 3.9 at 7,120: up to 224 slices (7,168 rows), 14 per CTA.
+ * Long rows, whose values do not fit sixteen SMs, and closures to random poses, whose halos are sent
+ * row by row, go the other way: a log of 7,120 poses with 96,000 edges 11.1 / 6.2, walks of
+ * 6,000 poses with 1 and 8 random closures per pose 6.6 / 3.7 and 20.1 / 5.9.
  * One CTA up to 13 slices: such a solve can go past convergence within its 500 iterations,
  * where rounding decides the iterates, and one CTA adds in the grid-wide solver's order (1.5
  * at 100 poses). Then four slices per CTA (a warp per SM sub-partition) up to 16 CTAs: 2.55 at
@@ -124,7 +125,7 @@ void DevMem::release() {
 #define CLUSTER_MAX_SLICES 224
 
 static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, int device,
-                          const std::vector<int> &grid_slices) {
+                          const std::vector<int> &grid_slices, double resident_us) {
     if (S.n_slices > CLUSTER_MAX_SLICES) return GSLAM_OK;
     const int max_ctas = pcg_cluster_max_ctas(device, GSLAM_RES_SMEM_MAX);
     int ctas = 1;
@@ -138,6 +139,7 @@ static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t s
     std::vector<int> lcol(S.n_slots, 0), keep(S.n_slices, 0), pos(S.n_slices, 0);
     if (max_ctas == 0 || !gslam_cluster_plan(S, 0, S.n_slices, ctas, shapes, 8, GSLAM_RES_SMEM_MAX, &part, &lcol, &keep, &pos))
         return GSLAM_OK;
+    if (gslam_cluster_us(part, 8) > 1.1 * resident_us) return GSLAM_OK; /* 1.1: no change of solver at a tie */
     /* the grid-wide solver's CTAs that own slices (the order of its sums) */
     int vctas = 0;
     for (size_t c = 0; c + 1 < grid_slices.size(); c++)
@@ -266,6 +268,7 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
             std::vector<int> lcol(S.n_slots, 0), hptr(rgrid + 1, 0), hrows;
             /* mixed / FP64 one-reduction solvers: every CTA's own layout must fit */
             bool fit32 = true, fit64 = true, fit_res = true;
+            int most_positions = 0, most_left = 0, most_halo = 0; /* of a CTA of the FP64 resident solver */
             const int rows32 = pcg_mixed_rows(false, L->res_slices), rows64 = pcg_mixed_rows(true, L->res_slices);
             std::vector<int> keep[3], pos[3]; /* FP64 resident, mixed, one-reduction */
             for (int v = 0; v < 3; v++) {
@@ -314,6 +317,10 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 fit64 = fit64 && l64.val_cap >= 0;
                 if (l32.v_rows < nh || l64.v_rows < nh) L->long_halo = true;
                 share(0, i, lr.val_cap);
+                const int positions = (int)((a1 - a0) / 32);
+                most_positions = std::max(most_positions, positions);
+                most_left = std::max(most_left, positions - (int)std::min<int64_t>(positions, std::max<int64_t>(lr.val_cap, 0) / 288));
+                most_halo = std::max(most_halo, (int)nh);
                 share(1, i, l32.val_cap);
                 share(2, i, l64.val_cap);
                 end_res = std::max(end_res, lr.end);
@@ -325,7 +332,7 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
             if (fit_res && !o.disable_resident) {
                 L->resident = true;
                 L->smem_bytes = (size_t)end_res;
-                const int rc = cluster_upload(L, S, st, device, cs);
+                const int rc = cluster_upload(L, S, st, device, cs, gslam_resident_us(most_positions, most_left, most_halo));
                 if (rc != GSLAM_OK) return rc;
             }
             /* mixed and one-reduction: values | local columns | z of own and halo rows | v of

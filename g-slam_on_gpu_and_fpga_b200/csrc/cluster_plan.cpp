@@ -89,8 +89,9 @@ bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, un
     for (int r = 0; r < ctas; r++)
         for (int h = 0; h < part->n_halo[r]; h++)
             part->exp[at[halo[r][h] - row_base]++] = (unsigned)r << 20 | (unsigned)h;
-    /* shared memory */
+    /* shared memory, and what sets the iteration's time */
     part->smem = 0;
+    part->positions = part->left = part->sent = part->width = 0;
     for (int r = 0; r < ctas; r++) {
         const int64_t n_slots = S.slice_ptr[part->bounds[r + 1]] - S.slice_ptr[part->bounds[r]];
         const ClusterSmem m = cluster_smem_layout(elem, n_slots, part->bounds[r + 1] - part->bounds[r], part->n_halo[r],
@@ -104,6 +105,16 @@ bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, un
         while (out > 0)
             for (int sl = a; sl < b && out > 0; sl++)
                 if ((*keep)[sl] > 0) { (*keep)[sl]--; out--; }
+        int positions = 0, kept = 0;
+        for (int sl = a; sl < b; sl++) {
+            const int width = (int)((S.slice_ptr[sl + 1] - S.slice_ptr[sl]) / 32);
+            positions += width;
+            kept += (*keep)[sl];
+            part->width = std::max(part->width, width);
+        }
+        part->positions = std::max(part->positions, positions);
+        part->left = std::max(part->left, positions - kept);
+        part->sent = std::max(part->sent, part->exp_ptr[32 * (b - sl0)] - part->exp_ptr[32 * (a - sl0)]);
         (*pos)[a] = 0;
         for (int sl = a + 1; sl < b; sl++) (*pos)[sl] = (*pos)[sl - 1] + (*keep)[sl - 1];
         part->smem = std::max(part->smem, (size_t)m.end);
@@ -111,4 +122,29 @@ bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, un
     /* one mbarrier phase counts at most 2^20 - 1 bytes; halo slots are 20-bit */
     if (16 * GSLAM_CLUSTER_CTAS + 24 * (int64_t)part->halo_max >= (1 << 20) - 1) return false;
     return true;
+}
+
+/*
+ * Least-squares fits to measured times per iteration: 190 plans (walks, walks with up to 40 near
+ * or 8 random closures per pose, landmark logs of 10 to 40 observations per landmark; 100 to 20,000
+ * poses, 1 to 16 CTAs), within 7 % of the measured time (root mean square), 26 % at most. A CTA's
+ * positions are its SpMV, a position left to L2 costs about as much again, a halo row sent costs
+ * a store to another SM, and the widest slice is the longest chain of one warp. With two rows per
+ * thread, D^-1 and the left-out positions come from L2 one after another, along the widest slice.
+ */
+double gslam_cluster_us(const gslam_cluster_part &p, int elem) {
+    const bool two_rows = p.shape == 3;
+    if (elem == 8) {
+        if (two_rows) return 2.6 + 0.019 * p.positions + 0.0021 * p.sent + 0.236 * p.width;
+        if (p.ctas == 1) return 1.1 + 0.022 * p.positions + 0.004 * p.left;
+        return 1.7 + 0.014 * p.positions + 0.017 * p.left + 0.0019 * p.sent + 0.020 * p.width;
+    }
+    if (two_rows) return 3.2 + 0.0053 * p.positions + 0.0098 * p.left + 0.0009 * p.sent + 0.067 * p.width;
+    return 2.0 + 0.0086 * p.positions + 0.007 * p.left + 0.001 * p.sent + 0.024 * p.width;
+}
+
+/* The same for the resident solver on the whole GPU (70 of these graphs up to 7,168 poses; 8 % at
+ * most): two reductions over 148 CTAs, a few slices per CTA and the halo rows it polls. */
+double gslam_resident_us(int positions, int left, int halo) {
+    return 2.8 + 0.035 * positions + 0.08 * left + 0.00155 * halo;
 }

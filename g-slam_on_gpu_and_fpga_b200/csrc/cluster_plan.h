@@ -13,6 +13,9 @@ struct gslam_cluster_part {
     int ctas = 0, threads = 0, shape = 0; /* shape: launch_pcg_cluster */
     int halo_max = 0;
     size_t smem = 0;                     /* dynamic shared memory of the largest CTA */
+    /* what an iteration's time follows: the most block positions (288 values) a CTA owns and
+     * leaves to L2, the most halo rows it sends, and the widest slice */
+    int positions = 0, left = 0, sent = 0, width = 0;
     std::vector<int> bounds;             /* [ctas + 1] slices */
     std::vector<int> n_halo;             /* [ctas] */
     std::vector<int> exp_ptr;            /* [rows of the graph + 1] */
@@ -27,5 +30,11 @@ struct gslam_cluster_part {
  * memory exceed the budget); *part and the graph's part of the arrays are then undefined. */
 bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, unsigned shapes, int elem, int64_t budget,
                         gslam_cluster_part *part, std::vector<int> *lcol, std::vector<int> *keep, std::vector<int> *pos);
+
+/* Estimated us per iteration of the cluster solver for a plan in values of `elem` bytes, and of
+ * the grid-wide FP64 resident solver for the most positions, left-out positions and halo rows of
+ * its CTAs. */
+double gslam_cluster_us(const gslam_cluster_part &p, int elem);
+double gslam_resident_us(int positions, int left, int halo);
 
 #endif

@@ -1,0 +1,56 @@
+"""Which solver a graph is given: the one inside a thread-block cluster (pcg_cluster.cu) or the
+grid-wide one, by their estimated times. Graphs with long rows, whose values do not fit the
+cluster's shared memory, or with closures to random poses, whose halo rows are sent one by one,
+ran up to 3.4 times slower in a cluster than on the whole GPU.
+
+test_absent_cta beyond every grid is no CTA at all and keeps a handle off the cluster solver.
+Where the choice is right, the chosen solver takes at most 1.3 times as long as the grid-wide one
+(device times of the same solve, the best of six; a wrong choice took 1.8 times and more)."""
+import importlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GRID = dict(test_absent_cta=1 << 20)
+ITS = 200
+
+
+@pytest.fixture(scope="module")
+def synth():
+    return importlib.import_module("g-slam_on_gpu_and_fpga_b200.synth")
+
+
+def _random_closures(synth, n, k, seed=1):
+    """A walk with k closures per pose to random poses: (init, i, j, meas, log_w) and the walk."""
+    cg = synth.city_grid(n, seed=seed)
+    rng = np.random.default_rng(seed)
+    i, j = rng.integers(0, n, k * n).astype(np.uint32), rng.integers(0, n, k * n).astype(np.uint32)
+    i, j = i[i != j], j[i != j]
+    rel = rng.normal(size=(len(i), 3)) * 0.1
+    cg.edge_i, cg.edge_j = np.concatenate([cg.edge_i, i]), np.concatenate([cg.edge_j, j])
+    cg.meas, cg.log_w = np.concatenate([cg.meas, rel]), np.concatenate([cg.log_w, np.zeros_like(rel)])
+    return cg
+
+
+def _single_us(make):
+    g = make()
+    g.linearise()
+    g.assemble()
+    t = [g.solve().solve_ms for _ in range(6)]
+    g.close()
+    return min(t)
+
+
+@pytest.mark.parametrize("kind", ["random closures", "landmark cliques"])
+def test_single_graph_avoids_a_slow_cluster(pkg, synth, kind):
+    opts = dict(tol=0.0, max_iter=ITS)
+    if kind == "landmark cliques":
+        log = synth.landmark_log(7120, seed=3, density=1e-2, max_obs=20)
+        make = lambda **o: pkg.PoseGraph.from_log(log, 0.1, **opts, **o)  # noqa: E731
+    else:
+        cg = _random_closures(synth, 6000, 8)
+        make = lambda **o: pkg.PoseGraph.from_se2(cg.init, cg.edge_i, cg.edge_j, cg.meas, cg.log_w, 0.1,  # noqa: E731
+                                                  **opts, **o)
+    assert _single_us(make) <= 1.3 * _single_us(lambda: make(**GRID))
