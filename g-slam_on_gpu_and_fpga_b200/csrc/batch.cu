@@ -1,6 +1,6 @@
 /*
- * batch.cu — many independent pose graphs solved in one persistent launch: those of a batch
- * that fit no thread-block cluster of their own (pcg_cluster.cu).
+ * batch.cu — many independent pose graphs solved in one persistent launch: batches that are not
+ * solved in one thread-block cluster per graph (pcg_cluster.cu).
  *
  * Not in the reference (its programs solve one graph per process; its README
  * sweeps lambda with a shell loop over runs). A batch is one block-diagonal system:

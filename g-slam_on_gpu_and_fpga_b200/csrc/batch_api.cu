@@ -6,8 +6,8 @@
  * No counterpart in the reference, which solves one graph per process and sweeps
  * lambda with a shell loop (README.md:137-160). A batch is one block-diagonal graph:
  * every graph's poses padded to whole 32-row slices, its own lambda and anchor, its own
- * PCG scalars: in a thread-block cluster of its own (pcg_cluster.cu) if it fits one, else in
- * one persistent launch of batch.cu's solver.
+ * PCG scalars: in a thread-block cluster of its own (pcg_cluster.cu), or all of them in one
+ * persistent launch of batch.cu's solver.
  */
 #include <cuda_runtime.h>
 
@@ -214,8 +214,10 @@ int gslam_create_se2_batch(const gslam_se2_graph *graphs, uint32_t n_graphs, con
 }
 
 /*
- * The graphs of a batch that get a thread-block cluster each (pcg_cluster.cu): those that
- * fit 16 CTAs (20,480 rows). The GPU is shared by all graphs at once, and few full CTAs use it
+ * Whether a batch's graphs get a thread-block cluster each (pcg_cluster.cu), and of how many
+ * CTAs: if all of them fit 16 (20,480 rows at most) and that is the faster way by the
+ * estimates, else the grid-wide solver takes the whole batch.
+ * The GPU is shared by all graphs at once, and few full CTAs use it
  * better than many sparse ones, so each takes the smallest cluster with 20 slices per CTA in
  * FP64, 40 in FP32 (about what shared memory holds), or 16 CTAs. Ms of solve per round, 64
  * graphs of 500 to 17,000 poses, 10 / 20 / 30 / 40 slices: FP64 14.3 / 10.3 / 11.4 / 11.9, FP32
@@ -226,14 +228,23 @@ int gslam_create_se2_batch(const gslam_se2_graph *graphs, uint32_t n_graphs, con
  * of equal cluster shape run side by side on their own streams, the largest clusters first,
  * and the GPU starts the next cluster as one ends; the graphs of a launch come in order of
  * falling size, so the last to start are short.
+ * A batch is not split between the two: the grid-wide solver's iteration is mostly barriers and the
+ * widest row's chain of loads, so it takes almost as long for a part of the batch as for all
+ * of it. Us per iteration, clusters and then a graph of 25,000 poses / all grid-wide: with 20
+ * graphs of 500 poses 17.3 / 15.2, 8 of 20,000 48.7 / 40.2; two graphs of 15,000 poses with 2
+ * random closures per pose, one of which fits no cluster, 48.6 / 26.7.
  */
+/* SMs that a cluster takes out of use: so many run at once that the others' SMs stay empty */
+static double cluster_sms(int ctas, int n_sm) {
+    return ctas == 16 ? n_sm / 7.0 : ctas == 8 ? n_sm / 15.0 : ctas == 4 ? n_sm / 33.0 : (double)ctas;
+}
+
 static int batch_clusters_build(gslam_graph *g, bool fp32) {
     BatchState &B = *g->batch;
     BatchClusters &K = B.clusters[fp32 ? 1 : 0];
     if (K.built) return GSLAM_OK;
     const gslam_structure &S = g->S;
     const int G = B.n_graphs, elem = fp32 ? 4 : 8;
-    K.in_cluster.assign(G, 0);
     K.launches.clear();
     const int max_ctas = pcg_cluster_max_ctas(g->device, GSLAM_RES_SMEM_MAX);
     std::vector<gslam_cluster_part> part(G);
@@ -250,24 +261,33 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
         while (c < max_ctas && c * per < ns) c *= 2;
         for (; c <= max_ctas; c *= 2)
             if (plan(q, c)) { ctas[q] = c; break; }
+        if (ctas[q] == 0) { K.built = true; return GSLAM_OK; }
         used += ctas[q];
     }
     for (bool more = true; more && 2 * used <= g->L.n_sm;) {
         more = false;
         for (int q = 0; q < G; q++)
-            if (ctas[q] > 0 && 2 * ctas[q] <= max_ctas && 8 * ctas[q] <= first(q + 1) - first(q)) {
+            if (2 * ctas[q] <= max_ctas && 8 * ctas[q] <= first(q + 1) - first(q)) {
                 used += ctas[q];
                 ctas[q] *= 2;
                 more = true;
             }
     }
-    K.all = true;
-    std::vector<int> order;
+    std::vector<int> order(G);
+    double longest = 0.0, sm_us = 0.0, sms = 0.0;
     for (int q = 0; q < G; q++) {
-        if (ctas[q] == 0 || (part[q].ctas != ctas[q] && !plan(q, ctas[q]))) { K.all = false; continue; }
-        K.in_cluster[q] = 1;
-        order.push_back(q);
+        /* a doubled cluster that does not fit after all (longer halos) is halved again */
+        if (part[q].ctas != ctas[q])
+            while (!plan(q, ctas[q])) ctas[q] /= 2;
+        order[q] = q;
+        const double us = gslam_cluster_us(part[q], elem), n = cluster_sms(ctas[q], g->L.n_sm);
+        longest = std::max(longest, us);
+        sms += n;
+        sm_us += n * us;
     }
+    /* at most what list scheduling needs; 0.9: no change of solver at a tie */
+    const double us = sms <= g->L.n_sm ? longest : sm_us / g->L.n_sm + longest;
+    if (us > 0.9 * gslam_batch_us(S.max_width, S.n_slots / 32, elem)) { K.built = true; return GSLAM_OK; }
     /* launches: cluster size and CTA shape */
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         if (part[a].ctas != part[b].ctas) return part[a].ctas > part[b].ctas;
@@ -294,28 +314,25 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
         for (int e : p.exp_ptr) exp_ptr.push_back(e + (int)exp.size());
         exp.insert(exp.end(), p.exp.begin(), p.exp.end());
     }
-    if (!jobs.empty()) {
-        DevMem &m = g->mem;
-        CK(dupload_all(m, g->st, { dpart(&K.d_jobs, jobs), dpart(&K.d_bounds, bounds), dpart(&K.d_halo, halo),
-                                   dpart(&K.d_lcol, lcol), dpart(&K.d_keep, keep), dpart(&K.d_pos, pos),
-                                   dpart(&K.d_exp_ptr, exp_ptr), dpart(&K.d_exp, exp),
-                                   dpart(&K.d_rest_skip, K.in_cluster) })); /* the last: what the grid-wide solver leaves alone */
-        if (!B.fork) CK(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming));
-        while (B.side.size() < K.launches.size()) {
-            cudaStream_t t;
-            cudaEvent_t e;
-            CK(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
-            B.side.push_back(t);
-            CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            B.side_done.push_back(e);
-        }
+    DevMem &m = g->mem;
+    CK(dupload_all(m, g->st, { dpart(&K.d_jobs, jobs), dpart(&K.d_bounds, bounds), dpart(&K.d_halo, halo),
+                               dpart(&K.d_lcol, lcol), dpart(&K.d_keep, keep), dpart(&K.d_pos, pos),
+                               dpart(&K.d_exp_ptr, exp_ptr), dpart(&K.d_exp, exp) }));
+    if (!B.fork) CK(cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming));
+    while (B.side.size() < K.launches.size()) {
+        cudaStream_t t;
+        cudaEvent_t e;
+        CK(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+        B.side.push_back(t);
+        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        B.side_done.push_back(e);
     }
     K.built = true;
     return GSLAM_OK;
 }
 
-/* Solves the batch's systems on the handle's stream: the graphs with clusters, then whatever
- * is left with the grid-wide solver. skip (may be null) marks graphs to leave alone. */
+/* Solves the batch's systems on the handle's stream, in clusters or with the grid-wide solver.
+ * skip (may be null) marks graphs to leave alone. */
 static int batch_launch(gslam_graph *g, const PcgParams &P, BatchParams BP, bool fp32, const std::vector<int> *skip) {
     BatchState &B = *g->batch;
     cudaStream_t st = g->st;
@@ -327,15 +344,10 @@ static int batch_launch(gslam_graph *g, const PcgParams &P, BatchParams BP, bool
         const int rc = batch_clusters_build(g, fp32);
         if (rc != GSLAM_OK) return rc;
     }
-    const int *rest_skip = K.d_rest_skip;
     if (skip) {
-        /* for the clusters, then with the graphs that have one, for the grid-wide solver */
-        std::vector<int> both(*skip);
-        for (int q = 0; q < G; q++) both.push_back((*skip)[q] || (clusters && K.in_cluster[q]));
-        if (!B.d_skip) CK(dalloc(g->mem, &B.d_skip, 2 * (size_t)G));
-        CK(cudaMemcpyAsync(B.d_skip, both.data(), 2 * (size_t)G * sizeof(int), cudaMemcpyHostToDevice, st));
+        if (!B.d_skip) CK(dalloc(g->mem, &B.d_skip, (size_t)G));
+        CK(cudaMemcpyAsync(B.d_skip, skip->data(), (size_t)G * sizeof(int), cudaMemcpyHostToDevice, st));
         BP.skip = B.d_skip;
-        rest_skip = B.d_skip + G;
     }
     if (!clusters || K.launches.empty()) {
         CK(launch_pcg_batch(st, P, BP, B.grid, B.block, B.smem_bytes, fp32));
@@ -380,10 +392,6 @@ static int batch_launch(gslam_graph *g, const PcgParams &P, BatchParams BP, bool
         CK(cudaEventRecord(B.side_done[i], B.side[i]));
     }
     for (size_t i = 0; i < K.launches.size(); i++) CK(cudaStreamWaitEvent(st, B.side_done[i], 0));
-    if (!K.all) {
-        BP.skip = rest_skip;
-        CK(launch_pcg_batch(st, P, BP, B.grid, B.block, B.smem_bytes, fp32));
-    }
     return GSLAM_OK;
 }
 

@@ -148,3 +148,11 @@ double gslam_cluster_us(const gslam_cluster_part &p, int elem) {
 double gslam_resident_us(int positions, int left, int halo) {
     return 2.8 + 0.035 * positions + 0.08 * left + 0.00155 * halo;
 }
+
+/* The grid-wide batch solver, which streams the matrix (100 batches of 1 to 30 graphs; 9 % root
+ * mean square, 38 % too low at most): its barriers, the widest slice's chain of loads, and the
+ * bytes. */
+double gslam_batch_us(int width, int64_t positions, int elem) {
+    return elem == 8 ? 7.6 + 0.447 * width + 1.08e-3 * (double)positions
+                     : 8.0 + 0.320 * width + 0.63e-3 * (double)positions;
+}

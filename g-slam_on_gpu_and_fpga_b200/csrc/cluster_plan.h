@@ -36,5 +36,7 @@ bool gslam_cluster_plan(const gslam_structure &S, int sl0, int sl1, int ctas, un
  * its CTAs. */
 double gslam_cluster_us(const gslam_cluster_part &p, int elem);
 double gslam_resident_us(int positions, int left, int halo);
+/* The same for the grid-wide batch solver: the widest slice and all positions of the batch. */
+double gslam_batch_us(int width, int64_t positions, int elem);
 
 #endif

@@ -73,8 +73,8 @@ struct DevLayout {
     int max_grid_alloc() const { return partial_capacity; }
 };
 
-/* A batch's graphs that are solved by one cluster each (pcg_cluster.cu), in one precision:
- * launches of equal cluster shape, largest clusters first. */
+/* A batch solved in one cluster per graph (pcg_cluster.cu), in one precision: launches of equal
+ * cluster shape, largest clusters first; none when the grid-wide solver takes the batch. */
 struct BatchClusters {
     struct Launch {
         int job0, n_jobs, ctas, threads, shape;
@@ -82,13 +82,10 @@ struct BatchClusters {
     };
     bool built = false;
     std::vector<Launch> launches;
-    std::vector<int> in_cluster; /* [n_graphs] 1: has a cluster */
-    bool all = false;            /* every graph has one */
     ClusterJob *d_jobs = nullptr;
     int *d_bounds = nullptr, *d_halo = nullptr, *d_lcol = nullptr, *d_exp_ptr = nullptr;
     int *d_keep = nullptr, *d_pos = nullptr;
     unsigned *d_exp = nullptr;
-    int *d_rest_skip = nullptr;  /* [n_graphs] graphs that the grid-wide solver leaves alone */
 };
 
 /* A batch of independent SE(2) graphs as one block-diagonal graph (batch.cu). */
@@ -119,8 +116,7 @@ struct BatchState {
     std::vector<cudaStream_t> side; /* the launches' streams, and their fork and join events */
     std::vector<cudaEvent_t> side_done;
     cudaEvent_t fork = nullptr;
-    int *d_skip = nullptr;       /* [2 n_graphs] graphs the FP64 rerun of a stagnated mixed batch leaves
-                                  * alone; the same and those with a cluster */
+    int *d_skip = nullptr;       /* [n_graphs] graphs the FP64 rerun of a stagnated mixed batch leaves alone */
     /* chunk sums of the per-graph norm kernels */
     double *d_chunk_part = nullptr;
     int max_chunks = 1;

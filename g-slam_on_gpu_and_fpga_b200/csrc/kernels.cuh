@@ -173,9 +173,8 @@ struct BatchParams {
     int *active;             /* graphs still iterating (set to n_graphs before launch) */
     const float *bf4;        /* FP32 inner solve: right-hand side (padded rows) */
     const int *skip;         /* [n_graphs] or null: graphs left exactly as they are (done from the
-                              * start, their vectors and results untouched: graphs a cluster
-                              * solves, and the mixed batch's FP64 rerun of only the graphs that
-                              * stagnated) */
+                              * start, their vectors and results untouched: the mixed batch's FP64
+                              * rerun of only the graphs that stagnated) */
     const int *cap;          /* [n_graphs] or null: each graph's own iteration cap (at most the
                               * launch's max_iter; the mixed batch's inner passes, each graph
                               * with what is left of its budget) */

@@ -311,7 +311,8 @@ class PoseGraph:
 class PoseGraphBatch(PoseGraph):
     """Many independent SE(2) graphs on one handle (gslam_create_se2_batch): one
     Gauss-Newton round of every graph per `round()`, each linear solve in a thread-block
-    cluster of its own (graphs above 20,480 rows in one grid-wide launch). Poses of graph q are
+    cluster of its own, or all of them in one grid-wide launch (if a graph is too large for a
+    cluster, or that is faster). Poses of graph q are
     `poses[offsets[q] : offsets[q] + sizes[q]]` of the concatenation."""
 
     @classmethod

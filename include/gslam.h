@@ -315,9 +315,9 @@ int gslam_landmark_map(gslam_graph *g, uint32_t *n_landmarks, uint32_t *ids, dou
  * gslam_get_poses / gslam_set_poses work on the concatenation.
  *
  * gslam_batch_round: one Gauss-Newton round of every graph; each linear solve runs in a
- * thread-block cluster of its own, and what does not fit one in ONE grid-wide launch
- * (block-Jacobi PCG with each graph's own alpha, beta and stopping test, tol / max_iter of
- * the handle's options, FP64). per_graph (host,
+ * thread-block cluster of its own, or, if a graph fits none or that is faster, all of them
+ * in ONE grid-wide launch (block-Jacobi PCG with each graph's own alpha, beta and stopping
+ * test, tol / max_iter of the handle's options, FP64). per_graph (host,
  * n_graphs entries, may be NULL) receives each graph's iterations, reason, relative
  * residual and update norm diff = ||dx|| / sqrt(3 n_poses). gslam_round on a batch
  * runs the same round and reports the largest iteration count and residual.

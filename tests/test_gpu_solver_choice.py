@@ -54,3 +54,45 @@ def test_single_graph_avoids_a_slow_cluster(pkg, synth, kind):
         make = lambda **o: pkg.PoseGraph.from_se2(cg.init, cg.edge_i, cg.edge_j, cg.meas, cg.log_w, 0.1,  # noqa: E731
                                                   **opts, **o)
     assert _single_us(make) <= 1.3 * _single_us(lambda: make(**GRID))
+
+
+def _batch(pkg, graphs, prec, rounds, its_cap=ITS, **opts):
+    """(best solve ms, pose steps of every graph after one round, iterations) of a batch."""
+    b = pkg.PoseGraphBatch.from_se2_list(graphs, 0.1, tol=0.0, max_iter=its_cap, inner_tol=0.0,
+                                         inner_max_iter=its_cap, precision=prec, **opts)
+    t, dx, its = [], None, None
+    for _ in range(rounds):
+        b.poses = b.init_poses
+        st = b.round_all()
+        t.append(st[0].solve_ms)
+        its = [s.iterations for s in st]
+        dx = [b.graph_poses(q, b.poses - b.init_poses) for q in range(len(graphs))]
+    b.close()
+    return min(t), dx, its
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("kind", ["one graph too large", "random closures"])
+def test_batch_avoids_slow_clusters(pkg, synth, kind, prec):
+    if kind == "one graph too large":
+        graphs = [synth.city_grid(25_000, seed=0)] + [synth.city_grid(5000, seed=1 + s) for s in range(20)]
+        bound = 1.05    # the clusters beside the grid-wide solve took 1.16 (mixed) and 1.18 times as long
+    else:
+        graphs = [_random_closures(synth, 15_000, 2, seed=s) for s in range(2)]
+        bound = 1.3     # 1.8 in FP64
+    assert _batch(pkg, graphs, prec, 8)[0] <= bound * _batch(pkg, graphs, prec, 8, **GRID)[0]
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
+def test_batch_in_clusters_takes_the_grid_wide_iterates(pkg, synth, prec):
+    """Clusters of 1 to 16 CTAs, with one and two rows per thread, are chosen here (the solve takes
+    about half as long) and take the grid-wide solver's steps: after 60 iterations the two
+    orders of the dot products' sums differ by far less than 1e-9; in FP32 they round a
+    coefficient differently now and then (1e-3 allowed)."""
+    graphs = [synth.city_grid(n, seed=n) for n in (37, 320, 330, 640, 650, 5000, 10240, 10250, 20480)]
+    ta, xa, ia = _batch(pkg, graphs, prec, 4, 60)
+    tb, xb, ib = _batch(pkg, graphs, prec, 4, 60, **GRID)
+    assert ta <= 0.7 * tb
+    assert ia == ib
+    for a, b in zip(xa, xb):
+        assert np.linalg.norm(a - b) <= (1e-9 if prec == 0 else 1e-3) * np.linalg.norm(b) + 1e-12
