@@ -460,8 +460,9 @@ __device__ __forceinline__ bool tag_row_load(const double *v4, int row, unsigned
 
 /* the smallest number whose rounded square root is not below tol, so that
  * rr < square_limit(tol) decides as sqrt(rr) < tol does (sqrt is monotonic and correctly
- * rounded) without a square root on the critical path */
+ * rounded) without a square root on the critical path; no root is below a tol of 0 or less */
 __device__ __forceinline__ double square_limit(double tol) {
+    if (tol <= 0.0) return 0.0;
     double y = tol * tol;
     for (int i = 0; i < 8 && sqrt(y) < tol; i++) y = __longlong_as_double(__double_as_longlong(y) + 1);
     for (int i = 0; i < 8 && y > 0.0 && sqrt(__longlong_as_double(__double_as_longlong(y) - 1)) >= tol; i++)
