@@ -216,11 +216,14 @@ __global__ void __launch_bounds__(BS, 1) k_pcg64_res(PcgParams P) {
             s_rr = s_bc[1];
             s_limit = square_limit(P.tol_rel * sqrt(s_bc[1]));
             s_beta = 0.0;
+            if (!s_ok) s_flag = 1 + GSLAM_STOP_TIMEOUT;
         }
         __syncthreads();
     }
     const double bnorm = sqrt(s_bc[1]);
-    int k = 0, reason = GSLAM_STOP_MAXIT, flag = s_ok ? 0 : 1 + GSLAM_STOP_TIMEOUT;
+    /* all threads read the same flag, as in the loop: s_ok may change at any time once a faster
+     * warp polls halo rows, and a warp that left alone would be missed at the barriers */
+    int k = 0, reason = GSLAM_STOP_MAXIT, flag = s_flag;
 
     while (!flag) {
         if (k >= P.max_iter) break;
