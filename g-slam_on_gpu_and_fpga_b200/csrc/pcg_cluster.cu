@@ -45,8 +45,8 @@
  * dot products), with batch.cu's arithmetic.
  *
  * Waits are bounded: a wait that runs out marks the solve as timed out and the CTA leaves
- * through the final cluster barrier (no CTA exits while another may store into its shared
- * memory).
+ * through the final cluster barrier, and a little after it (no CTA exits while another's
+ * store into its shared memory may be on its way).
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
         }
         if (!tma_wait(&s_mb[0], 0, P.spin_limit)) {
             s_flag = 1 + GSLAM_STOP_TIMEOUT;
-            tma_wait(&s_mb[0], 0, P.spin_limit); /* let the copy finish before the CTA leaves */
+            tma_drain(&s_mb[0], 0);
         }
         __syncthreads();
         const int cap = BATCH && P.cap != nullptr ? min(P.max_iter, __ldg(P.cap + J.graph)) : P.max_iter;
@@ -562,12 +562,6 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
             }
         }
         if (flag) reason = flag - 1;
-        if (!ONE && reason == GSLAM_STOP_TIMEOUT) {
-            /* a message sent before another CTA gave up has long arrived; the margin covers
-             * a limit of a few cycles */
-            const long long t0 = clock64();
-            while (clock64() - t0 < 100000) {}
-        }
         if (reason == GSLAM_STOP_TIMEOUT && threadIdx.x == 0) res_mark_timeout(P.res);
 #pragma unroll
         for (int i = 0; i < R; i++)
@@ -585,6 +579,13 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_cluster(const ClusterParams P) {
     if (!ONE) {
         __syncthreads();
         cl_sync();
+        if (absent || reason == GSLAM_STOP_TIMEOUT) {
+            /* the others may have sent to this CTA up to their arrival above, in phases that it does
+             * not wait for any more: 50 us for the last of that to land. A CTA that finished its
+             * solve has received all that was sent to it. */
+            const long long t0 = clock64();
+            while (clock64() - t0 < 100000) {}
+        }
     }
 }
 

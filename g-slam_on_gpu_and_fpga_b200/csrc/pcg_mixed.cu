@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
     if (!tma_wait(&s_bar, 0, P.spin_limit)) {
         atomicExch(&P.gs->abort, 1);
         s_ok = 0;
-        tma_wait(&s_bar, 0, P.spin_limit); /* let the copy finish before the CTA leaves */
+        tma_drain(&s_bar, 0);
     }
     __syncthreads();
     if (!s_ok) {

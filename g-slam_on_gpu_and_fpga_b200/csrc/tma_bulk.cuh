@@ -49,4 +49,9 @@ __device__ __forceinline__ bool tma_wait(uint64_t *bar, unsigned parity, long lo
     return true;
 }
 
+/* For a CTA that gives up: lets its copies land before it leaves, so that none is written into the
+ * shared memory of the CTA that follows on the SM. A limit of its own (about a second): the
+ * caller's may be shorter than any copy takes. */
+__device__ __forceinline__ void tma_drain(uint64_t *bar, unsigned parity) { tma_wait(bar, parity, 1ll << 31); }
+
 #endif
