@@ -124,22 +124,26 @@ void DevMem::release() {
 #define CLUSTER_CTA_SLICES 4
 #define CLUSTER_MAX_SLICES 224
 
-static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, int device,
-                          const std::vector<int> &grid_slices, double resident_us) {
+static int cluster_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st, const std::vector<int> &grid_slices,
+                          double resident_us) {
     if (S.n_slices > CLUSTER_MAX_SLICES) return GSLAM_OK;
-    const int max_ctas = pcg_cluster_max_ctas(device, GSLAM_RES_SMEM_MAX);
     int ctas = 1;
     if (S.n_slices > CLUSTER_ONE_SLICES)
-        while (ctas < max_ctas && CLUSTER_CTA_SLICES * ctas < S.n_slices) ctas *= 2;
-    /* a shape with an eighth of its slices to spare, so that the CTAs can be balanced by slots
-     * (log of 6,000 poses, 11.75 slices per CTA: 3.84 us per iteration in 12-slice CTAs, 3.32 in
-     * 16-slice ones) */
-    const unsigned shapes = 8 * S.n_slices <= 7 * 12 * ctas ? 15 : 8 * S.n_slices <= 7 * 16 * ctas ? 14 : 12;
+        while (ctas < GSLAM_CLUSTER_CTAS && CLUSTER_CTA_SLICES * ctas < S.n_slices) ctas *= 2;
     gslam_cluster_part part;
     std::vector<int> lcol(S.n_slots, 0), keep(S.n_slices, 0), pos(S.n_slices, 0);
-    if (max_ctas == 0 || !gslam_cluster_plan(S, 0, S.n_slices, ctas, shapes, 8, GSLAM_RES_SMEM_MAX, &part, &lcol, &keep, &pos))
-        return GSLAM_OK;
-    if (gslam_cluster_us(part, 8) > 1.1 * resident_us) return GSLAM_OK; /* 1.1: no change of solver at a tie */
+    for (int can = 0;; ctas = can) {
+        /* a shape with an eighth of its slices to spare, so that the CTAs can be balanced by slots
+         * (log of 6,000 poses, 11.75 slices per CTA: 3.84 us per iteration in 12-slice CTAs, 3.32 in
+         * 16-slice ones) */
+        const unsigned shapes = 8 * S.n_slices <= 7 * 12 * ctas ? 15 : 8 * S.n_slices <= 7 * 16 * ctas ? 14 : 12;
+        if (!gslam_cluster_plan(S, 0, S.n_slices, ctas, shapes, 8, GSLAM_RES_SMEM_MAX, &part, &lcol, &keep, &pos) ||
+            gslam_cluster_us(part, 8) > 1.1 * resident_us) /* 1.1: no change of solver at a tie */
+            return GSLAM_OK;
+        can = pcg_cluster_ctas(false, false, part.shape, ctas, GSLAM_RES_SMEM_MAX);
+        if (can == 0) return GSLAM_OK;
+        if (can == ctas) break;
+    }
     /* the grid-wide solver's CTAs that own slices (the order of its sums) */
     int vctas = 0;
     for (size_t c = 0; c + 1 < grid_slices.size(); c++)
@@ -332,7 +336,7 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
             if (fit_res && !o.disable_resident) {
                 L->resident = true;
                 L->smem_bytes = (size_t)end_res;
-                const int rc = cluster_upload(L, S, st, device, cs, gslam_resident_us(most_positions, most_left, most_halo));
+                const int rc = cluster_upload(L, S, st, cs, gslam_resident_us(most_positions, most_left, most_halo));
                 if (rc != GSLAM_OK) return rc;
             }
             /* mixed and one-reduction: values | local columns | z of own and halo rows | v of

@@ -246,7 +246,9 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
     const gslam_structure &S = g->S;
     const int G = B.n_graphs, elem = fp32 ? 4 : 8;
     K.launches.clear();
-    const int max_ctas = pcg_cluster_max_ctas(g->device, GSLAM_RES_SMEM_MAX);
+    int max_ctas = GSLAM_CLUSTER_CTAS;
+    for (int shape = 0; shape < 4; shape++)
+        if (GSLAM_BATCH_SHAPES >> shape & 1) max_ctas = std::min(max_ctas, pcg_cluster_ctas(fp32, true, shape, GSLAM_CLUSTER_CTAS, GSLAM_RES_SMEM_MAX));
     std::vector<gslam_cluster_part> part(G);
     std::vector<int> lcol(S.n_slots, 0), keep(S.n_slices, 0), pos(S.n_slices, 0), ctas(G, 0);
     auto first = [&](int q) { return B.pose_off[q] / 32; };
@@ -314,6 +316,12 @@ static int batch_clusters_build(gslam_graph *g, bool fp32) {
         for (int e : p.exp_ptr) exp_ptr.push_back(e + (int)exp.size());
         exp.insert(exp.end(), p.exp.begin(), p.exp.end());
     }
+    for (const BatchClusters::Launch &l : K.launches)
+        if (l.ctas == 1 && pcg_cluster_ctas(fp32, true, l.shape, 1, GSLAM_RES_SMEM_MAX) == 0) {
+            K.launches.clear();
+            K.built = true;
+            return GSLAM_OK;
+        }
     DevMem &m = g->mem;
     CK(dupload_all(m, g->st, { dpart(&K.d_jobs, jobs), dpart(&K.d_bounds, bounds), dpart(&K.d_halo, halo),
                                dpart(&K.d_lcol, lcol), dpart(&K.d_keep, keep), dpart(&K.d_pos, pos),

@@ -276,9 +276,10 @@ __host__ __device__ inline ClusterSmem cluster_smem_layout(int64_t elem, int64_t
 cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jobs, int threads, int shape,
                                size_t smem_bytes, bool fp32, bool batch);
 /* shape: 0 up to 12 slices per CTA, 1 up to 16, 2 up to 20, 3 up to 40 (two per warp) */
-/* Largest cluster the solver's kernels can be launched with (0: none), with this much
- * dynamic shared memory per CTA; also sets their attributes. */
-int pcg_cluster_max_ctas(int device, size_t smem_bytes);
+/* Prepares the kernel of a launch (its attributes), and returns the largest cluster of at most `ctas`
+ * CTAs (a power of two) that it can be launched with, with this much dynamic shared memory per
+ * CTA; 0: none. */
+int pcg_cluster_ctas(bool fp32, bool batch, int shape, int ctas, size_t smem_bytes);
 
 /* Mixed-precision solver (pcg_mixed.cu); fp64: the same kernel as the FP64 one-reduction
  * solver. */

@@ -604,8 +604,7 @@ static const void *fn_of(int shape) {
     }
 }
 
-/* kinds of launches: FP32 batches, FP64 batches, single graphs */
-#define CLUSTER_KINDS 3
+/* kinds of launches: 0 FP32 batches, 1 FP64 batches, 2 single graphs */
 static const void *cluster_fn(int kind, int shape, bool one) {
     switch (kind) {
     case 0: return one ? fn_of<float, true, true>(shape) : fn_of<float, false, true>(shape);
@@ -641,29 +640,20 @@ cudaError_t launch_pcg_cluster(cudaStream_t st, const ClusterParams &p, int n_jo
     return cudaLaunchKernelExC(&cfg, cluster_fn(kind, shape, p.ctas == 1), args);
 }
 
-int pcg_cluster_max_ctas(int device, size_t smem_bytes) {
-    (void)device;
-    int best = 0;
-    for (int v = 0; v < CLUSTER_KINDS * 8; v++) {
-        const bool one = v % 2 != 0;
-        const int shape = v / 2 % 4, threads = shape == 0 ? 384 : shape == 1 ? 512 : 640;
-        const void *fn = cluster_fn(v / 8, shape, one);
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess ||
-            cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-            cudaGetLastError();
-            return 0;
-        }
-        if (one) continue; /* one CTA needs no cluster */
-        int can = 0;
-        for (int c = GSLAM_CLUSTER_CTAS; c > 1; c /= 2) {
-            cudaLaunchConfig_t cfg;
-            cudaLaunchAttribute at[1];
-            cluster_config(&cfg, at, c, c, threads, smem_bytes, nullptr);
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) { can = c; break; }
-            cudaGetLastError();
-        }
-        best = v == 0 ? can : std::min(best, can);
+int pcg_cluster_ctas(bool fp32, bool batch, int shape, int ctas, size_t smem_bytes) {
+    const void *fn = cluster_fn(fp32 ? 0 : batch ? 1 : 2, shape, ctas == 1);
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
-    return std::max(best, 1);
+    for (; ctas > 1; ctas /= 2) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[1];
+        cluster_config(&cfg, at, ctas, ctas, shape == 0 ? 384 : shape == 1 ? 512 : 640, smem_bytes, nullptr);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) break;
+        cudaGetLastError();
+    }
+    return ctas; /* one CTA needs no cluster */
 }
