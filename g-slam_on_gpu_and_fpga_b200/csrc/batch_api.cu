@@ -699,3 +699,9 @@ int gslam_batch_layout(gslam_graph *g, uint32_t *n_graphs, uint32_t *pose_offset
     return GSLAM_OK;
 }
 
+int gslam_batch_in_clusters(const gslam_graph *g, int *yes) {
+    if (!g || !g->batch || !yes) BAD("not a batch");
+    const BatchClusters &K = g->batch->clusters[g->o.precision == GSLAM_PREC_MIXED ? 1 : 0];
+    *yes = g->o.test_absent_cta < 0 && !g->o.disable_resident && !K.launches.empty();
+    return GSLAM_OK;
+}

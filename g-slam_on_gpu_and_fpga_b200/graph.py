@@ -356,6 +356,14 @@ class PoseGraphBatch(PoseGraph):
     def n_graphs(self) -> int:
         return len(self.offsets)
 
+    @property
+    def in_clusters(self) -> bool:
+        """Whether the graphs are solved in a thread-block cluster each (else in one grid-wide
+        launch, which threads_per_cta and ctas_per_sm shape)."""
+        yes = C.c_int()
+        abi.check(abi.lib().gslam_batch_in_clusters(self._h, C.byref(yes)))
+        return bool(yes.value)
+
     def round_all(self):
         """One round of every graph; a RoundStats per graph."""
         st = (abi.SolveStats * self.n_graphs)()

@@ -326,6 +326,9 @@ int gslam_create_se2_batch(const gslam_se2_graph *graphs, uint32_t n_graphs, con
                            gslam_graph **out);
 int gslam_batch_round(gslam_graph *g, gslam_solve_stats *per_graph);
 int gslam_batch_layout(gslam_graph *g, uint32_t *n_graphs, uint32_t *pose_offset);
+/* *yes = 1 if a batch made with the handle's precision is solved in clusters, where
+ * threads_per_cta and ctas_per_sm have no effect. */
+int gslam_batch_in_clusters(const gslam_graph *g, int *yes);
 
 /*
  * Dense Gauss-Jordan inverse / solve, replacing the reference's dense check path
