@@ -205,8 +205,9 @@ template <> struct Inner<double> {
 /* T = float: the mixed solver; T = double: the FP64 one-reduction solver (one inner solve).
  * R: slices per warp (warp w owns slices w and w + BS / 32); DREGS: the rows' D^-1 stay in
  * registers for the whole solve, else they are read from L2 in every iteration; U: blocks
- * whose loads are issued together */
-template <int BS, int R, typename T, bool DREGS, int U>
+ * whose loads are issued together; FAR: v of some halo rows is in global memory (kernels of their
+ * own: the other layouts' lose up to 4 % to the registers it takes) */
+template <int BS, int R, typename T, bool DREGS, int U, bool FAR>
 __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
     constexpr bool F64 = sizeof(T) == 8;
     constexpr int W = BS / 32;
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
     const int64_t nsm = nval < ml.val_cap ? nval : ml.val_cap;
     T *sval = reinterpret_cast<T *>(smem);
     int *scol = reinterpret_cast<int *>(smem + ml.col_off);
-    const int n_shv = (int)ml.v_rows;
+    const int n_shv = FAR ? (int)ml.v_rows : n_halo;
     const Rows<T> sz(smem + ml.z_off, n_loc + n_halo), shv(smem + ml.v_off, n_shv);
     auto far_v = [&]() { return static_cast<T *>(P.halo_v); }; /* v of halo rows n_shv and up, at h0 + row */
 
@@ -375,7 +376,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
         if (!grid_barrier(P.gs, (unsigned)(++epoch), P.spin_limit, &s_ok)) { timed_out = true; break; }
         for (int h = hh; h < n_halo; h += BS) {
             sz.put(n_loc + h, ldcgt3(Inner<T>::z0(P), __ldg(P.halo_rows + h0 + h)));
-            if (h < n_shv) shv.put(h, zero);
+            if (!FAR || h < n_shv) shv.put(h, zero);
             else stt3(far_v(), h0 + h, zero);
         }
 #pragma unroll
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
             for (int h = hh + R * BS; h < n_halo; h += BS) {
                 T3<T> uh = zero;
                 if (k > 0 && !get_row(Inner<T>::u(P, seq & 1), __ldg(P.halo_rows + h0 + h), seq, P.gs, P.spin_limit, &uh)) s_ok = 0;
-                if (h < n_shv) {
+                if (!FAR || h < n_shv) {
                     halo_step(h, uh);
                 } else {
                     T3<T> zn, vn;
@@ -578,22 +579,22 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
  * 4.52, at 100,000 6.88 and 6.31; D^-1 loaded ahead of the product instead of after it
  * spills: 8.1. */
 struct MixKernel {
-    const void *fn;
+    const void *fn, *far; /* far: some halo rows' v in global memory */
     int block, max_slices;
 };
+template <int BS, int R, typename T, bool DREGS, int U>
+static MixKernel mix_kernel() {
+    return { (const void *)k_pcg_mixed<BS, R, T, DREGS, U, false>, (const void *)k_pcg_mixed<BS, R, T, DREGS, U, true>, BS,
+             R * BS / 32 };
+}
 static const MixKernel *mix_kernels(bool fp64, int *n) {
     static const MixKernel f[] = {
-        { (const void *)k_pcg_mixed<384, 1, float, true, 4>, 384, 12 },
-        { (const void *)k_pcg_mixed<512, 1, float, true, 4>, 512, 16 },
-        { (const void *)k_pcg_mixed<640, 1, float, true, 4>, 640, 20 },
-        { (const void *)k_pcg_mixed<384, 2, float, true, 4>, 384, 24 },
-        { (const void *)k_pcg_mixed<512, 2, float, false, 2>, 512, 32 },
+        mix_kernel<384, 1, float, true, 4>(), mix_kernel<512, 1, float, true, 4>(), mix_kernel<640, 1, float, true, 4>(),
+        mix_kernel<384, 2, float, true, 4>(), mix_kernel<512, 2, float, false, 2>(),
     };
     static const MixKernel d[] = {
-        { (const void *)k_pcg_mixed<384, 1, double, true, 4>, 384, 12 },
-        { (const void *)k_pcg_mixed<512, 1, double, true, 2>, 512, 16 },
-        { (const void *)k_pcg_mixed<384, 2, double, false, 4>, 384, 24 },
-        { (const void *)k_pcg_mixed<512, 2, double, false, 1>, 512, 32 },
+        mix_kernel<384, 1, double, true, 4>(), mix_kernel<512, 1, double, true, 2>(), mix_kernel<384, 2, double, false, 4>(),
+        mix_kernel<512, 2, double, false, 1>(),
     };
     *n = (int)(fp64 ? sizeof d / sizeof d[0] : sizeof f / sizeof f[0]);
     return fp64 ? d : f;
@@ -614,7 +615,7 @@ cudaError_t launch_pcg_mixed(cudaStream_t st, const PcgParams &p, int grid, int 
         if (max_slices <= k[i].max_slices) {
             PcgParams copy = p;
             void *args[] = { &copy };
-            return cudaLaunchCooperativeKernel(k[i].fn, dim3(grid), dim3(k[i].block), args, smem_bytes, st);
+            return cudaLaunchCooperativeKernel(p.halo_v ? k[i].far : k[i].fn, dim3(grid), dim3(k[i].block), args, smem_bytes, st);
         }
     return cudaErrorInvalidValue;
 }
@@ -624,13 +625,14 @@ int pcg_mixed_max_grid(int device, size_t smem_bytes) {
     if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
     for (int f = 0; f < 2; f++) {
         const MixKernel *k = mix_kernels(f != 0, &n);
-        for (int i = 0; i < n; i++) {
-            int a = 0;
-            if (cudaFuncSetAttribute(k[i].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, GSLAM_GRID_SMEM_MAX) != cudaSuccess ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k[i].fn, k[i].block, smem_bytes) != cudaSuccess)
-                return 0;
-            best = f == 0 && i == 0 ? a : std::min(best, a);
-        }
+        for (int i = 0; i < n; i++)
+            for (const void *fn : { k[i].fn, k[i].far }) {
+                int a = 0;
+                if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, GSLAM_GRID_SMEM_MAX) != cudaSuccess ||
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fn, k[i].block, smem_bytes) != cudaSuccess)
+                    return 0;
+                best = f == 0 && i == 0 && fn == k[i].fn ? a : std::min(best, a);
+            }
     }
     return best * n_sm;
 }
