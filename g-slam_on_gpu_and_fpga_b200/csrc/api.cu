@@ -313,13 +313,15 @@ int gslam_layout_upload(DevLayout *L, const gslam_structure &S, cudaStream_t st,
                 hptr[i + 1] = hptr[i] + (int)rem.size();
                 hrows.insert(hrows.end(), rem.begin(), rem.end());
                 const int64_t nh = (int64_t)rem.size(), nsl = cs[i + 1] - cs[i];
-                const MixedSmem l32 = mixed_smem_layout(4, a1 - a0, nsl, nh, rows32, GSLAM_GRID_SMEM_MAX);
-                const MixedSmem l64 = mixed_smem_layout(8, a1 - a0, nsl, nh, rows64, GSLAM_GRID_SMEM_MAX);
+                const int64_t v32 = mixed_v_rows(4, a1 - a0, nsl, nh, rows32, GSLAM_GRID_SMEM_MAX);
+                const int64_t v64 = mixed_v_rows(8, a1 - a0, nsl, nh, rows64, GSLAM_GRID_SMEM_MAX);
+                const MixedSmem l32 = mixed_smem_layout(4, a1 - a0, nsl, nh, v32, GSLAM_GRID_SMEM_MAX);
+                const MixedSmem l64 = mixed_smem_layout(8, a1 - a0, nsl, nh, v64, GSLAM_GRID_SMEM_MAX);
                 const ResidentSmem lr = resident_smem_layout(a1 - a0, nsl, nh, GSLAM_GRID_SMEM_MAX);
                 fit_res = fit_res && lr.val_cap >= 0;
                 fit32 = fit32 && l32.val_cap >= 0;
                 fit64 = fit64 && l64.val_cap >= 0;
-                if (l32.v_rows < nh || l64.v_rows < nh) L->long_halo = true;
+                if (v32 < nh || v64 < nh) L->long_halo = true;
                 share(0, i, lr.val_cap);
                 const int positions = (int)((a1 - a0) / 32);
                 most_positions = std::max(most_positions, positions);

@@ -111,24 +111,19 @@ __host__ __device__ inline ResidentSmem resident_smem_layout(int64_t n_slots, in
 }
 
 /* Shared-memory layout of one CTA of the mixed / FP64 one-reduction solver, from its own
- * sizes: the fixed parts (local columns, z of own and halo rows, v of halo rows: 16 bytes a
- * row in FP32, 24 in FP64) after the values, and as many values (whole multiples of 288, one
- * block position of a slice) as the budget leaves. Of a halo too long for it, v of the rows
- * beyond the first v_rows is in global memory (read and written by one thread of this CTA
- * each); v of the first `first` rows (the kernel's rows per CTA) never is. val_cap < 0: the
- * fixed parts alone exceed the budget. */
+ * sizes: the fixed parts (local columns, z of own and halo rows, v of the first v_rows halo rows:
+ * 16 bytes a row in FP32, 24 in FP64) after the values, and as many values (whole multiples of
+ * 288, one block position of a slice) as the budget leaves. val_cap < 0: the fixed parts alone
+ * exceed the budget. */
 struct MixedSmem {
-    int64_t val_cap, col_off, z_off, v_off, v_rows, end;
+    int64_t val_cap, col_off, z_off, v_off, end;
 };
 __host__ __device__ inline MixedSmem mixed_smem_layout(int64_t elem, int64_t n_slots, int64_t n_slices, int64_t n_halo,
-                                                       int64_t first, int64_t budget) {
+                                                       int64_t v_rows, int64_t budget) {
     auto up = [](int64_t b) { return (b + 127) / 128 * 128; };
     const int64_t row_b = elem == 8 ? 24 : 16;
-    const int64_t col_b = up(4 * n_slots), z_b = up(row_b * (32 * n_slices + n_halo));
-    const int64_t room = (budget - col_b - z_b) / 128 * 128 / row_b, least = n_halo < first ? n_halo : first;
+    const int64_t col_b = up(4 * n_slots), z_b = up(row_b * (32 * n_slices + n_halo)), v_b = up(row_b * v_rows);
     MixedSmem m;
-    m.v_rows = room >= n_halo ? n_halo : room > least ? room : least;
-    const int64_t v_b = up(row_b * m.v_rows);
     const int64_t fixed = col_b + z_b + v_b;
     m.val_cap = budget >= fixed ? (budget - fixed) / elem / 288 * 288 : -1;
     const int64_t nv = m.val_cap > 9 * n_slots ? 9 * n_slots : m.val_cap;
@@ -137,6 +132,16 @@ __host__ __device__ inline MixedSmem mixed_smem_layout(int64_t elem, int64_t n_s
     m.v_off = m.z_off + z_b;
     m.end = m.v_off + v_b;
     return m;
+}
+/* The halo rows whose v is in shared memory: all, or as many as fit beside the columns and z but
+ * at least the first `first` (the kernel's rows per CTA). v of the others is in global memory, read
+ * and written by one thread of this CTA each. */
+__host__ __device__ inline int64_t mixed_v_rows(int64_t elem, int64_t n_slots, int64_t n_slices, int64_t n_halo,
+                                                int64_t first, int64_t budget) {
+    const MixedSmem m = mixed_smem_layout(elem, n_slots, n_slices, n_halo, 0, budget);
+    const int64_t room = (budget - m.v_off + m.col_off) / 128 * 128 / (elem == 8 ? 24 : 16);
+    const int64_t least = n_halo < first ? n_halo : first;
+    return room >= n_halo ? n_halo : room > least ? room : least;
 }
 
 /* Round cost terms per edge and their total (kernels.cu); block_sums holds

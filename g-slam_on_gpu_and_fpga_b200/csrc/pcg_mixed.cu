@@ -234,13 +234,13 @@ __global__ void __launch_bounds__(BS, 1) k_pcg_mixed(PcgParams P) {
     const int64_t nval = 9 * (slot1 - slot0);
     const int h0 = __ldg(P.halo_ptr + blockIdx.x), n_halo = __ldg(P.halo_ptr + blockIdx.x + 1) - h0;
     /* dynamic shared memory, laid out per CTA from its own sizes (mixed_smem_layout, the
-     * host's feasibility check uses the same function): T values as far as they fit |
+     * host's feasibility check uses the same functions): T values as far as they fit |
      * local columns | z of own + halo rows | v of halo rows */
-    const MixedSmem ml = mixed_smem_layout(sizeof(T), slot1 - slot0, s1 - s0, n_halo, R * BS, P.smem_budget);
+    const int n_shv = FAR ? (int)mixed_v_rows(sizeof(T), slot1 - slot0, s1 - s0, n_halo, R * BS, P.smem_budget) : n_halo;
+    const MixedSmem ml = mixed_smem_layout(sizeof(T), slot1 - slot0, s1 - s0, n_halo, n_shv, P.smem_budget);
     const int64_t nsm = nval < ml.val_cap ? nval : ml.val_cap;
     T *sval = reinterpret_cast<T *>(smem);
     int *scol = reinterpret_cast<int *>(smem + ml.col_off);
-    const int n_shv = FAR ? (int)ml.v_rows : n_halo;
     const Rows<T> sz(smem + ml.z_off, n_loc + n_halo), shv(smem + ml.v_off, n_shv);
     auto far_v = [&]() { return static_cast<T *>(P.halo_v); }; /* v of halo rows n_shv and up, at h0 + row */
 
