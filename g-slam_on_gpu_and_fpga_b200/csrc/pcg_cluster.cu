@@ -8,7 +8,8 @@
  * distributed shared memory takes 0.66 us (16 CTAs x 256 threads) to 0.87 us (16 x 768),
  * and a cluster's shared memory (16 x 227 KB) holds the matrix of a graph of about 10,000
  * poses. So a graph that fits is solved by one cluster of 1 to 16 CTAs, and a batch by one
- * cluster per graph, as many at a time as the GPU holds.
+ * cluster per graph, as many at a time as the GPU holds, unless the grid-wide solvers are
+ * estimated to be faster (long rows, rows read by many CTAs: gslam_cluster_us).
  *
  * Layout: CTA r of a graph's cluster owns a contiguous range of its slices (balanced by
  * slot count), one thread per block row (two above 20 slices per CTA). Values (as far as they
@@ -25,8 +26,8 @@
  * all sums, and the halo's z, are there: one one-way trip per reduction. Warp 0 then adds
  * the sums and one thread advances the scalars. (Every warp storing its own slice's sum
  * into every CTA saves the step through warp 0, but the 320 messages per CTA and reduction
- * of a 16 x 640 cluster take longer: 6.6 us per iteration at 10,000 poses against 4.8, and
- * 5.2 against 4.0 at 7,120.)
+ * of a 16 x 640 cluster take longer: in the first form of this kernel 6.6 us per iteration at
+ * 10,000 poses against 4.8, and 5.2 against 4.0 at 7,120, which takes 3.0 now.)
  *
  * The two barriers' phases alternate (p.q, then r.r and r.z), and a CTA sends its sums of
  * phase n + 1 only after it has received every sum of phase n, so one buffer and one

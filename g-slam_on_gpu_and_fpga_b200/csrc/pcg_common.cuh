@@ -245,10 +245,10 @@ __device__ __forceinline__ bool grid_allreduce_rows(const double (&v)[NV][R], do
  * many readers of a line slow the writes to it. That also holds for readers that poll
  * before the data can be there (1.69 us when they poll at once), so the first poll waits
  * TAG_DELAY cycles after the CTA's own value left: the trip's length and part of the CTAs'
- * skew. Resident FP64 solver, us per iteration at 20,000 / 50,000 / 100,000 poses: no wait
- * 4.40 / 5.07 / 6.95, 400 cycles 4.12 / 4.76 / 6.80, 600 3.78 / 4.45 / 6.53, 700 3.70 / 4.37
- * / 6.39, 800 3.82 / 4.36 / 6.31, 1000 4.04 / 4.52 / 6.49. Later polls follow at once (a gap
- * of 150 cycles between them costs 0.1 us).
+ * skew. Resident FP64 solver, us per iteration at 20,000 / 50,000 / 100,000 poses: 600 cycles
+ * 3.54 / 4.43 / 5.94, 680 3.49 / 4.34 / 5.95, 750 3.50 / 4.28 / 5.97, 820 3.53 / 4.27 / 6.02 (without
+ * a wait 0.6 to 0.7 more than with 700, with 1000 0.1 to 0.3 more, in an earlier form of the
+ * solver). Later polls follow at once (a gap of 150 cycles between them costs 0.1 us).
  *
  * The slots are zeroed before every launch; number 1 is the first reduction. Two buffers
  * alternate: a CTA writes number n + 2 only after it has read every CTA's n + 1, which each

@@ -38,7 +38,8 @@ extern "C" {
 #define GSLAM_PREC_FP64_CG 2 /* FP64 block-Jacobi PCG with one grid reduction per iteration
                               * (Chronopoulos-Gear recurrence: the reference's iterates in exact
                               * arithmetic, other rounding); the graph must fit the resident
-                              * layout (<= 32 slices per SM). Batches solve it as FP64. */
+                              * layout: <= 32 slices per SM, and an SM's columns and the rows
+                              * they read in its shared memory. Batches solve it as FP64. */
 
 /* ---- factor families ---- */
 #define GSLAM_FACTORS_REFERENCE 0 /* ObsEdge + MotionEdge of src/cpu_pcg_fp64 */
